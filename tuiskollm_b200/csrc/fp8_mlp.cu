@@ -76,14 +76,14 @@ __global__ void __launch_bounds__(kThreads, SHALLOW ? 2 : 1)
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   Ctl* ctl = reinterpret_cast<Ctl*>(smem + STAGES * STAGE_BYTES);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   // token tiles vary fastest so that the CTAs sharing a weight tile run together (L2 reuse)
   const int tile_m = blockIdx.x, tile_n = blockIdx.y;
   const int nkb = p.k / kTileKBytes;
   const int tok0 = tile_m * BLOCK_TOK;
   const int up_row0 = p.intermediate + tile_n * kRows;
 
-  if (threadIdx.x == 0) {
+  if (warp == 0 && elect_one()) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&ctl->full[s], 1);
       mbar_init(&ctl->empty[s], 1);
@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(kThreads, SHALLOW ? 2 : 1)
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       // weights are streamed once when there is a single token tile, shared otherwise
       const uint64_t pol_a = l2_policy_evict_last();
       const uint64_t pol_w = gridDim.x == 1 ? l2_policy_evict_first() : pol_a;
@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(kThreads, SHALLOW ? 2 : 1)
     }
   } else if (warp == 1) {
     // -------------------------------------------------------------- UMMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       bool ok = true;
       for (int i = 0; i < nkb && ok; ++i) {
         const int s = i % STAGES;

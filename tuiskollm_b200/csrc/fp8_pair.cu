@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(kThreads, kStages <= 3 ? 2 : 1)
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   PairControl<kStages>* ctl = reinterpret_cast<PairControl<kStages>*>(smem + kStages * kStageBytes);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_cta_rank();  // 0 = even CTA (issues the MMAs), 1 = odd
   const int tile_m = blockIdx.x >> 1;        // 256-token tile; token tiles of a row pair run together
   const int pair = blockIdx.y;               // pair of 128-row weight tiles
@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(kThreads, kStages <= 3 ? 2 : 1)
   const int row0 = (2 * pair + static_cast<int>(rank)) * kRows;  // this CTA's weight rows
   const int nkb = p.k / kTileKBytes;
 
-  if (threadIdx.x == 0) {
+  if (warp == 0 && elect_one()) {
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&ctl->full[s], 1);
       mbar_init(&ctl->empty[s], 1);
@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(kThreads, kStages <= 3 ? 2 : 1)
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       const uint64_t pol_w = l2_policy_evict_last();  // re-read by the other token tiles
       const uint64_t pol_a = l2_policy_evict_last();
       const uint32_t bar0 = mapa_u32(smem_u32(&ctl->full[0]), 0);  // the even CTA's full[0]
@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(kThreads, kStages <= 3 ? 2 : 1)
     }
   } else if (warp == 1) {
     // -------------------------------------------------------------- UMMA issuer
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       bool ok = true;
       for (int i = 0; i < nkb && ok; ++i) {
         const int s = i % kStages;

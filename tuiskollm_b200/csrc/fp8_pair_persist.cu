@@ -127,14 +127,14 @@ __global__ void __launch_bounds__(kThreads, 1)
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   PersistControl* ctl = reinterpret_cast<PersistControl*>(smem + kStages * kStageBytes);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_cta_rank();  // 0 = even CTA (issues the MMAs), 1 = odd
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
   const int tiles_m = (p.rows + kTok - 1) / kTok;
   const int tiles = tiles_m * (p.out_rows / (2 * kRows));
   const int nkb = p.k / kTileKBytes;
 
-  if (threadIdx.x == 0) {
+  if (warp == 0 && elect_one()) {
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&ctl->full[s], 1);
       mbar_init(&ctl->empty[s], 1);
@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   // tile t = row pair * tiles_m + token tile: token tiles vary fastest
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       const uint64_t pol = l2_policy_evict_last();  // weight tiles are re-read by the other token tiles
       const uint32_t bar0 = mapa_u32(smem_u32(&ctl->full[0]), 0);  // the even CTA's full[0]
       bool ok = true;
@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   } else if (warp == 1) {
     // -------------------------------------------------------------- UMMA issuer
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       bool ok = true;
       int it = 0, round = 0;
       Walk<STREAM_K> walk(pair, pairs, tiles, nkb);

@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(kThreads, BLOCK_TOK <= 32 ? (DEEP == 1 ? 2 : (
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   Control<BLOCK_TOK>* ctl = reinterpret_cast<Control<BLOCK_TOK>*>(smem + STAGES * STAGE_BYTES);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int tile_n = blockIdx.x, tile_m = blockIdx.y, split = blockIdx.z;
   if (threadIdx.x == 0) TK100_STAMP(p, 0);
   const int kb_total = p.k / kTileKBytes;
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(kThreads, BLOCK_TOK <= 32 ? (DEEP == 1 ? 2 : (
   // tile themselves, so a full[] barrier takes two arrivals: the weight TMA and that warp.
   bool fused_quant = false;
   if constexpr (BLOCK_TOK == 16) fused_quant = p.x_bf16 != nullptr;
-  if (threadIdx.x == 0) {
+  if (warp == 0 && elect_one()) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&ctl->full[s], fused_quant ? 2 : 1);
       mbar_init(&ctl->empty[s], 1);
@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(kThreads, BLOCK_TOK <= 32 ? (DEEP == 1 ? 2 : (
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       const uint64_t pol_w = l2_policy_evict_first();  // weights are streamed once
       const uint64_t pol_a = l2_policy_evict_last();   // activation codes are re-read by every CTA
       // The weight tiles of the first pass over the ring are already on their way (requested
@@ -294,7 +294,7 @@ __global__ void __launch_bounds__(kThreads, BLOCK_TOK <= 32 ? (DEEP == 1 ? 2 : (
     }
   } else if (warp == 1) {
     // -------------------------------------------------------------- UMMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       bool ok = true;
       for (int i = 0; i < nkb && ok; ++i) {
         const int s = i % STAGES;

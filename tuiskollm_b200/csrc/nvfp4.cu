@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(nv_threads(BLOCK_TOK, GATE_UP), (GATE_UP || BL
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   Ctl* ctl = reinterpret_cast<Ctl*>(smem + STAGES * STAGE_BYTES);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   // token tiles vary fastest so that the CTAs sharing a weight tile run together (L2 reuse)
   const int tile_m = blockIdx.x, tile_n = blockIdx.y, split = blockIdx.z;
   const int tiles_m = gridDim.x, tiles_n = gridDim.y;
@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(nv_threads(BLOCK_TOK, GATE_UP), (GATE_UP || BL
   };
   const int pre = nkb < STAGES ? nkb : STAGES;
 
-  if (threadIdx.x == 0) {
+  if (warp == 0 && elect_one()) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&ctl->full[s], 1);
       mbar_init(&ctl->empty[s], 1);
@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(nv_threads(BLOCK_TOK, GATE_UP), (GATE_UP || BL
   if (pushed) cluster_arrive();
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       // the weights of the first ring pass were requested during set-up
       pdl_wait();
       for (int i = 0; i < pre; ++i) load_activations(i, i);
@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(nv_threads(BLOCK_TOK, GATE_UP), (GATE_UP || BL
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t sf_base = tmem + ACC_COLS;
       // a BLOCK_TOK < 128 tile sits in one 32-row quartile of its 128-row scale tile:
       // quartile q of the chunk lands in TMEM column q

@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   PairControl* ctl = reinterpret_cast<PairControl*>(smem + kStages * kStageBytes);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_cta_rank();  // 0 = even CTA (issues the MMAs), 1 = odd
   const int tile_m = blockIdx.x >> 1;        // 256-token tile
   const int pair = blockIdx.y;               // pair of weight tiles
@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   const int nkb = (p.k + kStageK - 1) / kStageK;
   const int chunks_per_tile = p.k / 64;
 
-  if (threadIdx.x == 0) {
+  if (warp == 0 && elect_one()) {
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&ctl->full[s], 1);
       mbar_init(&ctl->empty[s], 1);
@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   pdl_trigger();
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint64_t pol = l2_policy_evict_last();
       bool ok = true;
       pdl_wait();
@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       const uint32_t sf_base = tmem + kAccCols;
       // Per 64-element step: three scale copies (this CTA's weight rows, the two 128-token
       // scale tiles) into a rotating TMEM slot, then the MMA that reads them.  (Queueing a whole

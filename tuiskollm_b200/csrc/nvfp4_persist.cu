@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   float* xchg = reinterpret_cast<float*>(smem + STAGES * kStageBytes);
   Ctl* ctl = reinterpret_cast<Ctl*>(smem + STAGES * kStageBytes + (GATE_UP ? kXchgBytes : 0));
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_cta_rank();  // 0 = even CTA (issues the MMAs), 1 = odd
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
   const int tiles_m = (p.rows + kTok - 1) / kTok;
@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   const int nkb = (p.k + kStageK - 1) / kStageK;
   const int chunks_per_tile = p.k / 64;
 
-  if (threadIdx.x == 0) {
+  if (warp == 0 && elect_one()) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&ctl->full[s], 1);
       mbar_init(&ctl->empty[s], 1);
@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 #endif
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       const uint64_t pol = l2_policy_evict_last();
       bool ok = true;
       pdl_wait();
@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
   } else if (warp == 1) {
     // -------------------------------------------------------------- UMMA issuer
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       const uint32_t sf_base = tmem + kAccCols;
       bool ok = true;
       int it = 0, round = 0;
