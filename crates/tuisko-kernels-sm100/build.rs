@@ -12,13 +12,12 @@ const SOURCES: &[&str] = &[
     "norm_quant.cu",
     "fp8_proj.cu",
     "fp8_pair.cu",
-    "fp8_pair_persist.cu",
     "fp8_mlp.cu",
     "gdn.cu",
     "materialize.cu",
     "nvfp4.cu",
     "nvfp4_pair.cu",
-    "nvfp4_persist.cu",
+    "pair_gemm.cu",
     "peer_reduce.cu",
     "sampler.cu",
     "ops.cu",

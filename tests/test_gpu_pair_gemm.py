@@ -1,0 +1,153 @@
+"""The persistent CTA-pair contractions at the sizes where their tiling can go wrong: token counts
+around the 32-token batches and the 256-token tiles, weight rows that end inside a pair tile, a
+reduction that ends inside a stage, K split over the pairs of a cluster, several tiles per pair
+(accumulator rotation, overlapping accumulators), outputs that are not 16-byte aligned.  Expectation: the
+f64 oracle on the codes the kernel read; bound: one BF16 rounding (2^-8 relative) plus fp32 summation,
+asked for as 1e-2 of max(|expected|, floor) like the other projection tests."""
+import numpy as np
+import pytest
+import torch
+
+from gpu_util import assert_inactive_untouched, dev, host, max_relative_error, sentinel_plane
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def tk():
+    import tuiskollm_b200 as tk
+    return tk
+
+
+def _u16(t):
+    return host(t.view(torch.int16)).view(np.uint16)
+
+
+def _nvfp4_planes(tk, rows, k):
+    return (torch.zeros((rows, k // 2), dtype=torch.uint8, device="cuda"),
+            torch.zeros((tk.ops.nvfp4_scale_plane_bytes(rows, k),), dtype=torch.uint8, device="cuda"))
+
+
+@pytest.mark.parametrize("out_rows,k,rows,tok,splits", [
+    (256, 128, 33, 0, 0),      # one stage, one pair tile
+    (1040, 1024, 64, 0, 0),    # weight rows end inside a pair tile
+    (512, 1024, 301, 0, 0),    # ragged tokens, two tiles of 160
+    (512, 1024, 257, 32, 1),   # smallest token tile
+    (768, 2048, 100, 0, 2),    # K split in two
+    (512, 4096, 130, 160, 4),  # K split in four, odd number of batches
+    (40000, 256, 70, 64, 1),   # more tiles than pairs: three rounds of the two accumulators
+])
+def test_fp8_projection(tk, oracle, monkeypatch, out_rows, k, rows, tok, splits):
+    from tuiskollm_b200 import synth
+
+    monkeypatch.setenv("TK100_PAIR_TOK", str(tok))
+    monkeypatch.setenv("TK100_PAIR_SPLITS", str(splits))
+    c = tk.Context(device=0)
+    xb = synth.normal_bf16(61, rows, (rows, k))
+    w, s = synth.torch_fp8_weights(61, out_rows, out_rows, k, "cuda")
+    codes = torch.zeros((rows, k), dtype=torch.uint8, device="cuda")
+    scales = torch.zeros((rows,), dtype=torch.float32, device="cuda")
+    out = sentinel_plane((rows + 1, out_rows), torch.int16)
+    op = tk.ops.Fp8ProjectionOp(c)
+    op.launch(None, rows, out_rows, k, dev(xb.view(np.int16)), codes, scales, w, s, out)
+    torch.cuda.synchronize()
+    assert c.last_kernel.startswith("fp8_pair_persist_kernel"), c.last_kernel
+    assert f"splits={max(splits, 1)}" in c.last_kernel, c.last_kernel
+    assert c.device_status() == 0
+    oc, os_ = oracle.quantize_e4m3(xb)
+    assert np.array_equal(host(codes), oc)
+    exp = oracle.fp8_projection(oc, os_, host(w), _u16(s))
+    assert max_relative_error(_u16(out)[:rows], exp, 4 * float(np.abs(exp).mean())) <= 1e-2
+    assert_inactive_untouched(out, rows)
+    # an output plane that starts 2 bytes off a 16-byte boundary takes the narrow stores: same bits
+    flat = sentinel_plane((rows * out_rows + 1,), torch.int16)
+    op.launch(None, rows, out_rows, k, None, codes, scales, w, s, flat[1:])
+    torch.cuda.synchronize()
+    assert torch.equal(flat[1:].view(rows, out_rows), out[:rows])
+    assert c.device_status() == 0
+
+
+@pytest.mark.parametrize("rows,tok", [(33, 0), (96, 0), (129, 0), (257, 0), (300, 32)])
+def test_fp8_swiglu(tk, oracle, monkeypatch, rows, tok):
+    from tuiskollm_b200 import synth
+
+    monkeypatch.setenv("TK100_PAIR_TOK", str(tok))
+    hidden, inter = 1024, 1280
+    c = tk.Context(device=0, hidden=hidden, intermediate=inter)
+    xb = synth.normal_bf16(62, rows, (rows, hidden))
+    wc, ws = synth.fp8_weights(62, 1, 2 * inter, hidden)
+    codes = torch.zeros((rows, hidden), dtype=torch.uint8, device="cuda")
+    scales = torch.zeros((rows,), dtype=torch.float32, device="cuda")
+    out = sentinel_plane((rows + 1, inter), torch.int16)
+    tk.Fp8SwiGluOp(c).launch(None, rows, dev(xb.view(np.int16)), codes, scales, dev(wc), dev(ws.view(np.int16)), out)
+    torch.cuda.synchronize()
+    assert c.last_kernel.startswith("fp8_swiglu_kernel_pairs"), c.last_kernel
+    assert c.device_status() == 0
+    oc, os_ = oracle.quantize_e4m3(xb)
+    dots = oracle.fp8_projection(oc, os_, wc, ws)
+    exp = oracle.silu_mul(dots[:, :inter], dots[:, inter:])
+    assert max_relative_error(_u16(out)[:rows], exp, 4 * float(np.abs(exp).mean())) <= 1e-2
+    assert_inactive_untouched(out, rows)
+
+
+@pytest.mark.parametrize("hidden,inter,rows,tok,splits", [
+    (1024, 512, 33, 0, 0),
+    (1024, 1664, 97, 0, 0),     # down: K = 1664 ends half-way into its last stage
+    (1024, 1536, 160, 0, 0),
+    (1024, 1536, 301, 128, 1),
+    (1024, 512, 500, 256, 1),
+    (256, 12800, 520, 256, 1),  # several tiles per pair on overlapping accumulators
+    (256, 9728, 700, 128, 1),   # and on disjoint ones
+    (512, 9472, 70, 0, 4),      # down: K split in four over 37 stages
+])
+def test_nvfp4_mlp(tk, oracle, monkeypatch, hidden, inter, rows, tok, splits):
+    """gate/up + SwiGLU with the NVFP4 form of its output, then the down projection in both output
+    types; codes and scales of the intermediate are the quantiser's bit for bit."""
+    from tuiskollm_b200 import synth
+
+    monkeypatch.setenv("TK100_PAIR_TOK", str(tok))
+    xb = synth.normal_bf16(63, rows, (rows, hidden))
+    gu, gus, gud = synth.nvfp4_weights(63, 1, 2 * inter, hidden)
+    dn, dns, dnd = synth.nvfp4_weights(63, 2, hidden, inter)
+    a_div, m_div = float(np.float32(448.0 * 6.0 / 5.0)), float(np.float32(448.0 * 6.0 / 8.0))
+    c = tk.Context(device=0, hidden=hidden, intermediate=inter)
+    a_codes, a_scales = _nvfp4_planes(tk, rows, hidden)
+    m_codes, m_scales = _nvfp4_planes(tk, rows, inter)
+    mid = sentinel_plane((rows + 1, inter), torch.int16)
+    out = sentinel_plane((rows + 1, hidden), torch.int16)
+    part = sentinel_plane((rows + 1, hidden), torch.float32)
+    tk.Nvfp4SwiGluOp(c).launch_quantize(None, rows, dev(xb.view(np.int16)), dev(gu), dev(gus), float(gud), mid,
+                                        activation_codes=a_codes, activation_scales=a_scales,
+                                        input_global_divisor=a_div, output_global_divisor=m_div,
+                                        output_codes=m_codes, output_scales=m_scales)
+    assert c.last_kernel.startswith("nvfp4_persist_kernel"), c.last_kernel
+    if splits:
+        monkeypatch.setenv("TK100_PAIR_SPLITS", str(splits))
+        c2 = tk.Context(device=0, hidden=hidden, intermediate=inter)
+    else:
+        c2 = c
+    down = tk.Nvfp4DownOp(c2)
+    kw = dict(activation_codes=m_codes, activation_scales=m_scales, input_global_divisor=m_div)
+    down.launch(None, rows, None, dev(dn), dev(dns), float(dnd), out, **kw)
+    if splits:
+        assert f"splits={splits}" in c2.last_kernel, c2.last_kernel
+    down.launch_partial(None, rows, None, dev(dn), dev(dns), float(dnd), part, **kw)
+    torch.cuda.synchronize()
+    assert c.device_status() == 0 and c2.device_status() == 0
+    oc, osc = oracle.nvfp4_quantize(xb, a_div)
+    dots = oracle.nvfp4_w4a4_dot(oc, osc, a_div, gu, gus, float(gud))
+    exp_mid = oracle.silu_mul(dots[:, :inter], dots[:, inter:])
+    got_mid = _u16(mid)[:rows]
+    assert max_relative_error(got_mid, exp_mid, 4 * float(np.abs(exp_mid).mean())) <= 1e-2
+    mc, msc = oracle.nvfp4_quantize(got_mid, m_div)
+    assert np.array_equal(host(m_codes), mc)
+    assert np.array_equal(host(m_scales), msc)
+    exp = oracle.nvfp4_w4a4_dot(mc, msc, m_div, dn, dns, float(dnd))
+    floor = 4 * float(np.abs(exp).mean())
+    got = _u16(out)[:rows]
+    assert max_relative_error(got, exp, floor) <= 1e-2
+    got32 = host(part)[:rows]
+    assert (np.abs(got32 - exp) / np.maximum(np.abs(exp), floor)).max() <= 2e-3
+    assert np.array_equal(oracle.f32_to_bf16(got32), got)
+    for plane in (mid, out, part):
+        assert_inactive_untouched(plane, rows)

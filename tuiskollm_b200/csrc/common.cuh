@@ -47,6 +47,63 @@ __device__ __forceinline__ uint32_t f32x2_to_e2m1x2(float lo, float hi) {
       __nv_cvt_float2_to_fp4x2(make_float2(lo, hi), __NV_E2M1, cudaRoundNearest));
 }
 
+// silu(v) in the sign-stable form of the reference's NVFP4 route
+// (tuisko-kernels-sm89/src/nvfp4/swiglu.rs:142-155), ex2.approx for the exponential.
+__device__ __forceinline__ float silu_stable(float v) {
+  const float e = -fabsf(v) * 1.4426950408889634f;
+  float ex;  // .ftz: 2^e below the normal range reads as 0, as the e < -126 cut-off did
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(ex) : "f"(e));
+  return __fdividef(v >= 0.0f ? v : v * ex, 1.0f + ex);
+}
+
+// SiLU in the dense-FP8 path's form, v / (1 + ex2(-v * log2 e)) (tuisko-kernels-sm120
+// device/fp8_swiglu.rs:13-15).
+__device__ __forceinline__ float silu_fp8_path(float v) {
+  float ex;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(ex) : "f"(-v * 1.4426950408889634f));
+  return __fdividef(v, 1.0f + ex);
+}
+
+// t / s for a NVFP4 block: s is a decoded E4M3 scale (4 significant bits), inv = __frcp_rn(s).  One
+// residual step on the reciprocal's product (P. Markstein, "Computation of elementary functions on the
+// IBM RISC System/6000 processor", IBM J. Res. Dev. 34 (1990), theorem on the corrected quotient)
+// rounds like the division wherever an E2M1 code depends on it; quotients below the first rounding
+// boundary (signed zeros among them), past the saturation point, infinities and NaNs keep the product.
+__device__ __forceinline__ float nvfp4_quotient(float t, float s, float inv) {
+  const float q = __fmul_rn(t, inv);
+  const float corrected = __fmaf_rn(__fmaf_rn(-q, s, t), inv, q);
+  return (fabsf(q) > 0.125f && fabsf(q) < 8.0f) ? corrected : q;
+}
+
+// NVFP4 form of 16 consecutive BF16 values (8 packed pairs, low half first):
+//   scale = e4m3_rne_sat((amax * divisor) / 6),  code = e2m1_rne_sat((x * divisor) / scale),
+// signed zeros when the scale underflows to 0.  Codes low nibble first.
+__device__ __forceinline__ uint2 nvfp4_quantize_block(const uint32_t (&w)[8], float divisor, uint32_t* scale_code) {
+  float amax = 0.0f;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fmaxf(fabsf(bf16x2_lo(w[j])), fabsf(bf16x2_hi(w[j]))));
+  const uint32_t sc = f32x2_to_e4m3x2(__fdiv_rn(__fmul_rn(amax, divisor), 6.0f), 0.0f) & 0xffu;
+  *scale_code = sc;
+  const float s = e4m3_to_f32(sc);
+  uint32_t packed[2] = {0u, 0u};
+  if (s == 0.0f) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const uint32_t byte = ((w[j] & 0x8000u) ? 0x08u : 0u) | ((w[j] & 0x80000000u) ? 0x80u : 0u);
+      packed[j >> 2] |= byte << (8 * (j & 3));
+    }
+  } else {
+    const float inv = __frcp_rn(s);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const uint32_t byte = f32x2_to_e2m1x2(nvfp4_quotient(__fmul_rn(bf16x2_lo(w[j]), divisor), s, inv),
+                                            nvfp4_quotient(__fmul_rn(bf16x2_hi(w[j]), divisor), s, inv)) & 0xffu;
+      packed[j >> 2] |= byte << (8 * (j & 3));
+    }
+  }
+  return make_uint2(packed[0], packed[1]);
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

@@ -55,12 +55,6 @@ constexpr size_t sw_smem_bytes() {
          sizeof(SwControl<BLOCK_TOK, SHALLOW>);
 }
 
-__device__ __forceinline__ float silu_fp8_path(float v) {
-  float ex;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(ex) : "f"(-v * 1.4426950408889634f));
-  return __fdividef(v, 1.0f + ex);
-}
-
 template <int BLOCK_TOK, bool SHALLOW>
 __global__ void __launch_bounds__(kThreads, SHALLOW ? 2 : 1)
     fp8_swiglu_kernel(const __grid_constant__ CUtensorMap tmap_w,

@@ -268,13 +268,6 @@ int fp8_projection_stages(int block_tok);
 cudaError_t fp8_projection_prepare();  // sets the dynamic shared-memory attributes once
 // fp8_pair.cu: prefill route on CTA pairs (256-row x 256-token pair tiles, BF16 output only,
 // unsplit K; out_rows must be a multiple of 256).
-// Persistent form (fp8_pair_persist.cu): `pairs` resident CTA pairs walk the pair tiles.
-cudaError_t fp8_pair_persist_prepare();
-// stream_k: the pairs share the launch's tiles x K steps evenly; pieces of a tile meet in
-// p.partials (fp8_pair_stream_k_scratch_bytes) under tickets in p.counters (two per pair tile).
-cudaError_t launch_fp8_pair_persist(cudaStream_t stream, int pairs, const CUtensorMap& tmap_w,
-                                    const CUtensorMap& tmap_a, const Fp8ProjParams& p, bool stream_k);
-size_t fp8_pair_stream_k_scratch_bytes(int pairs);
 cudaError_t fp8_pair_prepare();
 cudaError_t launch_fp8_pair(cudaStream_t stream, const CUtensorMap& tmap_w, const CUtensorMap& tmap_a,
                             const Fp8ProjParams& p);
@@ -308,6 +301,41 @@ cudaError_t launch_peer_sum(cudaStream_t stream, int ctas, const PeerSumParams& 
 // [shards, rows] pairs -> [rows] pairs with the first-maximum rule.
 cudaError_t launch_argmax_merge(cudaStream_t stream, int rows, int shards,
                                 const ArgmaxPair* gathered, ArgmaxPair* out);
+
+// ---------------------------------------------------------------- pair_gemm.cu
+// Persistent CTA pairs for contractions of many tokens (see the file): plain FP8 / NVFP4 projections
+// and both gate/up + SwiGLU forms.
+constexpr int kPairGemmMaxSplits = 4;
+struct PairGemmParams {
+  int rows;             // active tokens M
+  int out_rows;         // outputs per token (the intermediate size with SwiGLU)
+  int k;                // reduction length in elements
+  int nkb;              // stages of 128 bytes of codes per row
+  int tok_tile;         // tokens per pair tile, a multiple of 32 up to 256
+  int tiles_m;          // token tiles
+  int row_units;        // pair tiles along the weights: 256 rows, or 128 outputs with SwiGLU
+  int splits;           // pairs per cluster that split K (1: persistent over the tiles)
+  int stages, stage_bytes;
+  int chunks_per_tile;  // NVFP4: 512-byte scale chunks per 128-row tile (k / 64)
+  int vector_out;       // `out` is 16-byte aligned
+  const float* act_scales;   // FP8: [rows]
+  const uint16_t* w_scales;  // FP8: BF16 per weight row
+  float out_scale;           // NVFP4
+  uint16_t* out;             // [rows, out_rows] BF16
+  float* out_f32;            // NVFP4 projection: unrounded fp32 instead
+  uint8_t* q_codes;          // NVFP4 SwiGLU: also the NVFP4 form of the outputs
+  uint8_t* q_scales;
+  float q_divisor;
+  uint32_t* status;
+};
+int pair_gemm_stage_bytes(bool nvfp4, int tok_tile);
+int pair_gemm_stages(int stage_bytes);
+// max_clusters[s], s = 1..kPairGemmMaxSplits: clusters of 2 s CTAs resident at once.
+cudaError_t pair_gemm_prepare(int* max_clusters);
+// `workers` clusters of `p.splits` pairs.
+cudaError_t launch_pair_gemm(cudaStream_t stream, bool nvfp4, bool swiglu, int workers, const CUtensorMap& map_w,
+                             const CUtensorMap& map_a, const CUtensorMap& map_wsf, const CUtensorMap& map_asf,
+                             const PairGemmParams& p);
 
 // -------------------------------------------------------------------- nvfp4.cu
 struct Nvfp4Params {
@@ -353,12 +381,6 @@ cudaError_t nvfp4_pair_prepare();
 cudaError_t launch_nvfp4_pair(cudaStream_t stream, bool gate_up, const CUtensorMap& tmap_w,
                               const CUtensorMap& tmap_a, const CUtensorMap& tmap_wsf,
                               const CUtensorMap& tmap_asf, const Nvfp4Params& p);
-// nvfp4_persist.cu: prefill route on persistent CTA pairs (256-row x 256-token pair tiles, one
-// pair per two SMs walking its share of the tiles).  `max_pairs`: pairs resident at once.
-cudaError_t nvfp4_persist_prepare(int* max_pairs);
-cudaError_t launch_nvfp4_persist(cudaStream_t stream, bool gate_up, int pairs, const CUtensorMap& tmap_w,
-                                 const CUtensorMap& tmap_a, const CUtensorMap& tmap_wsf,
-                                 const CUtensorMap& tmap_asf, const Nvfp4Params& p);
 cudaError_t launch_f32_to_bf16(cudaStream_t stream, long long n, const float* in, uint16_t* out);
 cudaError_t launch_nvfp4_quantize(cudaStream_t stream, int rows, int k, const uint16_t* x,
                                   float divisor, uint8_t* codes, uint8_t* scales);

@@ -77,15 +77,6 @@ __device__ __forceinline__ void nv_epilogue_barrier() {
   asm volatile("bar.sync 1, %0;" ::"n"(kEpilogueThreads) : "memory");
 }
 
-// silu(v) in the sign-stable form of the reference's NVFP4 route
-// (tuisko-kernels-sm89/src/nvfp4/swiglu.rs:142-155), ex2.approx for the exponential.
-__device__ __forceinline__ float silu_stable(float v) {
-  const float e = -fabsf(v) * 1.4426950408889634f;
-  float ex;  // .ftz: 2^e below the normal range reads as 0, as the e < -126 cut-off did
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(ex) : "f"(e));
-  return __fdividef(v >= 0.0f ? v : v * ex, 1.0f + ex);
-}
-
 // One value per lane, a 16-column block = 16 consecutive lanes: the block's E4M3 scale code
 // (bits 8..15 of the result) and this lane's E2M1 code (bits 0..3), as nvfp4_quantize_kernel
 // defines them.  Kept out of line so that the sixteen calls of an epilogue chunk do not interleave

@@ -3,6 +3,7 @@
 
 #include <cudaTypedefs.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -42,6 +43,8 @@ Tuning Tuning::from_environment() {
   t.swiglu_pairs = env_int("TK100_SWIGLU_PAIRS", t.swiglu_pairs);
   t.fp8_persist = env_int("TK100_FP8_PERSIST", t.fp8_persist);
   t.fp8_stream_k = env_int("TK100_FP8_STREAMK", t.fp8_stream_k);
+  t.pair_tok = env_int("TK100_PAIR_TOK", t.pair_tok);
+  t.pair_splits = env_int("TK100_PAIR_SPLITS", t.pair_splits);
   t.nvfp4_wide = env_int("TK100_NVFP4_WIDE", t.nvfp4_wide);
   t.nvfp4_wide_min_rows = env_int("TK100_NVFP4_WIDE_MIN_ROWS", t.nvfp4_wide_min_rows);
   t.nvfp4_persist = env_int("TK100_PERSIST", t.nvfp4_persist);
@@ -133,11 +136,6 @@ Status Context::create(const tk100_config& in, Context** out, std::string* error
     delete ctx;
     return TK100_ERR_MODULE;
   }
-  if ((e = fp8_pair_persist_prepare()) != cudaSuccess) {
-    *error = std::string("[gpu.module] preparing the persistent FP8 pair kernel: ") + cudaGetErrorString(e);
-    delete ctx;
-    return TK100_ERR_MODULE;
-  }
   if ((e = fp8_pair_prepare()) != cudaSuccess) {
     *error = std::string("[gpu.module] preparing the FP8 pair route: ") + cudaGetErrorString(e);
     delete ctx;
@@ -148,8 +146,8 @@ Status Context::create(const tk100_config& in, Context** out, std::string* error
     delete ctx;
     return TK100_ERR_MODULE;
   }
-  if ((e = nvfp4_persist_prepare(&ctx->persist_pairs_)) != cudaSuccess) {
-    *error = std::string("[gpu.module] preparing the persistent NVFP4 routes: ") + cudaGetErrorString(e);
+  if ((e = pair_gemm_prepare(ctx->pair_clusters_)) != cudaSuccess) {
+    *error = std::string("[gpu.module] preparing the persistent pair routes: ") + cudaGetErrorString(e);
     delete ctx;
     return TK100_ERR_MODULE;
   }
@@ -284,6 +282,59 @@ Status Context::scale_map(const void* base, uint64_t chunks, CUtensorMap* out) {
   return TK100_OK;
 }
 
+Status Context::swiglu_map(const void* base, uint64_t outputs, uint64_t row_bytes, CUtensorMap* out) {
+  const MapKey key{base, outputs, row_bytes, 16u, 2u};
+  auto it = maps_.find(key);
+  if (it != maps_.end()) {
+    *out = it->second;
+    return TK100_OK;
+  }
+  auto encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(encode_fn_);
+  CUtensorMap map;
+  const cuuint64_t dims[4] = {row_bytes, 32, 2, outputs / 32};
+  const cuuint64_t strides[3] = {row_bytes, outputs * row_bytes, 32 * row_bytes};
+  const cuuint32_t box[4] = {128u, 16u, 2u, 4u};
+  const cuuint32_t elem[4] = {1u, 1u, 1u, 1u};
+  CUresult r = encode(&map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, const_cast<void*>(base), dims, strides, box, elem,
+                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    return fail(TK100_ERR_DRIVER, "[gpu.driver] cuTensorMapEncodeTiled (gate/up plane) failed with CUresult " +
+                                      std::to_string(static_cast<int>(r)));
+  }
+  if (maps_.size() > 4096) maps_.clear();
+  maps_.emplace(key, map);
+  *out = map;
+  return TK100_OK;
+}
+
+Status Context::swiglu_scale_map(const void* base, uint64_t outputs, uint64_t chunks_per_tile, CUtensorMap* out) {
+  const uint64_t chunks = outputs / 128 * chunks_per_tile;
+  const MapKey key{base, chunks, 512u, 4u, 3u};
+  auto it = maps_.find(key);
+  if (it != maps_.end()) {
+    *out = it->second;
+    return TK100_OK;
+  }
+  auto encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(encode_fn_);
+  CUtensorMap map;
+  const cuuint64_t dims[4] = {64, 2, 2, chunks};
+  const cuuint64_t strides[3] = {256, chunks * 512, 512};
+  const cuuint32_t box[4] = {64u, 1u, 2u, 4u};
+  const cuuint32_t elem[4] = {1u, 1u, 1u, 1u};
+  CUresult r = encode(&map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, const_cast<void*>(base), dims, strides, box, elem,
+                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    return fail(TK100_ERR_DRIVER, "[gpu.driver] cuTensorMapEncodeTiled (gate/up scale plane) failed with CUresult " +
+                                      std::to_string(static_cast<int>(r)));
+  }
+  if (maps_.size() > 4096) maps_.clear();
+  maps_.emplace(key, map);
+  *out = map;
+  return TK100_OK;
+}
+
 // -------------------------------------------------------------- ResidualNormOp
 
 namespace {
@@ -318,6 +369,75 @@ Status check_plane(Context& ctx, const char* what, const char* plane, const void
     Status _s = (expr);                  \
     if (_s != TK100_OK) return _s;       \
   } while (0)
+
+}  // namespace
+
+// ------------------------------------------------------- persistent CTA pairs
+
+namespace {
+
+// Fewest tokens that run on pairs.
+constexpr int kPairMinRows = 33;
+
+struct PairPlan {
+  int tok_tile = 0, tiles_m = 0, splits = 1, workers = 0;
+  double cycles = 1e30;  // estimate; only compared with other plans
+};
+
+// Token tile and K splits of a pair_gemm launch: the cheapest by a count of SM cycles.  A stage of a pair
+// tile takes the longer of its MMAs (2 N cycles for 256 x N x 128 bytes) and of its delivery from L2
+// (about 56 bytes per cycle and SM measured on B200); a launch takes at least its weights at HBM rate
+// (about 3.9 KB per cycle).  Splitting K costs an exchange and wants at least 8 stages a split.
+PairPlan plan_pairs(const Context& ctx, int rows, int row_units, int nkb, bool nvfp4, double weight_bytes,
+                    bool may_split) {
+  PairPlan best;
+  const Tuning& tune = ctx.tuning();
+  const int least = (rows + 255) / 256;
+  // NVFP4: whole 128-token scale tiles (a 64-token block-scaled pair MMA is not taken by the hardware)
+  const int grain = nvfp4 ? 128 : 32;
+  for (int n = least; n < least + 4; ++n) {
+    int tok = ((rows + n - 1) / n + grain - 1) / grain * grain;
+    if (tune.pair_tok > 0 && tune.pair_tok <= 256 && tune.pair_tok % grain == 0) tok = tune.pair_tok;
+    const int tiles_m = (rows + tok - 1) / tok;
+    const long long tiles = static_cast<long long>(tiles_m) * row_units;
+    const double stage = std::max(2.0 * tok, pair_gemm_stage_bytes(nvfp4, tok) / 56.0);
+    for (int s = 1; s <= kPairGemmMaxSplits; ++s) {
+      if (tune.pair_splits > 0 && s != tune.pair_splits) continue;
+      const int clusters = ctx.pair_clusters(s);
+      if (clusters <= 0 || (s > 1 && (!may_split || nkb / s < 8 || tiles > clusters))) continue;
+      const long long waves = s > 1 ? 1 : (tiles + clusters - 1) / clusters;
+      const double body = static_cast<double>(waves) * ((nkb + s - 1) / s) * stage;
+      const double cycles = std::max(body, weight_bytes / 3900.0) + 4.0 * tok + (s > 1 ? 1500.0 : 0.0);
+      if (cycles < best.cycles) {
+        best.tok_tile = tok;
+        best.tiles_m = tiles_m;
+        best.splits = s;
+        best.workers = static_cast<int>(std::min<long long>(tiles, clusters));
+        best.cycles = cycles;
+      }
+    }
+  }
+  return best;
+}
+
+PairGemmParams pair_params(Context& ctx, const PairPlan& plan, int rows, int out_rows, int k, int row_units, bool nvfp4,
+                           const void* out) {
+  PairGemmParams q{};
+  q.rows = rows;
+  q.out_rows = out_rows;
+  q.k = k;
+  q.nkb = nvfp4 ? (k + 255) / 256 : k / 128;
+  q.tok_tile = plan.tok_tile;
+  q.tiles_m = plan.tiles_m;
+  q.row_units = row_units;
+  q.splits = plan.splits;
+  q.stage_bytes = pair_gemm_stage_bytes(nvfp4, plan.tok_tile);
+  q.stages = pair_gemm_stages(q.stage_bytes);
+  q.chunks_per_tile = k / 64;
+  q.vector_out = aligned(out, 16) ? 1 : 0;
+  q.status = ctx.status_word();
+  return q;
+}
 
 }  // namespace
 
@@ -684,8 +804,36 @@ Status Fp8ProjectionOp::launch(cudaStream_t stream, int rows, int out_rows, int 
     TK100_TRY(quantize(stream, rows, columns, input, activation_codes, activation_scales));
   }
 
-  // Prefill shapes with a plain BF16 output: CTA pairs (256-row x 256-token pair tiles) halve
-  // the operand bytes per MAC, which is what bounds the one-CTA kernel there.
+  // More than a few dozen tokens with a plain BF16 output: persistent CTA pairs.
+  {
+    const Tuning& tune = ctx_.tuning();
+    const bool wanted = tune.fp8_persist > 0 || tune.fp8_stream_k != 0 ||
+                        (tune.fp8_persist < 0 && rows >= kPairMinRows);
+    if (wanted && tune.fp8_pair != 0 && output && !logits_f32 && !argmax_scratch && ctx_.forced_block_tok() == 0 &&
+        ctx_.forced_splits() == 0) {
+      const int row_units = (out_rows + 255) / 256;
+      const int nkb = columns / 128;
+      const bool may_split = tune.fp8_stream_k != 0 || (tune.fp8_persist < 0 && tune.fp8_pair == 1);
+      const PairPlan plan = plan_pairs(ctx_, rows, row_units, nkb, false, static_cast<double>(out_rows) * columns,
+                                       may_split);
+      CUtensorMap map_w, map_a;
+      TK100_TRY(ctx_.tensor_map(weight_codes, static_cast<uint64_t>(out_rows), static_cast<uint64_t>(columns), 128,
+                                &map_w));
+      TK100_TRY(ctx_.tensor_map(activation_codes, static_cast<uint64_t>(rows), static_cast<uint64_t>(columns),
+                                static_cast<uint32_t>(plan.tok_tile / 2), &map_a));
+      PairGemmParams q = pair_params(ctx_, plan, rows, out_rows, columns, row_units, false, output);
+      q.act_scales = activation_scales;
+      q.w_scales = weight_scales;
+      q.out = output;
+      ctx_.count_launch();
+      ctx_.note_route(tune.fp8_stream_k != 0 ? "fp8_pair_stream_k_kernel" : "fp8_pair_persist_kernel", plan.tok_tile,
+                      plan.workers, plan.splits, 1);
+      return ctx_.check(launch_pair_gemm(stream, false, false, plan.workers, map_w, map_a, map_w, map_a, q),
+                        "launching the persistent FP8 pair projection");
+    }
+  }
+
+  // TK100_FP8_PERSIST=0: one pair tile (256 rows x 256 tokens) per CTA pair.
   {
     const Tuning& tune = ctx_.tuning();
     const int min_rows = tune.fp8_pair_min_rows;
@@ -697,23 +845,8 @@ Status Fp8ProjectionOp::launch(cudaStream_t stream, int rows, int out_rows, int 
     // walking K = 17408) leaves most SMs idle as well; the one-CTA kernel splits K over clusters
     // there (measured 44.6 against 57.0 us).
     const bool long_k_few_tiles = pair_ctas < ctx_.sm_count() / 2 && columns >= 16384;
-    // Stream-K on resident pairs (TK100_FP8_STREAMK=1, an experiment switch: measured slower than
-    // the routes below at every benchmarked shape): every pair streams the same share of the
-    // launch's tiles x K steps.
-    const long long pair_tile_count = pair_ctas / 2;
-    const int k_steps = columns / 128;
-    bool stream_k = false;
-    int stream_pairs = 0;
-    if (tune.fp8_stream_k != 0 && ctx_.persist_pairs() > 0) {
-      const long long steps = pair_tile_count * k_steps;
-      stream_pairs = static_cast<int>(steps < ctx_.persist_pairs() ? steps : ctx_.persist_pairs());
-      const bool fits = stream_pairs > 0 &&
-                        fp8_pair_stream_k_scratch_bytes(stream_pairs) <= ctx_.partial_bytes() &&
-                        static_cast<size_t>(2 * pair_tile_count) <= ctx_.counter_count();
-      stream_k = fits;
-    }
     if (tune.fp8_pair != 0 && rows >= min_rows && out_rows % 256 == 0 &&
-        ((pair_ctas >= 32 && !long_k_few_tiles) || tune.fp8_pair == 2 || stream_k) && output &&
+        ((pair_ctas >= 32 && !long_k_few_tiles) || tune.fp8_pair == 2) && output &&
         !logits_f32 && !argmax_scratch && ctx_.forced_block_tok() == 0 && ctx_.forced_splits() == 0) {
       CUtensorMap map_w, map_a;
       TK100_TRY(ctx_.tensor_map(weight_codes, static_cast<uint64_t>(out_rows),
@@ -735,23 +868,6 @@ Status Fp8ProjectionOp::launch(cudaStream_t stream, int rows, int out_rows, int 
       q.debug = debug_flags();
       q.stamps = debug_stamps();
       ctx_.count_launch();
-      if (stream_k) {
-        q.partials = ctx_.partials();
-        q.counters = ctx_.counters();
-        ctx_.note_route("fp8_pair_stream_k_kernel", 6, stream_pairs, 1, 1);
-        return ctx_.check(launch_fp8_pair_persist(stream, stream_pairs, map_w, map_a, q, true),
-                          "launching the stream-K FP8 pair projection");
-      }
-      // More pair tiles than pairs that fit the device at once: the resident pairs walk the tiles
-      // with two accumulators in rotation (TK100_FP8_PERSIST).
-      const long long pair_tiles = pair_ctas / 2;
-      if (tune.fp8_persist != 0 && ctx_.persist_pairs() > 0 &&
-          (pair_tiles > ctx_.persist_pairs() || tune.fp8_persist == 2)) {
-        const int pairs = static_cast<int>(pair_tiles < ctx_.persist_pairs() ? pair_tiles : ctx_.persist_pairs());
-        ctx_.note_route("fp8_pair_persist_kernel", 6, pairs, 1, 1);
-        return ctx_.check(launch_fp8_pair_persist(stream, pairs, map_w, map_a, q, false),
-                          "launching the persistent FP8 pair projection");
-      }
       ctx_.note_route("fp8_pair_kernel", q.deep_ring ? 6 : 3, 0, 1, 1);
       return ctx_.check(launch_fp8_pair(stream, map_w, map_a, q), "launching the FP8 pair projection");
     }
@@ -908,6 +1024,21 @@ Status Fp8SwiGluOp::launch(cudaStream_t stream, int rows, const uint16_t* input,
     TK100_TRY(Fp8ProjectionOp(ctx_, name).quantize(stream, rows, hidden, input, activation_codes,
                                                    activation_scales));
   }
+  if (ctx_.tuning().fp8_persist > 0 || (ctx_.tuning().fp8_persist < 0 && rows >= kPairMinRows)) {
+    const PairPlan plan = plan_pairs(ctx_, rows, inter / 128, hidden / 128, false, 2.0 * inter * hidden, false);
+    CUtensorMap map_w, map_a;
+    TK100_TRY(ctx_.swiglu_map(weight_codes, static_cast<uint64_t>(inter), static_cast<uint64_t>(hidden), &map_w));
+    TK100_TRY(ctx_.tensor_map(activation_codes, static_cast<uint64_t>(rows), static_cast<uint64_t>(hidden),
+                              static_cast<uint32_t>(plan.tok_tile / 2), &map_a));
+    PairGemmParams q = pair_params(ctx_, plan, rows, inter, hidden, inter / 128, false, output);
+    q.act_scales = activation_scales;
+    q.w_scales = weight_scales;
+    q.out = output;
+    ctx_.count_launch();
+    ctx_.note_route("fp8_swiglu_kernel_pairs", plan.tok_tile, plan.workers, plan.splits, 1);
+    return ctx_.check(launch_pair_gemm(stream, false, true, plan.workers, map_w, map_a, map_w, map_a, q),
+                      "launching the persistent FP8 SwiGLU");
+  }
   const int block_tok = rows <= 32 ? 32 : 128;
   CUtensorMap map_w, map_a;
   TK100_TRY(ctx_.tensor_map(weight_codes, static_cast<uint64_t>(2) * inter, static_cast<uint64_t>(hidden),
@@ -1053,39 +1184,42 @@ Status Nvfp4MlpOp::launch(cudaStream_t stream, bool gate_up, int rows, int out_r
       return quantise_after();
     }
   }
-  // Prefill shapes: persistent CTA pairs on 256-row x 256-token pair tiles (halves the operand
-  // bytes per MAC through the SM's L2 port and the scale copies per MAC; the epilogue of one tile
-  // runs under the next tile's MMAs).
-  if (ctx_.tuning().nvfp4_persist != 0 && rows >= ctx_.tuning().nvfp4_persist_min_rows &&
-      ctx_.persist_pairs() > 0 && (gate_up || out_rows % 256 == 0)) {
+  // More than a few dozen tokens: persistent CTA pairs.  An explicit choice of another route or of a
+  // reduction of the one-CTA kernels keeps those.
+  const Tuning& tune = ctx_.tuning();
+  const bool pairs_chosen = tune.nvfp4_persist > 0 ? rows >= tune.nvfp4_persist_min_rows
+                                                   : tune.nvfp4_persist < 0 && rows >= kPairMinRows;
+  if (pairs_chosen && tune.cluster == 3 && tune.swiglu_pairs != 0 && tune.nvfp4_wide == 0 &&
+      ctx_.forced_splits() == 0) {
+    const int row_units = gate_up ? out_rows / 128 : (out_rows + 255) / 256;
     const uint64_t w_rows = static_cast<uint64_t>(out_rows) * (gate_up ? 2 : 1);
     const uint64_t chunks_per_tile = static_cast<uint64_t>(columns / 64);
+    const PairPlan plan = plan_pairs(ctx_, rows, row_units, (columns + 255) / 256, true,
+                                     static_cast<double>(w_rows) * columns * 9 / 16, !gate_up && tune.nvfp4_persist < 0);
     CUtensorMap map_w, map_a, map_wsf, map_asf;
-    TK100_TRY(ctx_.tensor_map(weight_codes, w_rows, static_cast<uint64_t>(columns / 2), 128, &map_w));
-    TK100_TRY(ctx_.tensor_map(activation_codes, static_cast<uint64_t>(rows),
-                              static_cast<uint64_t>(columns / 2), 128, &map_a));
-    TK100_TRY(ctx_.scale_map(weight_scales, (w_rows / 128) * chunks_per_tile, &map_wsf));
-    TK100_TRY(ctx_.scale_map(activation_scales,
-                             static_cast<uint64_t>((rows + 127) / 128) * chunks_per_tile, &map_asf));
-    Nvfp4Params q{};
-    q.rows = rows;
-    q.out_rows = out_rows;
-    q.k = columns;
-    q.splits = 1;
-    q.up_row_offset = gate_up ? out_rows : 0;
+    if (gate_up) {
+      TK100_TRY(ctx_.swiglu_map(weight_codes, static_cast<uint64_t>(out_rows), static_cast<uint64_t>(columns / 2), &map_w));
+      TK100_TRY(ctx_.swiglu_scale_map(weight_scales, static_cast<uint64_t>(out_rows), chunks_per_tile, &map_wsf));
+    } else {
+      TK100_TRY(ctx_.tensor_map(weight_codes, w_rows, static_cast<uint64_t>(columns / 2), 128, &map_w));
+      TK100_TRY(ctx_.scale_map(weight_scales, (w_rows / 128) * chunks_per_tile, &map_wsf));
+    }
+    TK100_TRY(ctx_.tensor_map(activation_codes, static_cast<uint64_t>(rows), static_cast<uint64_t>(columns / 2),
+                              static_cast<uint32_t>(plan.tok_tile / 2), &map_a));
+    TK100_TRY(ctx_.scale_map(activation_scales, static_cast<uint64_t>((rows + 127) / 128) * chunks_per_tile, &map_asf));
+    PairGemmParams q = pair_params(ctx_, plan, rows, out_rows, columns, row_units, true, output);
     q.out_scale = 1.0f / (weight_scale_divisor * input_global_divisor);
     q.out = output;
     q.out_f32 = output_f32;
-    q.status = ctx_.status_word();
-    q.debug = debug_flags();
-    q.stamps = debug_stamps();
-    const long long tiles = static_cast<long long>((rows + 255) / 256) * (gate_up ? out_rows / 128 : out_rows / 256);
-    const int pairs = static_cast<int>(tiles < ctx_.persist_pairs() ? tiles : ctx_.persist_pairs());
+    if (next) {
+      q.q_codes = next->codes;
+      q.q_scales = next->scales;
+      q.q_divisor = next->divisor;
+    }
     ctx_.count_launch();
-    ctx_.note_route("nvfp4_persist_kernel", gate_up ? 1 : 0, pairs, 1, 1);
-    TK100_TRY(ctx_.check(launch_nvfp4_persist(stream, gate_up, pairs, map_w, map_a, map_wsf, map_asf, q),
-                         "launching the persistent NVFP4 projection"));
-    return quantise_after();
+    ctx_.note_route("nvfp4_persist_kernel", plan.tok_tile, plan.workers, plan.splits, 1);
+    return ctx_.check(launch_pair_gemm(stream, true, gate_up, plan.workers, map_w, map_a, map_wsf, map_asf, q),
+                      "launching the persistent NVFP4 projection");
   }
   // 256-token tiles (one CTA per SM, a third fewer operand bytes and issue slots per MAC) for
   // prefill shapes: the plain projection unsplit, and the gate/up pairs.

@@ -38,11 +38,15 @@ struct Tuning {
   int fp8_pair_min_rows = 256;
   int nvfp4_pair = 0;         // TK100_PAIR: 1 down, 2 gate_up too (cta_group::2 variant)
   int nvfp4_pair_min_rows = 1024;
-  int nvfp4_persist = 0;      // TK100_PERSIST=1: persistent CTA-pair route for NVFP4 prefill shapes
+  int nvfp4_persist = -1;     // TK100_PERSIST: persistent CTA pairs for NVFP4: 0 never, 1 from
+                              // TK100_PERSIST_MIN_ROWS tokens, -1 where the rule of the operator says
   int nvfp4_persist_min_rows = 512;  // TK100_PERSIST_MIN_ROWS
-  int fp8_stream_k = 0;       // TK100_FP8_STREAMK=1: stream-K on resident pairs wherever pairs can run (measured slower)
-  int fp8_persist = 0;        // TK100_FP8_PERSIST=1: persistent CTA pairs with two accumulators for FP8
-                              // prefill shapes of more pair tiles than resident pairs
+  int fp8_stream_k = 0;       // TK100_FP8_STREAMK=1: persistent pairs with K split over the pairs of a
+                              // cluster wherever a split fits
+  int fp8_persist = -1;       // TK100_FP8_PERSIST: persistent CTA pairs for FP8: 0 never, 1 or 2 wherever
+                              // pairs run, K unsplit; -1 where the rule of the operator says
+  int pair_tok = 0;           // TK100_PAIR_TOK: forced token tile of the persistent pairs
+  int pair_splits = 0;        // TK100_PAIR_SPLITS: forced K splits of the persistent pairs
   int nvfp4_wide = 0;         // TK100_NVFP4_WIDE: 256-token tiles (one CTA per SM) for NVFP4 prefill
                               // shapes: 1 down, 2 the gate/up pairs too
   int nvfp4_wide_min_rows = 512;  // TK100_NVFP4_WIDE_MIN_ROWS
@@ -75,9 +79,16 @@ class Context {
   // NVFP4 scale plane as rows of one 512-byte chunk (128 x u32), boxes of 4 chunks, unswizzled.
   Status scale_map(const void* base, uint64_t chunks, CUtensorMap* out);
 
+  // The two planes of a gate/up weight as pair_gemm.cu reads them: code boxes of 128 bytes x (16 gate
+  // rows, 16 up rows) x 4 blocks of 32 outputs, and scale boxes of (16 gate lanes, 16 up lanes) x 4
+  // chunks.  `outputs` = rows of one half.
+  Status swiglu_map(const void* base, uint64_t outputs, uint64_t row_bytes, CUtensorMap* out);
+  Status swiglu_scale_map(const void* base, uint64_t outputs, uint64_t chunks_per_tile, CUtensorMap* out);
+
   const tk100_config& config() const { return config_; }
   int sm_count() const { return sm_count_; }
-  int persist_pairs() const { return persist_pairs_; }
+  // Clusters of `splits` CTA pairs (pair_gemm.cu) that fit the device at once.
+  int pair_clusters(int splits) const { return pair_clusters_[splits]; }
   float* partials() const { return partials_; }
   size_t partial_bytes() const { return partial_bytes_; }
   unsigned int* counters() const { return counters_; }
@@ -109,7 +120,7 @@ class Context {
   Context() = default;
   tk100_config config_{};
   int sm_count_ = 0;
-  int persist_pairs_ = 0;  // CTA pairs of the persistent NVFP4 kernel that fit the device at once
+  int pair_clusters_[kPairGemmMaxSplits + 1] = {};
   float* partials_ = nullptr;
   size_t partial_bytes_ = 0;
   unsigned int* counters_ = nullptr;
