@@ -6,6 +6,7 @@ that is impossible the import fails loudly.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.util
 import os
 
 from . import build as _build
@@ -91,6 +92,7 @@ SIGNATURES = {
 }
 
 _lib = None
+_native = None
 
 
 def library_path() -> str:
@@ -111,3 +113,18 @@ def load() -> C.CDLL:
             fn.argtypes = args
         _lib = lib
     return _lib
+
+
+def native(general):
+    """The compiled launch binding, bound to the loaded library's functions; ``general(name, context,
+    stream, *arguments)`` takes the calls it does not read itself."""
+    global _native
+    if _native is None:
+        lib = load()
+        path = _build.build_binding()
+        spec = importlib.util.spec_from_file_location("tuiskollm_b200._native", path)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        module.bind(lambda name: C.cast(getattr(lib, name), _vp).value, general)
+        _native = module
+    return _native

@@ -4,7 +4,8 @@ Names, argument order and error classes follow the reference
 (``ResidualNormOp::launch_plain/launch_residual``, ``FullAttentionQkvOp::launch``,
 ``GdnInputProjectionOp::launch``, ``LmHeadOp::launch``).  Planes are torch CUDA tensors
 (or raw integer device addresses); BF16 planes may be ``torch.bfloat16`` or ``uint16``/
-``int16`` bit views.  Nothing here computes: every method is one C-ABI call.
+``int16`` bit views.  Nothing here computes: every method is one C-ABI call, the launches of a
+model step through the compiled binding (csrc/binding.cpp), the rest through ctypes.
 """
 from __future__ import annotations
 
@@ -45,6 +46,15 @@ def _stream(stream) -> int:
     return stream.cuda_stream
 
 
+def _launch(name, context, stream, *arguments):
+    """One launch through ctypes: what the compiled binding does for plain arguments, for every form
+    of argument and with the errors of the planes' checks."""
+    fn = getattr(context._lib, name)
+    types = _lib.SIGNATURES[name][1][2:]
+    context.check(fn(context.handle, _stream(stream),
+                     *[_ptr(a) if t is C.c_void_p else a for a, t in zip(arguments, types, strict=True)]))
+
+
 class Context:
     """Owns one ``tk100_ctx`` (one per GPU / rank)."""
 
@@ -52,6 +62,7 @@ class Context:
                  rms_norm_epsilon: float = 1e-6, max_rows: int = 2048,
                  workspace_bytes: int = 0):
         self._lib = _lib.load()
+        self._native = _lib.native(_launch)
         cfg = _lib.Config(_lib.ABI_VERSION, device, hidden, intermediate, rms_norm_epsilon,
                           max_rows, workspace_bytes)
         handle = C.c_void_p()
@@ -113,24 +124,21 @@ class ResidualNormOp:
 
     def launch_plain(self, stream, batch, input, weight, output):
         c = self.ctx
-        c.check(c._lib.tk100_rms_norm(c.handle, _stream(stream), batch, _ptr(input), _ptr(weight),
-                                      _ptr(output)))
+        c._native.tk100_rms_norm(c, stream, batch, input, weight, output)
 
     def launch_residual(self, stream, batch, residual_input, branch, weight, residual_output,
                         normalized_output):
         c = self.ctx
-        c.check(c._lib.tk100_residual_rms_norm(c.handle, _stream(stream), batch,
-                                               _ptr(residual_input), _ptr(branch), _ptr(weight),
-                                               _ptr(residual_output), _ptr(normalized_output)))
+        c._native.tk100_residual_rms_norm(c, stream, batch, residual_input, branch, weight, residual_output,
+                                          normalized_output)
 
     def launch_quantize(self, stream, batch, residual_input, branch, weight, residual_output,
                         normalized_output, activation_codes, activation_scales):
         """Fused producer: (residual add +) RMSNorm + per-token E4M3 quantisation, one kernel."""
         c = self.ctx
-        c.check(c._lib.tk100_residual_rms_norm_quantize(
-            c.handle, _stream(stream), batch, _ptr(residual_input), _ptr(branch), _ptr(weight),
-            _ptr(residual_output), _ptr(normalized_output), _ptr(activation_codes),
-            _ptr(activation_scales)))
+        c._native.tk100_residual_rms_norm_quantize(c, stream, batch, residual_input, branch, weight,
+                                                   residual_output, normalized_output, activation_codes,
+                                                   activation_scales)
 
 
     def launch_quantize_nvfp4(self, stream, batch, residual_input, branch, weight, residual_output,
@@ -138,10 +146,10 @@ class ResidualNormOp:
                               input_global_divisor, nvfp4_codes, nvfp4_scales):
         """Fused producer with both quantised forms: E4M3 (optional) and NVFP4, one kernel."""
         c = self.ctx
-        c.check(c._lib.tk100_residual_rms_norm_quantize_nvfp4(
-            c.handle, _stream(stream), batch, _ptr(residual_input), _ptr(branch), _ptr(weight),
-            _ptr(residual_output), _ptr(normalized_output), _ptr(activation_codes),
-            _ptr(activation_scales), input_global_divisor, _ptr(nvfp4_codes), _ptr(nvfp4_scales)))
+        c._native.tk100_residual_rms_norm_quantize_nvfp4(c, stream, batch, residual_input, branch, weight,
+                                                         residual_output, normalized_output, activation_codes,
+                                                         activation_scales, input_global_divisor, nvfp4_codes,
+                                                         nvfp4_scales)
 
 
 class Fp8ProjectionOp:
@@ -152,17 +160,14 @@ class Fp8ProjectionOp:
 
     def quantize(self, stream, rows, columns, input, activation_codes, activation_scales):
         c = self.ctx
-        c.check(c._lib.tk100_quantize_activation_e4m3(c.handle, _stream(stream), rows, columns,
-                                                      _ptr(input), _ptr(activation_codes),
-                                                      _ptr(activation_scales)))
+        c._native.tk100_quantize_activation_e4m3(c, stream, rows, columns, input, activation_codes,
+                                                 activation_scales)
 
     def launch(self, stream, rows, out_rows, columns, input, activation_codes, activation_scales,
                weight_codes, weight_scales, output):
         c = self.ctx
-        c.check(c._lib.tk100_fp8_projection(c.handle, _stream(stream), rows, out_rows, columns,
-                                            _ptr(input), _ptr(activation_codes),
-                                            _ptr(activation_scales), _ptr(weight_codes),
-                                            _ptr(weight_scales), _ptr(output)))
+        c._native.tk100_fp8_projection(c, stream, rows, out_rows, columns, input, activation_codes,
+                                       activation_scales, weight_codes, weight_scales, output)
 
 
 class FullAttentionQkvOp:
@@ -177,10 +182,9 @@ class FullAttentionQkvOp:
     def launch(self, stream, rows, input, activation_codes, activation_scales, weight_codes,
                weight_scales, output):
         c = self.ctx
-        fn = getattr(c._lib, self._entry)
-        c.check(fn(c.handle, _stream(stream), rows, self.out_rows, _ptr(input),
-                   _ptr(activation_codes), _ptr(activation_scales), _ptr(weight_codes),
-                   _ptr(weight_scales), _ptr(output)))
+        fn = getattr(c._native, self._entry)
+        fn(c, stream, rows, self.out_rows, input, activation_codes, activation_scales, weight_codes,
+           weight_scales, output)
 
 
 class GdnInputProjectionOp(FullAttentionQkvOp):
@@ -201,9 +205,8 @@ class Fp8SwiGluOp:
     def launch(self, stream, rows, input, activation_codes, activation_scales, weight_codes,
                weight_scales, output):
         c = self.ctx
-        fn = getattr(c._lib, self._entry)
-        c.check(fn(c.handle, _stream(stream), rows, _ptr(input), _ptr(activation_codes),
-                   _ptr(activation_scales), _ptr(weight_codes), _ptr(weight_scales), _ptr(output)))
+        fn = getattr(c._native, self._entry)
+        fn(c, stream, rows, input, activation_codes, activation_scales, weight_codes, weight_scales, output)
 
 
 class Fp8DownOp(Fp8SwiGluOp):
@@ -223,9 +226,8 @@ class GdnOutputProjectionOp:
     def launch(self, stream, rows, input, activation_codes, activation_scales, weight_codes,
                weight_scales, output):
         c = self.ctx
-        c.check(c._lib.tk100_fp8_gdn_output(c.handle, _stream(stream), rows, self.columns, _ptr(input),
-                                            _ptr(activation_codes), _ptr(activation_scales),
-                                            _ptr(weight_codes), _ptr(weight_scales), _ptr(output)))
+        c._native.tk100_fp8_gdn_output(c, stream, rows, self.columns, input, activation_codes,
+                                       activation_scales, weight_codes, weight_scales, output)
 
 
 class Materializer:
@@ -340,10 +342,8 @@ class GdnPrepareOp:
     def launch(self, stream, batch, input, control_weights, a_log, dt_bias, projected,
                convolution_weights, state_rows, history, log_decay, beta, convolved):
         c = self.ctx
-        c.check(c._lib.tk100_gdn_prepare(
-            c.handle, _stream(stream), batch, _ptr(input), _ptr(control_weights), _ptr(a_log),
-            _ptr(dt_bias), _ptr(projected), _ptr(convolution_weights), _ptr(state_rows),
-            _ptr(history), _ptr(log_decay), _ptr(beta), _ptr(convolved)))
+        c._native.tk100_gdn_prepare(c, stream, batch, input, control_weights, a_log, dt_bias, projected,
+                                    convolution_weights, state_rows, history, log_decay, beta, convolved)
 
 
 class GdnRecurrenceOp:
@@ -356,9 +356,8 @@ class GdnRecurrenceOp:
     def launch(self, stream, batch, qkv, projected, log_decay, beta, norm_weight, state_rows,
                state, output):
         c = self.ctx
-        c.check(c._lib.tk100_gdn_recurrence(
-            c.handle, _stream(stream), batch, _ptr(qkv), _ptr(projected), _ptr(log_decay),
-            _ptr(beta), _ptr(norm_weight), _ptr(state_rows), _ptr(state), _ptr(output)))
+        c._native.tk100_gdn_recurrence(c, stream, batch, qkv, projected, log_decay, beta, norm_weight,
+                                       state_rows, state, output)
 
 
 class LmHeadOp:
@@ -374,11 +373,9 @@ class LmHeadOp:
     def launch(self, stream, rows, input, activation_codes, activation_scales, weight_codes,
                weight_scales, output, logits_f32=None, argmax_scratch=None, pairs=None):
         c = self.ctx
-        c.check(c._lib.tk100_fp8_lm_head(c.handle, _stream(stream), rows, self.vocab_rows,
-                                         self.vocab_offset, _ptr(input), _ptr(activation_codes),
-                                         _ptr(activation_scales), _ptr(weight_codes),
-                                         _ptr(weight_scales), _ptr(output), _ptr(logits_f32),
-                                         _ptr(argmax_scratch), _ptr(pairs)))
+        c._native.tk100_fp8_lm_head(c, stream, rows, self.vocab_rows, self.vocab_offset, input,
+                                    activation_codes, activation_scales, weight_codes, weight_scales, output,
+                                    logits_f32, argmax_scratch, pairs)
 
     def launch_sharded(self, stream, rows, input, activation_codes, activation_scales, weight_codes,
                        weight_scales, output, logits_f32, argmax_scratch, world, rank, peer_buffers,
@@ -422,18 +419,16 @@ class _Nvfp4Op:
                  activation_scales):
         """NVFP4 activation quantiser (this library's own definition; see the header)."""
         c = self.ctx
-        c.check(c._lib.tk100_nvfp4_quantize_activation(
-            c.handle, _stream(stream), rows, columns, _ptr(input), input_global_divisor,
-            _ptr(activation_codes), _ptr(activation_scales)))
+        c._native.tk100_nvfp4_quantize_activation(c, stream, rows, columns, input, input_global_divisor,
+                                                  activation_codes, activation_scales)
 
     def launch(self, stream, batch, input, weight_codes, weight_scales, weight_scale_divisor,
                output, *, activation_codes, activation_scales, input_global_divisor):
         """The reference's argument order, followed by the W4A4 additions as keywords."""
         c = self.ctx
-        fn = getattr(c._lib, self._entry)
-        c.check(fn(c.handle, _stream(stream), batch, _ptr(input), _ptr(activation_codes),
-                   _ptr(activation_scales), input_global_divisor, _ptr(weight_codes),
-                   _ptr(weight_scales), weight_scale_divisor, _ptr(output)))
+        fn = getattr(c._native, self._entry)
+        fn(c, stream, batch, input, activation_codes, activation_scales, input_global_divisor, weight_codes,
+           weight_scales, weight_scale_divisor, output)
 
 
 class Nvfp4SwiGluOp(_Nvfp4Op):
@@ -447,11 +442,10 @@ class Nvfp4SwiGluOp(_Nvfp4Op):
         """The same projection, also leaving the NVFP4 codes and block scales of its output for
         ``Nvfp4DownOp.launch(input=None, ...)`` (in the projection's epilogue up to 32 rows)."""
         c = self.ctx
-        c.check(c._lib.tk100_nvfp4_gate_up_swiglu_quantize(
-            c.handle, _stream(stream), batch, _ptr(input), _ptr(activation_codes),
-            _ptr(activation_scales), input_global_divisor, _ptr(weight_codes),
-            _ptr(weight_scales), weight_scale_divisor, _ptr(output), output_global_divisor,
-            _ptr(output_codes), _ptr(output_scales)))
+        c._native.tk100_nvfp4_gate_up_swiglu_quantize(c, stream, batch, input, activation_codes,
+                                                      activation_scales, input_global_divisor, weight_codes,
+                                                      weight_scales, weight_scale_divisor, output,
+                                                      output_global_divisor, output_codes, output_scales)
 
 
 class Nvfp4DownOp(_Nvfp4Op):
@@ -464,10 +458,9 @@ class Nvfp4DownOp(_Nvfp4Op):
                        activation_scales, input_global_divisor):
         """Row-parallel shard: unrounded fp32 partial sums for a later all-reduce."""
         c = self.ctx
-        c.check(c._lib.tk100_nvfp4_down_partial(
-            c.handle, _stream(stream), batch, _ptr(input), _ptr(activation_codes),
-            _ptr(activation_scales), input_global_divisor, _ptr(weight_codes),
-            _ptr(weight_scales), weight_scale_divisor, _ptr(partial_output)))
+        c._native.tk100_nvfp4_down_partial(c, stream, batch, input, activation_codes, activation_scales,
+                                           input_global_divisor, weight_codes, weight_scales,
+                                           weight_scale_divisor, partial_output)
 
 
 def f32_to_bf16(context: Context, stream, count, input, output):
