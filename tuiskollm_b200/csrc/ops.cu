@@ -1189,7 +1189,7 @@ Status Nvfp4MlpOp::launch(cudaStream_t stream, bool gate_up, int rows, int out_r
   const Tuning& tune = ctx_.tuning();
   const bool pairs_chosen = tune.nvfp4_persist > 0 ? rows >= tune.nvfp4_persist_min_rows
                                                    : tune.nvfp4_persist < 0 && rows >= kPairMinRows;
-  if (pairs_chosen && tune.cluster == 3 && tune.swiglu_pairs != 0 && tune.nvfp4_wide == 0 &&
+  if (pairs_chosen && tune.cluster == 3 && tune.swiglu_pairs < 0 && tune.nvfp4_wide == 0 &&
       ctx_.forced_splits() == 0) {
     const int row_units = gate_up ? out_rows / 128 : (out_rows + 255) / 256;
     const uint64_t w_rows = static_cast<uint64_t>(out_rows) * (gate_up ? 2 : 1);

@@ -50,7 +50,8 @@ struct Tuning {
   int nvfp4_wide = 0;         // TK100_NVFP4_WIDE: 256-token tiles (one CTA per SM) for NVFP4 prefill
                               // shapes: 1 down, 2 the gate/up pairs too
   int nvfp4_wide_min_rows = 512;  // TK100_NVFP4_WIDE_MIN_ROWS
-  int swiglu_pairs = 1;       // TK100_SWIGLU_PAIRS=0: one CTA holds the gate and the up tile
+  int swiglu_pairs = -1;      // TK100_SWIGLU_PAIRS=0: one CTA holds the gate and the up tile, 1: a CTA
+                              // each; at every token count (-1: persistent pairs for large launches)
   int fused_exchange = 1;     // TK100_FUSED_TAIL=0: argmax finalize / exchange as launches of their own
   int argmax_spread = 1;      // TK100_ARGMAX_SPREAD=0: every CTA's maxima go straight to the caller's keys
   int fused_quant = 0;        // TK100_FUSED_QUANT=1: launches of one wave and at most 4 rows quantise
