@@ -151,3 +151,26 @@ def test_nvfp4_mlp(tk, oracle, monkeypatch, hidden, inter, rows, tok, splits):
     assert np.array_equal(oracle.f32_to_bf16(got32), got)
     for plane in (mid, out, part):
         assert_inactive_untouched(plane, rows)
+
+
+def test_quantised_output_planes_are_held_to_the_quantisers_alignment(tk):
+    """More than 32 rows: what the quantiser launch refuses, the epilogue's quantisation refuses."""
+    rows, hidden, inter = 40, 256, 256
+    c = tk.Context(device=0, hidden=hidden, intermediate=inter)
+    codes, scales = _nvfp4_planes(tk, rows, hidden)
+    w = torch.zeros((2 * inter, hidden // 2), dtype=torch.uint8, device="cuda")
+    ws = torch.zeros((tk.ops.nvfp4_scale_plane_bytes(2 * inter, hidden),), dtype=torch.uint8, device="cuda")
+    mid = torch.zeros((rows * inter + 8,), dtype=torch.bfloat16, device="cuda")
+    m_codes = torch.zeros((rows * inter // 2 + 16,), dtype=torch.uint8, device="cuda")
+    m_scales = torch.zeros((tk.ops.nvfp4_scale_plane_bytes(rows, inter) + 16,), dtype=torch.uint8, device="cuda")
+    op = tk.Nvfp4SwiGluOp(c)
+    for planes in ((mid[8:], m_codes, m_scales), (mid, m_codes[16:], m_scales), (mid, m_codes, m_scales[16:])):
+        with pytest.raises(tk.GpuError) as info:
+            op.launch_quantize(None, rows, None, w, ws, 1.0, planes[0], activation_codes=codes, activation_scales=scales,
+                               input_global_divisor=1.0, output_global_divisor=1.0, output_codes=planes[1],
+                               output_scales=planes[2])
+        assert info.value.code == "gpu.launch"
+    op.launch_quantize(None, rows, None, w, ws, 1.0, mid, activation_codes=codes, activation_scales=scales,
+                       input_global_divisor=1.0, output_global_divisor=1.0, output_codes=m_codes, output_scales=m_scales)
+    torch.cuda.synchronize()
+    assert c.last_kernel.startswith("nvfp4_persist_kernel") and c.device_status() == 0

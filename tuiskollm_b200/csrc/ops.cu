@@ -1212,6 +1212,11 @@ Status Nvfp4MlpOp::launch(cudaStream_t stream, bool gate_up, int rows, int out_r
     q.out = output;
     q.out_f32 = output_f32;
     if (next) {
+      // the planes the quantiser launch of the other routes takes at these sizes, and no others
+      const char* quantiser = "NVFP4 activation quantiser";
+      TK100_TRY(check_plane(ctx_, quantiser, "input", output, 32));
+      TK100_TRY(check_plane(ctx_, quantiser, "activation codes", next->codes, 128));
+      TK100_TRY(check_plane(ctx_, quantiser, "activation scales", next->scales, 128));
       q.q_codes = next->codes;
       q.q_scales = next->scales;
       q.q_divisor = next->divisor;
