@@ -201,3 +201,39 @@ def test_rejected_launches_report_gpu_launch(tk, ctx):
     with pytest.raises(tk.GpuError) as info:
         tk.Context(device=99)
     assert info.value.code == "gpu.context"
+
+
+@pytest.mark.parametrize("cols,rows", [(256, 64), (5120, 3), (5120, 500)])
+def test_quotients_of_every_scale_round_as_the_division(tk, oracle, cols, rows):
+    """E4M3 and NVFP4 codes come from residual steps on one reciprocal per row or block: rows whose scale
+    runs through the whole BF16 range (the E4M3 route leaves the reciprocal for the division below 2^-80),
+    quotients on the rounding boundaries, signed zeros, and a NaN that must not disturb its neighbours."""
+    rng = np.random.default_rng(cols + rows)
+    exps = rng.integers(-130, 120, rows)
+    x = rng.standard_normal((rows, cols)) * np.exp2(exps.astype(np.float64))[:, None]
+    # small integers over a power of two: quotients that are, or are next to, halves of a code step
+    grid = rows // 2
+    x[:grid] = rng.integers(-28, 29, (grid, cols)) * np.exp2(exps[:grid].astype(np.float64))[:, None] / 4
+    x[:, 5::16] = np.where(rng.random(x[:, 5::16].shape) < 0.5, 0.0, -0.0)
+    bits = oracle.f32_to_bf16(np.clip(x, -3e38, 3e38).astype(np.float32))
+    codes, scales = (torch.zeros((rows, cols), dtype=torch.uint8, device="cuda"),
+                     torch.zeros((rows,), dtype=torch.float32, device="cuda"))
+    c = tk.Context(device=0)
+    op = tk.ops.Fp8ProjectionOp(c)
+    op.quantize(None, rows, cols, dev(bits.view(np.int16)), codes, scales)
+    oc, os_ = oracle.quantize_e4m3(bits)
+    assert np.array_equal(host(scales), os_) and np.array_equal(host(codes), oc)
+    c4 = torch.zeros((rows, cols // 2), dtype=torch.uint8, device="cuda")
+    s4 = torch.zeros((tk.ops.nvfp4_scale_plane_bytes(rows, cols),), dtype=torch.uint8, device="cuda")
+    for divisor in (1.0, 448.0, 448.0 * 6.0 / 5.0):
+        tk.Nvfp4SwiGluOp(c).quantize(None, rows, cols, dev(bits.view(np.int16)), divisor, c4, s4)
+        qc, qs = oracle.nvfp4_quantize(bits, float(np.float32(divisor)))
+        assert np.array_equal(host(c4), qc) and np.array_equal(host(s4), qs), divisor
+    assert c.device_status() == 0
+    bits[:, 7] = 0x7FC0
+    op.quantize(None, rows, cols, dev(bits.view(np.int16)), codes, scales)
+    clean = bits.copy()
+    clean[:, 7] = 0
+    oc, os_ = oracle.quantize_e4m3(clean)
+    oc[:, 7] = 0x7F
+    assert np.array_equal(host(scales), os_) and np.array_equal(host(codes), oc)

@@ -24,7 +24,50 @@ __device__ __forceinline__ uint32_t f32_to_bf16_bits(float v) {
 }
 
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
-  return f32_to_bf16_bits(lo) | (f32_to_bf16_bits(hi) << 16);
+  uint32_t w;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(w) : "f"(hi), "f"(lo));
+  return w;
+}
+
+// Two fp32 values in a 64-bit register; each operation is the IEEE one on both halves, in one issue slot.
+using F32x2 = unsigned long long;
+__device__ __forceinline__ F32x2 f32x2(float lo, float hi) {
+  F32x2 v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+  return v;
+}
+__device__ __forceinline__ F32x2 f32x2_splat(float v) { return f32x2(v, v); }
+__device__ __forceinline__ F32x2 bf16x2_to_f32x2(uint32_t w) { return f32x2(bf16x2_lo(w), bf16x2_hi(w)); }
+__device__ __forceinline__ float2 f32x2_parts(F32x2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ F32x2 add2(F32x2 a, F32x2 b) {
+  F32x2 v;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+  return v;
+}
+__device__ __forceinline__ F32x2 mul2(F32x2 a, F32x2 b) {
+  F32x2 v;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+  return v;
+}
+__device__ __forceinline__ F32x2 fma2(F32x2 a, F32x2 b, F32x2 c) {
+  F32x2 v;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(a), "l"(b), "l"(c));
+  return v;
+}
+__device__ __forceinline__ uint32_t f32x2_to_bf16x2(F32x2 v) {
+  const float2 f = f32x2_parts(v);
+  return pack_bf16x2(f.x, f.y);
+}
+
+// max(|.|) of two packed BF16 pairs, NaNs ignored as by fmaxf (`acc` starts at 0).
+__device__ __forceinline__ uint32_t bf16x2_absmax(uint32_t acc, uint32_t w) {
+  uint32_t r;
+  asm("max.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(acc), "r"(w & 0x7fff7fffu));
+  return r;
 }
 
 // Two f32 -> two E4M3FN codes, round-to-nearest-even, saturating to +-448
@@ -64,43 +107,73 @@ __device__ __forceinline__ float silu_fp8_path(float v) {
   return __fdividef(v, 1.0f + ex);
 }
 
-// t / s for a NVFP4 block: s is a decoded E4M3 scale (4 significant bits), inv = __frcp_rn(s).  One
-// residual step on the reciprocal's product (P. Markstein, "Computation of elementary functions on the
-// IBM RISC System/6000 processor", IBM J. Res. Dev. 34 (1990), theorem on the corrected quotient)
-// rounds like the division wherever an E2M1 code depends on it; quotients below the first rounding
-// boundary (signed zeros among them), past the saturation point, infinities and NaNs keep the product.
-__device__ __forceinline__ float nvfp4_quotient(float t, float s, float inv) {
-  const float q = __fmul_rn(t, inv);
-  const float corrected = __fmaf_rn(__fmaf_rn(-q, s, t), inv, q);
-  return (fabsf(q) > 0.125f && fabsf(q) < 8.0f) ? corrected : q;
+// x / s by a residual step on the product with the correctly rounded reciprocal (P. Markstein, "Computation
+// of elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34 (1990)).  Operands
+// come negated: `negative` = -x, ninv = -__frcp_rn(s); that keeps the sign of a zero quotient, which the
+// residual of the plain form (0 - 0) would lose.  One step lands within one unit in the last place and
+// exactly on every quotient that fp32 holds; a second one rounds like the division.
+__device__ __forceinline__ F32x2 quotient_step(F32x2 q, F32x2 negative, F32x2 s, F32x2 ninv) {
+  return fma2(fma2(q, s, negative), ninv, q);
+}
+
+// E4M3 codes of a packed BF16 pair divided by `scale` (e4m3_rn_satfinite of the IEEE quotient).  Two
+// residual steps; they need a scale whose residuals stay in the normal range (e4m3_scale_is_ordinary).
+__device__ __forceinline__ bool e4m3_scale_is_ordinary(float scale) { return scale >= 0x1p-80f && scale <= 0x1p120f; }
+__device__ __forceinline__ uint32_t e4m3_pair_ordinary(uint32_t w, F32x2 scale, F32x2 ninv) {
+  const F32x2 n = bf16x2_to_f32x2(w ^ 0x80008000u);
+  const float2 q = f32x2_parts(quotient_step(quotient_step(mul2(n, ninv), n, scale, ninv), n, scale, ninv));
+  return f32x2_to_e4m3x2(q.x, q.y);
+}
+__device__ __forceinline__ uint32_t e4m3_pair(uint32_t w, float scale) {
+  return f32x2_to_e4m3x2(__fdiv_rn(bf16x2_lo(w), scale), __fdiv_rn(bf16x2_hi(w), scale));
+}
+
+// NVFP4 codes of N packed BF16 pairs of one block: code = e2m1_rne_sat((x * divisor) / s), signed zeros
+// when s == 0; two codes a byte, low nibble first.  s is a decoded E4M3 scale (4 significant bits) and an
+// E2M1 rounding boundary has 3, so a quotient is on a boundary exactly or more than 1.007 half units in
+// the last place away from it: one residual step decides every code as the division does.  An infinite
+// product keeps the division (its residual is NaN).
+template <int N>
+__device__ __forceinline__ void nvfp4_codes(const uint32_t (&w)[N], float block_max, float divisor, float s,
+                                            uint32_t (&packed)[N / 4]) {
+#pragma unroll
+  for (int j = 0; j < N / 4; ++j) packed[j] = 0u;
+  if (s == 0.0f) {
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      const uint32_t byte = ((w[j] & 0x8000u) ? 0x08u : 0u) | ((w[j] & 0x80000000u) ? 0x80u : 0u);
+      packed[j >> 2] |= byte << (8 * (j & 3));
+    }
+  } else if (__fmul_rn(block_max, divisor) <= 3.0e38f) {
+    const F32x2 ndiv = f32x2_splat(-divisor), ninv = f32x2_splat(-__frcp_rn(s)), s2 = f32x2_splat(s);
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      const F32x2 n = mul2(bf16x2_to_f32x2(w[j]), ndiv);
+      const float2 q = f32x2_parts(quotient_step(mul2(n, ninv), n, s2, ninv));
+      packed[j >> 2] |= (f32x2_to_e2m1x2(q.x, q.y) & 0xffu) << (8 * (j & 3));
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      const uint32_t byte = f32x2_to_e2m1x2(__fdiv_rn(__fmul_rn(bf16x2_lo(w[j]), divisor), s),
+                                            __fdiv_rn(__fmul_rn(bf16x2_hi(w[j]), divisor), s));
+      packed[j >> 2] |= (byte & 0xffu) << (8 * (j & 3));
+    }
+  }
 }
 
 // NVFP4 form of 16 consecutive BF16 values (8 packed pairs, low half first):
 //   scale = e4m3_rne_sat((amax * divisor) / 6),  code = e2m1_rne_sat((x * divisor) / scale),
 // signed zeros when the scale underflows to 0.  Codes low nibble first.
 __device__ __forceinline__ uint2 nvfp4_quantize_block(const uint32_t (&w)[8], float divisor, uint32_t* scale_code) {
-  float amax = 0.0f;
+  uint32_t m = 0u;
 #pragma unroll
-  for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fmaxf(fabsf(bf16x2_lo(w[j])), fabsf(bf16x2_hi(w[j]))));
+  for (int j = 0; j < 8; ++j) m = bf16x2_absmax(m, w[j]);
+  const float amax = fmaxf(bf16x2_lo(m), bf16x2_hi(m));
   const uint32_t sc = f32x2_to_e4m3x2(__fdiv_rn(__fmul_rn(amax, divisor), 6.0f), 0.0f) & 0xffu;
   *scale_code = sc;
-  const float s = e4m3_to_f32(sc);
-  uint32_t packed[2] = {0u, 0u};
-  if (s == 0.0f) {
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const uint32_t byte = ((w[j] & 0x8000u) ? 0x08u : 0u) | ((w[j] & 0x80000000u) ? 0x80u : 0u);
-      packed[j >> 2] |= byte << (8 * (j & 3));
-    }
-  } else {
-    const float inv = __frcp_rn(s);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const uint32_t byte = f32x2_to_e2m1x2(nvfp4_quotient(__fmul_rn(bf16x2_lo(w[j]), divisor), s, inv),
-                                            nvfp4_quotient(__fmul_rn(bf16x2_hi(w[j]), divisor), s, inv)) & 0xffu;
-      packed[j >> 2] |= byte << (8 * (j & 3));
-    }
-  }
+  uint32_t packed[2];
+  nvfp4_codes(w, amax, divisor, e4m3_to_f32(sc), packed);
   return make_uint2(packed[0], packed[1]);
 }
 

@@ -7,12 +7,18 @@
 // (tuisko-kernels-sm120/src/residual_norm.rs:155-226 followed by
 // tuisko-kernels-sm120/src/device/fp8_projection.rs:54-126).
 //
+// Reading and writing a row's 48 KB bounds it from a few hundred rows up (2048 rows with both quantised
+// forms: 98 MB, 15.3 us at the copy rate); below that its chain of two block reductions does.  With an
+// IEEE divide per value and code and unpacked fp32 rows, instruction issue came first: fp32 pairs, BF16
+// rows kept packed and quotients from one reciprocal per row or block took 2048 rows from 31.7 to
+// 23.9 us, 512 from 11.3 to 8.7, one row from 3.8 to 3.0.
+//
 // Numeric contract (bit-exact parts marked *):
 //   res  = bf16_rn(f32(x) + f32(branch))                                  *
 //   r    = 1/sqrt(sum(res^2)/H + eps), fp32, fixed summation order
 //   y    = bf16_rn(res * r * (1 + w)), evaluated left to right in fp32
 //   amax = max |y|; scale = amax == 0 ? 1 : amax / 448   (IEEE fp32 divide)   *
-//   code = e4m3_rn_satfinite(y / scale)                  (IEEE fp32 divide)   *
+//   code = e4m3_rn_satfinite(y / scale)                  (IEEE fp32 quotient) *
 // The starred results are bit-exact functions of their inputs; `codes`/`scale`
 // are exact with respect to the normalised row this same kernel wrote.
 #include <cstdlib>
@@ -52,13 +58,13 @@ __global__ void __launch_bounds__(1024)
   const int chunks_per_row = hidden >> 3;
   const size_t row_off = static_cast<size_t>(row) * hidden;
 
-  float v[CHUNKS][8];
+  uint32_t v[CHUNKS][4];  // the row as packed BF16 pairs: rounded residual, later the normalised row
   // The norm weight of this thread's columns is requested together with the row (one memory
   // latency less on the chain load -> reduce -> scale -> reduce -> store); with three or four
   // chunks per thread the registers do not allow it and the weight is loaded where it is used.
   constexpr bool EARLY_WEIGHT = DO_NORM && CHUNKS <= 2;
   Chunk wreg[EARLY_WEIGHT ? CHUNKS : 1];
-  float sum = 0.0f;
+  F32x2 sum = f32x2_splat(0.0f);
 #pragma unroll
   for (int i = 0; i < CHUNKS; ++i) {
     const int c = threadIdx.x + i * blockDim.x;
@@ -69,34 +75,31 @@ __global__ void __launch_bounds__(1024)
         Chunk b = *reinterpret_cast<const Chunk*>(branch + row_off + c * 8);
         Chunk r;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float lo = __fadd_rn(bf16x2_lo(a.w[j]), bf16x2_lo(b.w[j]));
-          const float hi = __fadd_rn(bf16x2_hi(a.w[j]), bf16x2_hi(b.w[j]));
-          r.w[j] = pack_bf16x2(lo, hi);
-        }
+        for (int j = 0; j < 4; ++j) r.w[j] = f32x2_to_bf16x2(add2(bf16x2_to_f32x2(a.w[j]), bf16x2_to_f32x2(b.w[j])));
         *reinterpret_cast<Chunk*>(residual_out + row_off + c * 8) = r;
         a = r;  // the norm consumes the rounded residual
       }
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        v[i][2 * j] = bf16x2_lo(a.w[j]);
-        v[i][2 * j + 1] = bf16x2_hi(a.w[j]);
-      }
+      for (int j = 0; j < 4; ++j) v[i][j] = a.w[j];
       if (DO_NORM) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) sum = __fmaf_rn(v[i][j], v[i][j], sum);
+        for (int j = 0; j < 4; ++j) {
+          const F32x2 f = bf16x2_to_f32x2(v[i][j]);
+          sum = fma2(f, f, sum);
+        }
       }
     } else {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) v[i][j] = 0.0f;
+      for (int j = 0; j < 4; ++j) v[i][j] = 0u;
     }
   }
 
-  float amax = 0.0f;
   if (DO_NORM) {
-    sum = block_reduce<false>(sum, scratch);
-    const float mean = __fdiv_rn(sum, static_cast<float>(hidden));
-    const float inv_rms = __frsqrt_rn(__fadd_rn(mean, eps));
+    const float2 halves = f32x2_parts(sum);
+    const float total = block_reduce<false>(__fadd_rn(halves.x, halves.y), scratch);
+    const float mean = __fdiv_rn(total, static_cast<float>(hidden));
+    const F32x2 inv_rms = f32x2_splat(__frsqrt_rn(__fadd_rn(mean, eps)));
+    const F32x2 one = f32x2_splat(1.0f);
 #pragma unroll
     for (int i = 0; i < CHUNKS; ++i) {
       const int c = threadIdx.x + i * blockDim.x;
@@ -107,13 +110,9 @@ __global__ void __launch_bounds__(1024)
         Chunk o;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const float lo = __fmul_rn(__fmul_rn(v[i][2 * j], inv_rms),
-                                     __fadd_rn(1.0f, bf16x2_lo(wv.w[j])));
-          const float hi = __fmul_rn(__fmul_rn(v[i][2 * j + 1], inv_rms),
-                                     __fadd_rn(1.0f, bf16x2_hi(wv.w[j])));
-          o.w[j] = pack_bf16x2(lo, hi);
-          v[i][2 * j] = bf16x2_lo(o.w[j]);  // keep the rounded value for the quantiser
-          v[i][2 * j + 1] = bf16x2_hi(o.w[j]);
+          o.w[j] = f32x2_to_bf16x2(mul2(mul2(bf16x2_to_f32x2(v[i][j]), inv_rms),
+                                        add2(one, bf16x2_to_f32x2(wv.w[j]))));
+          v[i][j] = o.w[j];  // keep the rounded value for the quantiser
         }
         *reinterpret_cast<Chunk*>(normalized_out + row_off + c * 8) = o;
       }
@@ -127,27 +126,17 @@ __global__ void __launch_bounds__(1024)
 #pragma unroll
     for (int i = 0; i < CHUNKS; ++i) {
       const int c = threadIdx.x + i * blockDim.x;  // chunk index; block g = c / 2
-      float bmax = 0.0f;
+      uint32_t m = 0u;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) bmax = fmaxf(bmax, fabsf(v[i][j]));
+      for (int j = 0; j < 4; ++j) m = bf16x2_absmax(m, v[i][j]);
+      float bmax = fmaxf(bf16x2_lo(m), bf16x2_hi(m));
       bmax = fmaxf(bmax, __shfl_xor_sync(0xffffffffu, bmax, 1));
       if (c < chunks_per_row) {
         const float raw = __fdiv_rn(__fmul_rn(bmax, nv.divisor), 6.0f);
         const uint32_t sc = f32x2_to_e4m3x2(raw, 0.0f) & 0xffu;
-        const float sd = e4m3_to_f32(sc);
-        uint32_t packed = 0u;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          uint32_t byte;
-          if (sd == 0.0f) {
-            byte = (signbit(v[i][2 * j]) ? 0x08u : 0u) | (signbit(v[i][2 * j + 1]) ? 0x80u : 0u);
-          } else {
-            byte = f32x2_to_e2m1x2(__fdiv_rn(__fmul_rn(v[i][2 * j], nv.divisor), sd),
-                                   __fdiv_rn(__fmul_rn(v[i][2 * j + 1], nv.divisor), sd)) & 0xffu;
-          }
-          packed |= byte << (8 * j);
-        }
-        *reinterpret_cast<uint32_t*>(nv.codes + static_cast<size_t>(row) * (hidden >> 1) + c * 4) = packed;
+        uint32_t packed[1];
+        nvfp4_codes(v[i], bmax, nv.divisor, e4m3_to_f32(sc), packed);
+        *reinterpret_cast<uint32_t*>(nv.codes + static_cast<size_t>(row) * (hidden >> 1) + c * 4) = packed[0];
         if ((c & 1) == 0) {
           const int g = c >> 1;
           const size_t off = (static_cast<size_t>(row >> 7) * (groups >> 2) + (g >> 2)) * 512 +
@@ -159,29 +148,33 @@ __global__ void __launch_bounds__(1024)
   }
 
   if (DO_QUANT) {
+    uint32_t m = 0u;
 #pragma unroll
     for (int i = 0; i < CHUNKS; ++i) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(v[i][j]));
+      for (int j = 0; j < 4; ++j) m = bf16x2_absmax(m, v[i][j]);
     }
-    amax = block_reduce<true>(amax, scratch);
+    const float amax = block_reduce<true>(fmaxf(bf16x2_lo(m), bf16x2_hi(m)), scratch);
     if (!(amax <= 3.0e38f) && threadIdx.x == 0) atomicOr(status, STATUS_NONFINITE_INPUT);
     const float scale = (amax == 0.0f) ? 1.0f : __fdiv_rn(amax, 448.0f);
     if (threadIdx.x == 0) scales[row] = scale;
+    auto store_codes = [&](auto&& pair) {
 #pragma unroll
-    for (int i = 0; i < CHUNKS; ++i) {
-      const int c = threadIdx.x + i * blockDim.x;
-      if (c < chunks_per_row) {
-        uint32_t q[4];
+      for (int i = 0; i < CHUNKS; ++i) {
+        const int c = threadIdx.x + i * blockDim.x;
+        if (c < chunks_per_row) {
+          uint32_t q[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          q[j] = f32x2_to_e4m3x2(__fdiv_rn(v[i][2 * j], scale), __fdiv_rn(v[i][2 * j + 1], scale));
+          for (int j = 0; j < 4; ++j) q[j] = pair(v[i][j]);
+          *reinterpret_cast<uint2*>(codes + row_off + c * 8) = make_uint2(q[0] | (q[1] << 16), q[2] | (q[3] << 16));
         }
-        uint2 packed;
-        packed.x = q[0] | (q[1] << 16);
-        packed.y = q[2] | (q[3] << 16);
-        *reinterpret_cast<uint2*>(codes + row_off + c * 8) = packed;
       }
+    };
+    if (e4m3_scale_is_ordinary(scale)) {
+      const F32x2 scale2 = f32x2_splat(scale), ninv = f32x2_splat(-__frcp_rn(scale));
+      store_codes([&](uint32_t w) { return e4m3_pair_ordinary(w, scale2, ninv); });
+    } else {
+      store_codes([&](uint32_t w) { return e4m3_pair(w, scale); });
     }
   }
 }
@@ -258,11 +251,12 @@ cudaError_t launch_resnorm_quant(cudaStream_t stream, int rows, int hidden, cons
   const Nvfp4Out nv{nvfp4_codes, nvfp4_scales, nvfp4_divisor};
   int threads = 0, chunks = 0;
   if (!norm_geometry(hidden, &threads, &chunks)) return cudaErrorInvalidValue;
-  // A row per CTA: with one 16-byte chunk per thread (640 threads for 5120 columns) three CTAs
-  // share an SM, so 256 or 512 rows run as one and a bit, or two, waves of CTAs that each sit
-  // through two block reductions.  More chunks per thread = smaller CTAs = more rows in flight per
-  // SM: take the fewest chunks that put all rows into one wave, the most when none does.
-  {
+  // A row per CTA: with one 16-byte chunk per thread (640 threads for 5120 columns) three CTAs share an
+  // SM, and rows beyond that wave run better on CTAs of half the threads and twice the chunks, more of
+  // which are in different phases at once.  One / two / four chunks, 5120 columns with both quantised
+  // forms: 301 rows 7.3 / 7.7 / 9.4 us, 512 rows 9.4 / 8.7 / 11.8, 1200 rows 17.2 / 16.0 / 19.1, 2048
+  // rows 25.7 / 23.9 / 25.6; two / four chunks, quantiser alone on 1024 rows of 6144: 4.8 / 4.3 us.
+  if (chunks <= 2) {
     static int sms = 0;
     if (sms == 0) {
       int device = 0;
@@ -271,13 +265,10 @@ cudaError_t launch_resnorm_quant(cudaStream_t stream, int rows, int hidden, cons
         sms = 148;
       }
     }
-    const int row_chunks = hidden >> 3;
-    while (chunks * 2 <= kMaxChunks && rows > sms * (2048 / threads)) {
-      const int c = chunks * 2;
-      const int t = ((row_chunks + c - 1) / c + 31) & ~31;
-      if (t < 128) break;
-      chunks = c;
-      threads = t;
+    const int half = (((hidden >> 3) + 2 * chunks - 1) / (2 * chunks) + 31) & ~31;
+    if (rows > sms * (2048 / threads) && half >= 128) {
+      chunks *= 2;
+      threads = half;
     }
   }
   const bool has_branch = branch != nullptr;

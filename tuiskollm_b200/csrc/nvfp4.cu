@@ -700,31 +700,8 @@ __global__ void __launch_bounds__(256)
     const uint4* src = reinterpret_cast<const uint4*>(x + static_cast<size_t>(r) * k + g * 16);
     const uint4 a = src[0], b = src[1];
     const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-    float v[16];
-    float amax = 0.0f;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      v[2 * j] = bf16x2_lo(w[j]);
-      v[2 * j + 1] = bf16x2_hi(w[j]);
-      amax = fmaxf(amax, fmaxf(fabsf(v[2 * j]), fabsf(v[2 * j + 1])));
-    }
-    const float raw = __fdiv_rn(__fmul_rn(amax, divisor), 6.0f);
-    const uint32_t sc = f32x2_to_e4m3x2(raw, 0.0f) & 0xffu;
-    const float s = e4m3_to_f32(sc);
-    uint32_t packed[2] = {0u, 0u};
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      uint32_t byte;
-      if (s == 0.0f) {
-        byte = (signbit(v[2 * j]) ? 0x08u : 0u) | (signbit(v[2 * j + 1]) ? 0x80u : 0u);
-      } else {
-        byte = f32x2_to_e2m1x2(__fdiv_rn(__fmul_rn(v[2 * j], divisor), s),
-                               __fdiv_rn(__fmul_rn(v[2 * j + 1], divisor), s)) & 0xffu;
-      }
-      packed[j >> 2] |= byte << (8 * (j & 3));
-    }
-    *reinterpret_cast<uint2*>(codes + static_cast<size_t>(r) * (k >> 1) + g * 8) =
-        make_uint2(packed[0], packed[1]);
+    uint32_t sc;
+    *reinterpret_cast<uint2*>(codes + static_cast<size_t>(r) * (k >> 1) + g * 8) = nvfp4_quantize_block(w, divisor, &sc);
     const size_t off = (static_cast<size_t>(r >> 7) * (groups >> 2) + (g >> 2)) * 512 +
                        static_cast<size_t>(r & 31) * 16 + ((r & 127) >> 5) * 4 + (g & 3);
     scales[off] = static_cast<uint8_t>(sc);
