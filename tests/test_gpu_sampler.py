@@ -142,3 +142,27 @@ def test_invalid_options_are_refused_before_any_launch(tk, ctx):
         with pytest.raises(tk.GpuError, match=r"engine\.sampling"):
             tk.Sampler(ctx, VOCAB, [tk.SamplingOptions()], [stops]).sample(None, logits)
     assert ctx.launch_count == before
+
+
+@pytest.mark.parametrize("vocab", [32, 40, 8184, 8200, 262_144, 262_152, 600_000])
+def test_candidate_bound_at_block_edges(tk, ctx, oracle, vocab):
+    """The bound from the thread maxima: fewer values than threads, slices that end inside or just past a
+    block of 8192, two and more blocks per slice, all of the best values in one thread's share, ties."""
+    rng = np.random.default_rng(vocab)
+    one_thread = rng.standard_normal(vocab).astype(np.float32)
+    share = np.concatenate([np.arange(8) + 8 * (5 + 256 * i) for i in range(4)])
+    share = share[share < vocab]
+    one_thread[share] = 50.0 + np.arange(share.size)
+    ties = np.where(rng.random(vocab) < 0.01, 2.0, rng.choice([-1.0, 0.0, -0.0, 1.0], vocab)).astype(np.float32)
+    ramp = (np.arange(vocab) // 7).astype(np.float32)
+    rows = [oracle.f32_to_bf16(r) for r in (one_thread, ties, ramp, ramp[::-1].copy())]
+    for top_k in (1, 20, 32):
+        sampler = tk.Sampler(ctx, vocab, [tk.SamplingOptions(top_k=top_k, seed=1)] * len(rows), [(1, 2)] * len(rows))
+        sampler.sample(None, rows_to_device(rows), want_top=True)
+        torch.cuda.synchronize()
+        top = host(sampler.top)[:, :top_k]
+        for r, row in enumerate(rows):
+            index, value = oracle.top_k_select(row, top_k)
+            assert list(top[r, :, 1].view(np.uint32)) == list(index), (top_k, r)
+            assert np.array_equal(top[r, :, 0].copy().view(np.float32), value), (top_k, r)
+    assert ctx.device_status(None) == 0

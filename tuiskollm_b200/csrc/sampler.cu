@@ -2,14 +2,19 @@
 // replacing the host `Sampler` (tuisko-engine/src/sampling.rs:76-231) and the device -> host copy
 // of a 248 320-wide logit row that feeds it.
 //
-// One launch for a decode batch of up to 8 rows.  A row of BF16 logits (0.5 MB) is cut into
-// slices, one CTA each; every warp streams its share with 16-byte loads and keeps the 32 best
-// (value, index) keys it has seen, one per lane, sorted -- a few candidates enter one by one (a
-// ballot, a population count and one shuffle each), many at once through a bitonic sort and
-// merge across the lanes.  Lists fold pairwise (warp -> CTA through shared memory); the CTAs leave
-// theirs in a caller-owned scratch and take a ticket; the CTA that draws a row's last ticket
-// merges them and runs the reference's scalar selection on the k survivors (same float / double
-// operations in the same order), so no second launch and no host hop follow.
+// One launch for a decode batch of up to 8 rows.  A row of BF16 logits (0.5 MB) is cut into slices of
+// about 8000 values, one CTA each, 32 values per thread, all requested before the first is used.  The
+// top_k-th largest of the 256 thread maxima is a bound that at most top_k threads reach: only they
+// write candidates (about as many as top_k, never more than 32 per thread) to shared memory, and one
+// warp sorts those.  Inside a CTA a candidate is 32 bits, its order above its position in the slice;
+// sorts and merges run on one key per lane with warp shuffles.  The CTAs leave their 32 keys in a
+// caller-owned scratch and take a ticket; the CTA that draws a row's last ticket merges them and runs
+// the reference's scalar selection on the k survivors (same float / double operations in the same
+// order), so no second launch and no host hop follow.
+//
+// What bounds it is this chain of latencies, not the 4 MB of eight rows: 8.7 us for eight rows of
+// 248 320 values, against 20.4 us with sorted 64-bit lists kept by every warp, whose shuffles (two per
+// exchange, 330 per warp before the first value was dropped) filled the issue slots.
 #include <math.h>
 
 #include "common.cuh"
@@ -21,14 +26,15 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
-constexpr int kList = 32;  // keys a warp keeps = the largest admitted top_k
+constexpr int kList = 32;  // keys a list keeps = the largest admitted top_k
+constexpr int kPerThread = 32;                           // values of a block per thread
+constexpr int kBlockChunks = kThreads * kPerThread / 8;  // 8192 values: positions fit 16 bits
 
-// Larger key = earlier in the reference's order: value descending under the IEEE total order
-// (+0 above -0), then index ascending (sampling.rs:219-224: only a strictly greater value
+// Larger order = earlier in the reference's order: value descending under the IEEE total order
+// (+0 above -0); of equal ones the lower index (sampling.rs:219-224: only a strictly greater value
 // displaces a retained one).
-__device__ __forceinline__ uint64_t make_key(uint32_t bf16_bits, uint32_t index) {
-  const uint32_t ord = (bf16_bits & 0x8000u) ? (~bf16_bits & 0xffffu) : (bf16_bits | 0x8000u);
-  return (static_cast<uint64_t>(ord) << 32) | static_cast<uint64_t>(~index);
+__device__ __forceinline__ uint32_t order_of(uint32_t bf16_bits) {
+  return (bf16_bits & 0x8000u) ? (~bf16_bits & 0xffffu) : (bf16_bits | 0x8000u);
 }
 __device__ __forceinline__ uint32_t key_index(uint64_t key) { return ~static_cast<uint32_t>(key); }
 __device__ __forceinline__ float key_value(uint64_t key) {
@@ -71,18 +77,21 @@ __device__ __forceinline__ uint64_t shfl64(uint64_t v, int src) {
   return __shfl_sync(0xffffffffu, v, src);
 }
 
-__device__ __forceinline__ uint64_t max64(uint64_t a, uint64_t b) { return a > b ? a : b; }
-__device__ __forceinline__ uint64_t min64(uint64_t a, uint64_t b) { return a < b ? a : b; }
+template <class Key>
+__device__ __forceinline__ Key greater_of(Key a, Key b) { return a > b ? a : b; }
+template <class Key>
+__device__ __forceinline__ Key lesser_of(Key a, Key b) { return a < b ? a : b; }
 
 // Bitonic sort of one key per lane into descending order (lane 0 the largest): 15 exchanges.
-__device__ __forceinline__ uint64_t sort_descending(uint64_t v, int lane) {
+template <class Key>
+__device__ __forceinline__ Key sort_descending(Key v, int lane) {
 #pragma unroll
   for (int k = 2; k <= 32; k <<= 1) {
 #pragma unroll
     for (int j = k >> 1; j > 0; j >>= 1) {
-      const uint64_t other = __shfl_xor_sync(0xffffffffu, v, j);
+      const Key other = __shfl_xor_sync(0xffffffffu, v, j);
       const bool keep_max = ((lane & j) == 0) == ((lane & k) == 0);
-      v = keep_max ? max64(v, other) : min64(v, other);
+      v = keep_max ? greater_of(v, other) : lesser_of(v, other);
     }
   }
   return v;
@@ -90,44 +99,36 @@ __device__ __forceinline__ uint64_t sort_descending(uint64_t v, int lane) {
 
 // The 32 largest of two descending lists (one key per lane each), descending: reversing one list
 // makes the lane-wise maxima a bitonic sequence of exactly those keys; 5 exchanges sort it.
-__device__ __forceinline__ uint64_t merge_descending(uint64_t a, uint64_t b, int lane) {
-  uint64_t v = max64(a, __shfl_sync(0xffffffffu, b, 31 - lane));
+template <class Key>
+__device__ __forceinline__ Key merge_descending(Key a, Key b, int lane) {
+  Key v = greater_of(a, __shfl_sync(0xffffffffu, b, 31 - lane));
 #pragma unroll
   for (int j = 16; j > 0; j >>= 1) {
-    const uint64_t other = __shfl_xor_sync(0xffffffffu, v, j);
-    v = ((lane & j) == 0) ? max64(v, other) : min64(v, other);
+    const Key other = __shfl_xor_sync(0xffffffffu, v, j);
+    v = ((lane & j) == 0) ? greater_of(v, other) : lesser_of(v, other);
   }
   return v;
 }
 
-// The warp's sorted list lives one key per lane (`held`, lane 0 the best).  Offers `cand` of
-// every lane whose `want` is set; `kth` is the key at position top_k - 1 (0 while the list is short).
-// Many candidates at once (the first batches of a scan) go through a sort and a merge; a few
-// enter one by one, each by a ballot, a population count and one shuffle.
-__device__ __forceinline__ void offer(uint64_t& held, uint64_t& kth, uint64_t cand, bool want,
-                                      int lane, int top_k) {
-  unsigned pending = __ballot_sync(0xffffffffu, want);
-  if (__popc(pending) >= 6) {
-    held = merge_descending(held, sort_descending(want ? cand : 0ull, lane), lane);
-    kth = shfl64(held, top_k - 1);
-    return;
+// Warp 0 ends with the 32 largest keys of the CTA's eight descending lists (one per warp).
+template <class Key>
+__device__ __forceinline__ Key fold_warps(Key held, Key (*lists)[kList], int warp, int lane) {
+#pragma unroll
+  for (int half = kWarps / 2; half > 0; half >>= 1) {
+    if (warp >= half && warp < 2 * half) lists[warp][lane] = held;
+    __syncthreads();
+    if (warp < half) held = merge_descending(held, lists[warp + half][lane], lane);
   }
-  while (pending) {
-    const int src = __ffs(pending) - 1;
-    pending &= pending - 1;
-    const uint64_t c = shfl64(cand, src);
-    if (c > kth) {  // uniform across the warp: c and kth are
-      const int pos = __popc(__ballot_sync(0xffffffffu, held > c));
-      const uint64_t up = __shfl_up_sync(0xffffffffu, held, 1);
-      if (lane > pos) held = up;
-      else if (lane == pos) held = c;
-      kth = shfl64(held, top_k - 1);
-    }
-  }
+  return held;
 }
 
 __global__ void __launch_bounds__(kThreads, 1) sampler_kernel(SamplerParams p) {
-  __shared__ uint64_t lists[kWarps][kList];
+  __shared__ union {
+    uint32_t local[kWarps][kList];  // thread maxima, folded
+    uint32_t candidates[kList * kPerThread];
+    uint64_t global[kWarps][kList];  // slices' lists, folded
+  } lists;
+  __shared__ uint32_t bound, candidate_count;
   __shared__ int is_last;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int row = blockIdx.y, slice = blockIdx.x, slices = gridDim.x;
@@ -136,74 +137,73 @@ __global__ void __launch_bounds__(kThreads, 1) sampler_kernel(SamplerParams p) {
   uint64_t* row_scratch = p.scratch + static_cast<size_t>(row) * (slices * kList);
   unsigned int* ticket = reinterpret_cast<unsigned int*>(p.scratch + static_cast<size_t>(p.rows) * slices * kList) + row;
 
-  pdl_wait();
   pdl_trigger();
+  pdl_wait();
 
-  // 8-value chunks of the row, dealt to (slice, warp) in contiguous runs.
+  // 8-value chunks of the row, dealt to the slices in contiguous runs and walked in blocks of
+  // kBlockChunks (one block while the vocabulary has at most 32 * 8192 values).
   const int chunks = p.vocab / 8;
-  const int parts = slices * kWarps;
-  const int part = slice * kWarps + warp;
-  const int begin = static_cast<int>(static_cast<long long>(chunks) * part / parts);
-  const int end = static_cast<int>(static_cast<long long>(chunks) * (part + 1) / parts);
+  const int begin = static_cast<int>(static_cast<long long>(chunks) * slice / slices);
+  const int end = static_cast<int>(static_cast<long long>(chunks) * (slice + 1) / slices);
 
-  uint64_t held = 0, kth = 0;
+  uint64_t held = 0;
   bool nonfinite = false;
-  for (int base = begin; base < end; base += 32) {
-    const int chunk = base + lane;
-    uint32_t w[4] = {0, 0, 0, 0};
-    const bool live = chunk < end;
-    if (live) {
-      const uint4 v = __ldg(reinterpret_cast<const uint4*>(logits) + chunk);
-      w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
+  for (int base = begin; base < end; base += kBlockChunks) {
+    uint4 w[kPerThread / 8];
+#pragma unroll
+    for (int i = 0; i < kPerThread / 8; ++i) {
+      const int chunk = base + i * kThreads + tid;
+      w[i] = chunk < end ? __ldg(reinterpret_cast<const uint4*>(logits) + chunk) : make_uint4(0u, 0u, 0u, 0u);
     }
-    uint64_t cand[8];
+    // Keys of this block: order above 0xffff - position, so a lower index wins a tie; 0 is no value
+    // (the lowest order with the highest position is still above it).
+    uint32_t key[kPerThread];
+    uint32_t best = 0;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const uint32_t bits = (w[j >> 1] >> ((j & 1) * 16)) & 0xffffu;
-      nonfinite |= live && (bits & 0x7f80u) == 0x7f80u;
-      cand[j] = live ? make_key(bits, static_cast<uint32_t>(chunk * 8 + j)) : 0;
-    }
-    if (kth == 0) {
-      // The list is not full yet (the first 256 values of the warp's share): sort the eight
-      // batches side by side -- independent exchange chains hide each other's shuffle latency --
-      // and fold them as a tree, instead of eight sort-and-merge rounds one after the other.
+    for (int i = 0; i < kPerThread / 8; ++i) {
+      const bool live = base + i * kThreads + tid < end;
+      const uint32_t words[4] = {w[i].x, w[i].y, w[i].z, w[i].w};
 #pragma unroll
-      for (int k = 2; k <= 32; k <<= 1) {
-#pragma unroll
-        for (int jj = k >> 1; jj > 0; jj >>= 1) {
-          const bool keep_max = ((lane & jj) == 0) == ((lane & k) == 0);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const uint64_t other = __shfl_xor_sync(0xffffffffu, cand[j], jj);
-            cand[j] = keep_max ? max64(cand[j], other) : min64(cand[j], other);
-          }
-        }
+      for (int j = 0; j < 8; ++j) {
+        const uint32_t bits = (words[j >> 1] >> ((j & 1) * 16)) & 0xffffu;
+        nonfinite |= (bits & 0x7f80u) == 0x7f80u;
+        const uint32_t position = static_cast<uint32_t>((i * kThreads + tid) * 8 + j);
+        key[i * 8 + j] = live ? (order_of(bits) << 16) | (0xffffu - position) : 0u;
+        best = greater_of(best, key[i * 8 + j]);
       }
-#pragma unroll
-      for (int span = 4; span > 0; span >>= 1) {
-#pragma unroll
-        for (int j = 0; j < span; ++j) cand[j] = merge_descending(cand[j], cand[j + span], lane);
-      }
-      held = merge_descending(held, cand[0], lane);
-      kth = shfl64(held, top_k - 1);
-    } else {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) offer(held, kth, cand[j], cand[j] > kth, lane, top_k);
     }
+    const uint32_t maxima = fold_warps(sort_descending(best, lane), lists.local, warp, lane);
+    if (warp == 0) {
+      const uint32_t kth = __shfl_sync(0xffffffffu, maxima, top_k - 1);
+      if (lane == 0) {
+        bound = greater_of(kth, 1u);  // fewer than top_k threads have values: all of theirs
+        candidate_count = 0;
+      }
+    }
+    __syncthreads();
+    const uint32_t least = bound;
+    if (best >= least) {  // at most top_k threads: keys are distinct
+#pragma unroll
+      for (int i = 0; i < kPerThread; ++i) {
+        if (key[i] >= least) lists.candidates[atomicAdd(&candidate_count, 1u)] = key[i];
+      }
+    }
+    __syncthreads();
+    if (warp == 0) {
+      const int count = static_cast<int>(candidate_count);
+      uint32_t top = 0;
+      for (int c = 0; c < count; c += kList) {
+        const uint32_t sorted = sort_descending(c + lane < count ? lists.candidates[c + lane] : 0u, lane);
+        top = c == 0 ? sorted : merge_descending(top, sorted, lane);
+      }
+      const uint32_t index = static_cast<uint32_t>(base) * 8u + (0xffffu - (top & 0xffffu));
+      const uint64_t wide = top == 0u ? 0ull : (static_cast<uint64_t>(top >> 16) << 32) | static_cast<uint64_t>(~index);
+      held = base == begin ? wide : merge_descending(held, wide, lane);
+    }
+    __syncthreads();  // the shared lists are free again
   }
   if (nonfinite) atomicOr(p.status, STATUS_NONFINITE_LOGIT);
 
-  // The CTA's eight lists fold into warp 0's as a tree of merges through shared memory.
-  auto fold_warps = [&]() {
-#pragma unroll
-    for (int half = kWarps / 2; half > 0; half >>= 1) {
-      if (warp >= half && warp < 2 * half) lists[warp][lane] = held;
-      __syncthreads();
-      if (warp < half) held = merge_descending(held, lists[warp + half][lane], lane);
-      __syncthreads();
-    }
-  };
-  fold_warps();
   if (warp == 0) {
     row_scratch[slice * kList + lane] = held;
     __threadfence();
@@ -214,8 +214,7 @@ __global__ void __launch_bounds__(kThreads, 1) sampler_kernel(SamplerParams p) {
   if (!is_last) return;
   __threadfence();
 
-  // The row's last CTA: every warp merges its share of the slices' lists, then the same tree.
-  held = 0;
+  // The row's last CTA: every warp merges its share of the slices' lists, then the tree over the warps.
   {
     // at most 32 slices: four lists per warp, all requested before the first merge
     uint64_t other[4];
@@ -224,10 +223,9 @@ __global__ void __launch_bounds__(kThreads, 1) sampler_kernel(SamplerParams p) {
       const int s = warp + i * kWarps;
       other[i] = s < slices ? *reinterpret_cast<volatile uint64_t*>(row_scratch + s * kList + lane) : 0ull;
     }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) held = merge_descending(held, other[i], lane);
+    held = merge_descending(merge_descending(other[0], other[1], lane), merge_descending(other[2], other[3], lane), lane);
   }
-  fold_warps();
+  held = fold_warps(held, lists.global, warp, lane);
   if (warp != 0) return;
   if (lane == 0) *ticket = 0;  // ready for the next launch
 
@@ -249,7 +247,7 @@ __global__ void __launch_bounds__(kThreads, 1) sampler_kernel(SamplerParams p) {
     // Lane i ends with the running sum over survivors 0..i, added in survivor order (the
     // reference's three loops walk this same sequence).
     double running = 0.0;
-#pragma unroll 1
+#pragma unroll 4
     for (int i = 0; i < top_k; ++i) {
       const double w = __shfl_sync(0xffffffffu, my_weight, i);
       if (i <= lane) running += w;
