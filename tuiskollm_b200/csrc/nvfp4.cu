@@ -235,7 +235,6 @@ __global__ void __launch_bounds__(nv_threads(BLOCK_TOK, GATE_UP), (GATE_UP || BL
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = ctl->tmem_base;
-  pdl_trigger();
   // the cluster's barriers exist from here on; the matching wait comes just before the first
   // access to a peer's shared memory
   if (pushed) cluster_arrive();
@@ -259,6 +258,10 @@ __global__ void __launch_bounds__(nv_threads(BLOCK_TOK, GATE_UP), (GATE_UP || BL
       }
     }
   } else if (warp == 1) {
+    // The next kernel may start once the last blocks are under way: its CTAs then fill the slots that
+    // this kernel's epilogues give back.  From the set-up on they would take part of this kernel's
+    // bandwidth and wait (MLP, one token: 32.3 us with the trigger there, 31.7 here, 32.0 behind the
+    // loop, 33.7 without one).
     if (elect_one()) {
       const uint32_t sf_base = tmem + ACC_COLS;
       // a BLOCK_TOK < 128 tile sits in one 32-row quartile of its 128-row scale tile:
@@ -297,6 +300,7 @@ __global__ void __launch_bounds__(nv_threads(BLOCK_TOK, GATE_UP), (GATE_UP || BL
                        slot + 8 + sfb_quartile, acc);
           }
         }
+        if (i == max(0, nkb - 1 - STAGES / 2)) pdl_trigger();
         umma_commit(&ctl->empty[s]);
       }
       umma_commit(&ctl->tmem_full);
