@@ -10,7 +10,7 @@
 //
 //   warp 0     TMA producer, one ring across all tiles of the pair (as many stages as fit 200 KB)
 //   warp 1     even CTA: scale copies (NVFP4) and MMAs for both CTAs
-//   warps 2-9  epilogue: two warps per TMEM lane quadrant, alternate 32-token batches
+//   warps 2-   epilogue: two (NVFP4 SwiGLU: four) warps per TMEM lane quadrant, alternate 32-token batches
 //
 // Two accumulators in TMEM let the epilogue of one tile run under the MMAs of the next.  FP8: two times
 // 256 columns.  NVFP4 keeps 128 columns for scale factors (two stages of 4 x 16), which leaves 384: two
@@ -44,10 +44,17 @@ constexpr int kStageKBytes = 128;  // K bytes per row and stage (128 FP8 or 256 
 constexpr int kWTile = kRows * kStageKBytes;
 constexpr int kSfTile = 2048;      // scales of 128 rows x 16 groups
 constexpr int kMaxStages = 12;
-constexpr int kEpilogueWarps = 8;
-constexpr int kThreads = 64 + 32 * kEpilogueWarps;
 constexpr int kBatch = 32;         // tokens an epilogue warp handles at a time
-constexpr int kStagingPerWarp = kBatch * 64;
+// Epilogue warps.  SwiGLU with the quantisation behind it is a long dependent chain per value, and eight warps
+// did not get through a 256-token NVFP4 tile under the next tile's MMAs: gate/up of 512 tokens 47.5 -> 44.7 us
+// with sixteen, 301 tokens 45.2 -> 41.1, 2048 tokens 160.5 -> 157.5.  FP8 tiles have twice the MMA time per value;
+// there sixteen warps and the 96 registers they leave were slower (512 tokens 66.0 -> 68.6 us).
+__host__ __device__ constexpr int epilogue_warps(bool nv, bool swiglu) { return nv && swiglu ? 16 : 8; }
+__host__ __device__ constexpr int block_threads(bool nv, bool swiglu) { return 64 + 32 * epilogue_warps(nv, swiglu); }
+// transposition space of a warp: 32 rows (SwiGLU: 16 outputs) of 2 bytes per token
+__host__ __device__ constexpr int staging_per_warp(bool swiglu) { return kBatch * (swiglu ? 32 : 64); }
+constexpr int kStagingBytes = epilogue_warps(false, false) * staging_per_warp(false);
+static_assert(epilogue_warps(true, true) * staging_per_warp(true) == kStagingBytes, "one ring size for all kernels");
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kSfCols = 128;      // NVFP4: two stages of scale columns
 constexpr uint32_t kSfStageCols = 64;  // per stage: 4 K steps x 16 (4 weight + up to 8 token columns)
@@ -63,7 +70,7 @@ struct Control {
 };
 
 constexpr size_t kRingBytes =
-    (kSmemLimit - 1024 - kEpilogueWarps * kStagingPerWarp - sizeof(Control)) / 1024 * 1024;
+    (kSmemLimit - 1024 - kStagingBytes - sizeof(Control)) / 1024 * 1024;
 
 __device__ __forceinline__ uint4 lds128(uint32_t addr) {
   uint4 v;
@@ -75,14 +82,16 @@ __device__ __forceinline__ void sts128(uint32_t addr, const uint4& v) {
 }
 
 template <bool NV, bool SWIGLU>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(block_threads(NV, SWIGLU), 1)
     pair_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
                      const __grid_constant__ CUtensorMap map_wsf, const __grid_constant__ CUtensorMap map_asf,
                      const __grid_constant__ PairGemmParams p) {
+  constexpr int EW = epilogue_warps(NV, SWIGLU);
+  constexpr int PARTS = EW / 4;  // warps that share a TMEM lane quadrant, on alternate batches
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  Control* ctl = reinterpret_cast<Control*>(smem + kRingBytes + kEpilogueWarps * kStagingPerWarp);
+  Control* ctl = reinterpret_cast<Control*>(smem + kRingBytes + kStagingBytes);
 
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const uint32_t cta = cluster_cta_rank();
@@ -115,7 +124,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&ctl->acc_full[b], 1);
-      mbar_init(&ctl->acc_empty[b], 2 * kEpilogueWarps);
+      mbar_init(&ctl->acc_empty[b], 2 * EW);
     }
     fence_mbar_init();
     prefetch_tensormap(&map_w);
@@ -282,8 +291,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     // ----------------------------------------------------------------- epilogue
     const int ew = warp - 2;
     const int quad = warp & 3;   // TMEM lane quadrant this warp may read
-    const int part = ew >> 2;    // which of the quadrant's two warps
-    const uint32_t stg = smem_u32(smem + kRingBytes + ew * kStagingPerWarp);
+    const int part = ew >> 2;    // which of the quadrant's warps
+    const uint32_t stg = smem_u32(smem + kRingBytes + ew * staging_per_warp(SWIGLU));
     const uint32_t acc_empty0 = mapa_u32(smem_u32(&ctl->acc_empty[0]), leader);
     const int batches = tok_tile / kBatch;
 
@@ -436,7 +445,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       const uint32_t taddr = tmem + (static_cast<uint32_t>(quad * 32) << 16) + static_cast<uint32_t>(b) * acc_stride;
       if (splits > 1) {
         // park the batches other splits finish over the ring, whose loads and reads are all done
-        for (int o = part; o < batches; o += 2) {
+        for (int o = part; o < batches; o += PARTS) {
           if (o % splits == split || tok0 + o * kBatch >= p.rows) continue;
           uint32_t f[2][16];
           tmem_ld_16x256b_x4(taddr + o * kBatch, f[0]);
@@ -450,19 +459,19 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         break;  // one tile per cluster; finished behind the cluster barrier below
       }
-      // two warps share a quadrant: batches part, part + 2, ... in the order in which columns are due
+      // batches part, part + PARTS, ... in the order in which columns are due
       const int due = overlap ? overlap_batches : batches;  // columns the next tile waits for
       if (part >= due) {
         __syncwarp();
         if (lane == 0) mbar_arrive_remote(acc_empty0 + static_cast<uint32_t>(b) * 8u);
       }
-      for (int o = part; o < batches; o += 2) {
+      for (int o = part; o < batches; o += PARTS) {
         const int batch = (overlap && b == 0) ? batches - 1 - o : o;
         uint32_t f[2][16];
         tmem_ld_16x256b_x4(taddr + batch * kBatch, f[0]);
         tmem_ld_16x256b_x4(taddr + (16u << 16) + batch * kBatch, f[1]);
         tmem_ld_wait();
-        if (o < due && o + 2 >= due) {
+        if (o < due && o + PARTS >= due) {
           tc_fence_before_sync();
           __syncwarp();
           if (lane == 0) mbar_arrive_remote(acc_empty0 + static_cast<uint32_t>(b) * 8u);
@@ -481,8 +490,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         float ws[4];
         row_scales(unit, ws);
         const uint32_t taddr = tmem + (static_cast<uint32_t>(quad * 32) << 16);
-        // this split's batches are split, split + splits, ...; the quadrant's two warps alternate
-        for (int o = split + part * splits; o < batches; o += 2 * splits) {
+        // this split's batches are split, split + splits, ...; the quadrant's warps alternate
+        for (int o = split + part * splits; o < batches; o += PARTS * splits) {
           const int t0 = tok0 + o * kBatch;
           if (t0 >= p.rows) break;
           uint32_t own[2][16];
@@ -544,7 +553,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 template <bool NV, bool SWIGLU>
 cudaError_t pg_launch(cudaStream_t stream, int workers, const CUtensorMap& w, const CUtensorMap& a,
                       const CUtensorMap& wsf, const CUtensorMap& asf, const PairGemmParams& p) {
-  return launch_kernel_cluster(pair_gemm_kernel<NV, SWIGLU>, dim3(2 * p.splits * workers), dim3(kThreads),
+  return launch_kernel_cluster(pair_gemm_kernel<NV, SWIGLU>, dim3(2 * p.splits * workers), dim3(block_threads(NV, SWIGLU)),
                                kSmemLimit, stream, dim3(2 * p.splits), w, a, wsf, asf, p);
 }
 
@@ -575,7 +584,7 @@ cudaError_t pair_gemm_prepare(int* max_clusters) {
   for (int s = 1; s <= kPairGemmMaxSplits; ++s) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * s * 512, 1, 1);
-    cfg.blockDim = dim3(kThreads);
+    cfg.blockDim = dim3(block_threads(true, true));
     cfg.dynamicSmemBytes = kSmemLimit;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
