@@ -512,20 +512,20 @@ __global__ void __launch_bounds__(nv_threads(BLOCK_TOK, GATE_UP), (GATE_UP || BL
         const float* base =
             p.partials + (static_cast<size_t>(tile_m) * tiles_n + tile_n) * tile_elems + row_in_tile;
 #pragma unroll 1
-        for (int j0 = half * 8; j0 < valid_tok; j0 += 16) {
-          float v[8][8];  // [split][token]: every load of the batch is issued before the adds
+        for (int j0 = half * 4; j0 < valid_tok; j0 += 8) {
+          float v[8][4];  // [split][token]: every load of the batch is issued before the adds
 #pragma unroll
           for (int sp = 0; sp < 8; ++sp) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
+            for (int j = 0; j < 4; ++j) {
               v[sp][j] = (sp < p.splits && j0 + j < valid_tok)
                              ? __ldcg(base + sp * split_stride + (j0 + j) * kRows)
                              : 0.0f;
             }
           }
-          float acc[8];
+          float acc[4];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
+          for (int j = 0; j < 4; ++j) {
             acc[j] = 0.0f;
 #pragma unroll
             for (int sp = 0; sp < 8; ++sp) {
@@ -533,7 +533,7 @@ __global__ void __launch_bounds__(nv_threads(BLOCK_TOK, GATE_UP), (GATE_UP || BL
             }
           }
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
+          for (int j = 0; j < 4; ++j) {
             if (j0 + j < valid_tok && row_ok) {
               const size_t o = static_cast<size_t>(tok0 + j0 + j) * p.out_rows + n;
               const float v = __fmul_rn(acc[j], s);
@@ -580,20 +580,26 @@ __global__ void __launch_bounds__(nv_threads(BLOCK_TOK, GATE_UP), (GATE_UP || BL
           for (int j = 0; j < 16; ++j) oth[j] = ld_dsmem_f32(other_addr + (c + j) * kRows * 4, pair_rank ^ 1u);
         }
         tmem_ld_wait();
-        uint32_t bits[16];
+        uint32_t pairs[8];  // two rounded outputs each
+        auto bits = [&](int j) { return (pairs[j >> 1] >> ((j & 1) * 16)) & 0xffffu; };
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const float mine_v = __fmul_rn(__uint_as_float(own[j]), p.out_scale);
-          const float oth_v = __fmul_rn(oth[j], p.out_scale);
-          const float gate = pair_rank == 0 ? mine_v : oth_v;
-          const float up = pair_rank == 0 ? oth_v : mine_v;
-          bits[j] = f32_to_bf16_bits(__fmul_rn(silu_stable(gate), up));
+        for (int j = 0; j < 16; j += 2) {
+          float y[2];
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const float mine_v = __fmul_rn(__uint_as_float(own[j + e]), p.out_scale);
+            const float oth_v = __fmul_rn(oth[j + e], p.out_scale);
+            const float gate = pair_rank == 0 ? mine_v : oth_v;
+            const float up = pair_rank == 0 ? oth_v : mine_v;
+            y[e] = __fmul_rn(silu_stable(gate), up);
+          }
+          pairs[j >> 1] = pack_bf16x2(y[0], y[1]);
         }
         if (row_ok && p.out) {
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
             if (c0 + j < valid_tok) {
-              p.out[static_cast<size_t>(tok0 + c0 + j) * p.out_rows + n] = static_cast<uint16_t>(bits[j]);
+              p.out[static_cast<size_t>(tok0 + c0 + j) * p.out_rows + n] = static_cast<uint16_t>(bits(j));
             }
           }
         }
@@ -620,7 +626,7 @@ __global__ void __launch_bounds__(nv_threads(BLOCK_TOK, GATE_UP), (GATE_UP || BL
 #pragma unroll
           for (int j = 0; j < 16; ++j) {
             if (c0 + j < valid_tok) {  // warp-uniform
-              const uint32_t packed = nvfp4_code_of_lane(bits[j], p.q_divisor);
+              const uint32_t packed = nvfp4_code_of_lane(bits(j), p.q_divisor);
               const uint32_t nib = packed & 0xfu;
               store_q(j, nib, __shfl_xor_sync(0xffffffffu, nib, 1), packed >> 8);
             }
