@@ -4,6 +4,11 @@
 // nvfp4_scale_offset :410-422).  Both are lossless byte movers: source planes are uploaded as the
 // checkpoint stores them and rearranged in HBM, so the host never walks 11 MB of scale codes
 // byte by byte.
+//
+// Both kernels wait for the kernel in front of them before they read or write anything: what they write
+// may still be read there, and the kernel behind waits for these alone.  They release nothing early, and a
+// thread ends behind a fence on its stores, because a projection behind them requests weights ahead of its
+// own wait.
 #include <type_traits>
 
 #include "common.cuh"
@@ -20,6 +25,7 @@ constexpr int kGatherThreads = 256;
 template <bool VEC>
 __global__ void __launch_bounds__(kGatherThreads) gather_planes_kernel(GatherParams p) {
   using Word = typename std::conditional<VEC, uint4, uint8_t>::type;
+  pdl_wait();
   const size_t total = p.offset[p.planes] / sizeof(Word);
   const size_t stride = static_cast<size_t>(gridDim.x) * kGatherThreads;
   for (size_t i = static_cast<size_t>(blockIdx.x) * kGatherThreads + threadIdx.x; i < total; i += stride) {
@@ -30,6 +36,7 @@ __global__ void __launch_bounds__(kGatherThreads) gather_planes_kernel(GatherPar
     const Word* source = reinterpret_cast<const Word*>(p.source[plane] + (byte - p.offset[plane]));
     reinterpret_cast<Word*>(p.output)[i] = *source;
   }
+  __threadfence();
 }
 
 // One CTA permutes 128 rows x 64 groups (16 tiles of 512 bytes): rows are read as 64-byte runs
@@ -40,6 +47,7 @@ constexpr int kSwizzleGroups = 64;
 
 __global__ void __launch_bounds__(kSwizzleThreads) swizzle_scales_kernel(SwizzleParams p) {
   __shared__ __align__(16) uint8_t tile[128][kSwizzleGroups + 16];  // +16: rows land in different banks
+  pdl_wait();
   const int tid = threadIdx.x;
   const size_t row_tile = blockIdx.y;
   const size_t group0 = static_cast<size_t>(blockIdx.x) * kSwizzleGroups;
@@ -87,6 +95,7 @@ __global__ void __launch_bounds__(kSwizzleThreads) swizzle_scales_kernel(Swizzle
     uint8_t* dst = p.output + (row_tile * tiles_per_row + group0 / 4 + t) * 512 + row_mod32 * 16;
     *reinterpret_cast<uint4*>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
   }
+  __threadfence();
 }
 
 }  // namespace
