@@ -21,8 +21,10 @@ the peers over NVLink and merges (N > 1): two kernel launches per step.
             inside the timed region, one stream synchronisation per step (graph replay, and
             `e2e.eager` with every operator call made from the host)
   roofline  the projection kernel alone against the measured HBM copy bandwidth
-  configs   (N = 1) every other benchmark configuration as its own measured row with its
-            roofline and the CPU oracle beside it
+  configs   (N = 1) every other benchmark configuration as its own measured row: time, kernel and
+            fraction of its roofline; the rows in full (bytes, flops, nominal peaks, end-to-end and
+            CPU figures) go to stderr, one JSON line each, so that the line stays short enough for
+            a reader that keeps only the end of a run's output
 
 `--impl reference` times the CPU restatement of the reference's qualification oracle for
 the same workload on the host cores (the reference is Rust + cuda-oxide for sm_120 and can
@@ -486,6 +488,16 @@ class Protocol:
         for name, _replay, ops, inner in self.cases:
             out[name]["operations_per_sample"] = ops * inner
         return out
+
+
+def line_row(row):
+    """What the printed line carries of a configuration row."""
+    short = {k: row[k] for k in ("config", "op", "M", "N", "K") if k in row}
+    short["us"] = {k: round(row["us"][k], 3) for k in ("median", "p10", "p90")}
+    roofline = row["roofline"]
+    short["kernel"], short["bound"] = roofline["kernel"], roofline["bound"]
+    short["frac"] = round(roofline["frac"], 4)
+    return short
 
 
 def hbm_roofline(kernel, nbytes, us, peak, peak_kind):
@@ -1782,7 +1794,9 @@ def run_native(args):
             if row_clocks.get("sm_mhz"):
                 for r in rows:
                     r["kilocycles_at_median_sm_clock"] = r["us"]["median"] * row_clocks["sm_mhz"] / 1e3
-            line["configs"] = rows
+            for r in rows:
+                print(json.dumps({"config_row": r}), file=sys.stderr, flush=True)
+            line["configs"] = [line_row(r) for r in rows]
             if deviation is not None:
                 line["w4a4_vs_a16"] = deviation
         print(json.dumps(line), flush=True)

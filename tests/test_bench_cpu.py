@@ -33,3 +33,25 @@ def test_operations_per_sample_reach_the_floor():
         assert ops * (inner - 1) < floor, name       # no more graph launches than needed
     proto.add("explicit", lambda: None, 4, inner=1)
     assert proto.cases[-1][3] == 1
+
+
+def test_printed_line_stays_short():
+    """A reader that keeps the last 32 KB of a run's output still finds the whole line: with the rows
+    in full (about 800 bytes each, 70 and more of them) it did not."""
+    import json
+    import xtask
+
+    bench = _bench()
+    roofline = bench.tensor_roofline("fp8_projection_kernel<128,0> splits=7 cluster-leader", 3.65e11 / 3, 1.7e8 / 3,
+                                     148.12345678901234, 4500.0, 2, 6535.4)
+    row = {"config": "decode", "op": "nvfp4_gate_up_swiglu_quantize", "M": 2048, "N": 16384, "K": 17408,
+           "weight_copies": 12, "us": {"median": 148.12345678901234, "p10": 1.0 / 3, "p90": 2.0 / 3, "samples": 40,
+                                       "operations_per_sample": 32},
+           "roofline": roofline, "e2e": {"us": 1.0 / 3, "note": "x" * 80},
+           "cpu_baseline": {"value": 1.0 / 3, "us_full_shape": 1e9 / 3, "sample": "x" * 160},
+           "kilocycles_at_median_sm_clock": 1e3 / 3}
+    assert len(json.dumps(row)) > 800
+    short = [bench.line_row(row) for _ in range(90)]
+    assert len(json.dumps(short)) < 24 << 10        # the rest of the line takes about 4 KB
+    line = {"config": {"rows": 1, "vocab": 248320}, "protocol": {"us_per_step": {"median": 186.0}}, "configs": short}
+    assert xtask.perf_rows(line)[("nvfp4_gate_up_swiglu_quantize", 2048, 16384)] == 148.123   # what the gate reads
