@@ -36,6 +36,7 @@ def _nvfp4_planes(tk, rows, k):
     (768, 2048, 100, 0, 2),    # K split in two
     (512, 4096, 130, 160, 4),  # K split in four, odd number of batches
     (40000, 256, 70, 64, 1),   # more tiles than pairs: three rounds of the two accumulators
+    (512, 1024, 64, 0, 5),     # a split count no cluster has: the plan's own
 ])
 def test_fp8_projection(tk, oracle, monkeypatch, out_rows, k, rows, tok, splits):
     from tuiskollm_b200 import synth
@@ -52,7 +53,7 @@ def test_fp8_projection(tk, oracle, monkeypatch, out_rows, k, rows, tok, splits)
     op.launch(None, rows, out_rows, k, dev(xb.view(np.int16)), codes, scales, w, s, out)
     torch.cuda.synchronize()
     assert c.last_kernel.startswith("fp8_pair_persist_kernel"), c.last_kernel
-    assert f"splits={max(splits, 1)}" in c.last_kernel, c.last_kernel
+    assert f"splits={splits if 1 <= splits <= 4 else 1}" in c.last_kernel, c.last_kernel
     assert c.device_status() == 0
     oc, os_ = oracle.quantize_e4m3(xb)
     assert np.array_equal(host(codes), oc)
@@ -67,11 +68,12 @@ def test_fp8_projection(tk, oracle, monkeypatch, out_rows, k, rows, tok, splits)
     assert c.device_status() == 0
 
 
-@pytest.mark.parametrize("rows,tok", [(33, 0), (96, 0), (129, 0), (257, 0), (300, 32)])
-def test_fp8_swiglu(tk, oracle, monkeypatch, rows, tok):
+@pytest.mark.parametrize("rows,tok,splits", [(33, 0, 0), (96, 0, 0), (129, 0, 0), (257, 0, 0), (300, 32, 0), (40, 0, 3)])
+def test_fp8_swiglu(tk, oracle, monkeypatch, rows, tok, splits):
     from tuiskollm_b200 import synth
 
     monkeypatch.setenv("TK100_PAIR_TOK", str(tok))
+    monkeypatch.setenv("TK100_PAIR_SPLITS", str(splits))  # gate/up does not split: its plan ignores it
     hidden, inter = 1024, 1280
     c = tk.Context(device=0, hidden=hidden, intermediate=inter)
     xb = synth.normal_bf16(62, rows, (rows, hidden))
@@ -110,6 +112,7 @@ def test_nvfp4_mlp(tk, oracle, monkeypatch, hidden, inter, rows, tok, splits):
     gu, gus, gud = synth.nvfp4_weights(63, 1, 2 * inter, hidden)
     dn, dns, dnd = synth.nvfp4_weights(63, 2, hidden, inter)
     a_div, m_div = float(np.float32(448.0 * 6.0 / 5.0)), float(np.float32(448.0 * 6.0 / 8.0))
+    monkeypatch.setenv("TK100_PAIR_SPLITS", str(splits))  # gate/up does not split: its plan ignores it
     c = tk.Context(device=0, hidden=hidden, intermediate=inter)
     a_codes, a_scales = _nvfp4_planes(tk, rows, hidden)
     m_codes, m_scales = _nvfp4_planes(tk, rows, inter)
@@ -120,20 +123,15 @@ def test_nvfp4_mlp(tk, oracle, monkeypatch, hidden, inter, rows, tok, splits):
                                         activation_codes=a_codes, activation_scales=a_scales,
                                         input_global_divisor=a_div, output_global_divisor=m_div,
                                         output_codes=m_codes, output_scales=m_scales)
-    assert c.last_kernel.startswith("nvfp4_persist_kernel"), c.last_kernel
-    if splits:
-        monkeypatch.setenv("TK100_PAIR_SPLITS", str(splits))
-        c2 = tk.Context(device=0, hidden=hidden, intermediate=inter)
-    else:
-        c2 = c
-    down = tk.Nvfp4DownOp(c2)
+    assert c.last_kernel.startswith("nvfp4_persist_kernel") and "splits=1" in c.last_kernel, c.last_kernel
+    down = tk.Nvfp4DownOp(c)
     kw = dict(activation_codes=m_codes, activation_scales=m_scales, input_global_divisor=m_div)
     down.launch(None, rows, None, dev(dn), dev(dns), float(dnd), out, **kw)
     if splits:
-        assert f"splits={splits}" in c2.last_kernel, c2.last_kernel
+        assert f"splits={splits}" in c.last_kernel, c.last_kernel
     down.launch_partial(None, rows, None, dev(dn), dev(dns), float(dnd), part, **kw)
     torch.cuda.synchronize()
-    assert c.device_status() == 0 and c2.device_status() == 0
+    assert c.device_status() == 0
     oc, osc = oracle.nvfp4_quantize(xb, a_div)
     dots = oracle.nvfp4_w4a4_dot(oc, osc, a_div, gu, gus, float(gud))
     exp_mid = oracle.silu_mul(dots[:, :inter], dots[:, inter:])

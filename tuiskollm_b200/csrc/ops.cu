@@ -388,8 +388,10 @@ struct PairPlan {
 // tile takes the longer of its MMAs (2 N cycles for 256 x N x 128 bytes) and of its delivery from L2
 // (about 56 bytes per cycle and SM measured on B200); a launch takes at least its weights at HBM rate
 // (about 3.9 KB per cycle).  Splitting K costs an exchange and wants at least 8 stages a split.
+// A forced split count holds where it is admitted; where it is not (gate/up never splits) the plan is
+// chosen as without it.
 PairPlan plan_pairs(const Context& ctx, int rows, int row_units, int nkb, bool nvfp4, double weight_bytes,
-                    bool may_split) {
+                    bool may_split, bool forced = true) {
   PairPlan best;
   const Tuning& tune = ctx.tuning();
   const int least = (rows + 255) / 256;
@@ -402,7 +404,7 @@ PairPlan plan_pairs(const Context& ctx, int rows, int row_units, int nkb, bool n
     const long long tiles = static_cast<long long>(tiles_m) * row_units;
     const double stage = std::max(2.0 * tok, pair_gemm_stage_bytes(nvfp4, tok) / 56.0);
     for (int s = 1; s <= kPairGemmMaxSplits; ++s) {
-      if (tune.pair_splits > 0 && s != tune.pair_splits) continue;
+      if (forced && tune.pair_splits > 0 && s != tune.pair_splits) continue;
       const int clusters = ctx.pair_clusters(s);
       if (clusters <= 0 || (s > 1 && (!may_split || nkb / s < 8 || tiles > clusters))) continue;
       const long long waves = s > 1 ? 1 : (tiles + clusters - 1) / clusters;
@@ -417,7 +419,8 @@ PairPlan plan_pairs(const Context& ctx, int rows, int row_units, int nkb, bool n
       }
     }
   }
-  return best;
+  if (best.workers == 0 && forced) return plan_pairs(ctx, rows, row_units, nkb, nvfp4, weight_bytes, may_split, false);
+  return best;  // an unsplit plan is always admitted
 }
 
 PairGemmParams pair_params(Context& ctx, const PairPlan& plan, int rows, int out_rows, int k, int row_units, bool nvfp4,
