@@ -104,7 +104,9 @@ TK100_API const char* tk100_last_kernel(tk100_ctx* ctx);
 
 /* Declares a weight-code plane (`rows` x `row_bytes` bytes, 128-byte aligned: an FP8 plane has
  * row_bytes = K, a packed NVFP4 plane K / 2) so that its TMA tensor map is encoded now, at load
- * time, instead of on the plane's first launch; registered maps are never evicted.  Replaces the
+ * time, instead of on the plane's first launch; registered maps are never evicted.  A plane of the
+ * shape of gate/up weights (2 * intermediate rows over `hidden` columns) has two maps, one for up to
+ * 32 rows and one for more, and gets both.  NVFP4 scale planes are not declared.  Replaces the
  * per-operator `prepare` step of the reference (`*Op::new`, e.g.
  * tuisko-kernels-sm120/src/fp8/projection.rs:525-545).  Optional: an undeclared plane is encoded
  * on first use and cached.  Not stream-ordered, host work only. */

@@ -358,6 +358,43 @@ def test_registered_plane_is_not_encoded_again(tk, ctx, oracle):
         ctx.register_plane(wd.view(-1)[1:1 + 1024 * 64].view(1024, 64))   # not 128-byte aligned
 
 
+@pytest.mark.parametrize("fp4", [False, True])
+def test_registered_gate_up_plane_is_not_encoded_again(tk, fp4):
+    """The same for gate/up weights on both sides of 32 rows, which read the plane through two maps."""
+    hidden, inter = 512, 256
+    c = tk.Context(device=0, hidden=hidden, intermediate=inter)
+    k_bytes = hidden // 2 if fp4 else hidden
+    w = torch.randint(0, 0x70, (2 * inter, k_bytes), dtype=torch.uint8, device="cuda")
+    scale_bytes = tk.ops.nvfp4_scale_plane_bytes
+    ws = torch.full((scale_bytes(2 * inter, hidden),), 0x38, dtype=torch.uint8, device="cuda") if fp4 else \
+        torch.full((2 * inter,), 0x3C00, dtype=torch.int16, device="cuda")
+
+    def launch(rows, plane):
+        codes = torch.randint(0, 0x70, (128, k_bytes), dtype=torch.uint8, device="cuda")
+        scales = torch.full((scale_bytes(128, hidden),), 0x38, dtype=torch.uint8, device="cuda") if fp4 else \
+            torch.ones((128,), dtype=torch.float32, device="cuda")
+        out = torch.empty((rows, inter), dtype=torch.int16, device="cuda")
+        keep.append((codes, scales))  # no later plane at these addresses
+        before = c.tensor_map_counts[1]
+        if fp4:
+            tk.Nvfp4SwiGluOp(c).launch(None, rows, None, plane, ws, 1.0, out, activation_codes=codes,
+                                       activation_scales=scales, input_global_divisor=1.0)
+        else:
+            tk.Fp8SwiGluOp(c).launch(None, rows, None, codes, scales, plane, ws, out)
+        return c.tensor_map_counts[1] - before
+
+    keep = []
+    c.register_plane(w)
+    assert c.tensor_map_counts[0] == 2
+    other = w.clone()
+    assert launch(3, w) == 1                      # the activation plane only
+    assert launch(40, w) == (3 if fp4 else 1)     # with the two scale planes of the NVFP4 form
+    assert launch(3, other) == 2                  # the undeclared copy's map for up to 32 rows ...
+    assert launch(40, other) == (3 if fp4 else 2) # ... and for more (the weight scales' map is cached)
+    torch.cuda.synchronize()
+    assert c.device_status() == 0
+
+
 @pytest.mark.parametrize("out_rows,rows", [(1024, 700), (4096, 1300), (4096, 2600)])
 def test_persistent_pair_route_matches_pair_route_bit_for_bit(tk, oracle, out_rows, rows, monkeypatch):
     """TK100_FP8_PERSIST: resident CTA pairs walk the pair tiles with two TMEM accumulators in

@@ -55,6 +55,12 @@ Tuning Tuning::from_environment() {
   return t;
 }
 
+#define TK100_TRY(expr)                  \
+  do {                                   \
+    Status _s = (expr);                  \
+    if (_s != TK100_OK) return _s;       \
+  } while (0)
+
 // --------------------------------------------------------------------- Context
 
 Status Context::check(cudaError_t e, const char* operation) {
@@ -250,9 +256,15 @@ Status Context::register_plane(const void* base, uint64_t rows, uint64_t row_byt
   }
   const MapKey key{base, rows, row_bytes, 128u, 0u};
   CUtensorMap map;
-  Status s = encode_map(key, &map);
-  if (s != TK100_OK) return s;
+  TK100_TRY(encode_map(key, &map));
   pinned_maps_[key] = map;
+  // A plane of the shape of gate/up weights is also read through the map that interleaves its halves.
+  const uint64_t inter = config_.intermediate, hidden = config_.hidden;
+  if (rows == 2 * inter && inter % 128 == 0 && (row_bytes == hidden || row_bytes == hidden / 2)) {
+    const MapKey halves{base, inter, row_bytes, 16u, 2u};
+    TK100_TRY(encode_swiglu_map(halves, &map));
+    pinned_maps_[halves] = map;
+  }
   return TK100_OK;
 }
 
@@ -282,26 +294,36 @@ Status Context::scale_map(const void* base, uint64_t chunks, CUtensorMap* out) {
   return TK100_OK;
 }
 
-Status Context::swiglu_map(const void* base, uint64_t outputs, uint64_t row_bytes, CUtensorMap* out) {
-  const MapKey key{base, outputs, row_bytes, 16u, 2u};
-  auto it = maps_.find(key);
-  if (it != maps_.end()) {
-    *out = it->second;
-    return TK100_OK;
-  }
+Status Context::encode_swiglu_map(const MapKey& key, CUtensorMap* out) {
   auto encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(encode_fn_);
-  CUtensorMap map;
-  const cuuint64_t dims[4] = {row_bytes, 32, 2, outputs / 32};
-  const cuuint64_t strides[3] = {row_bytes, outputs * row_bytes, 32 * row_bytes};
+  const cuuint64_t dims[4] = {key.row_bytes, 32, 2, key.rows / 32};
+  const cuuint64_t strides[3] = {key.row_bytes, key.rows * key.row_bytes, 32 * key.row_bytes};
   const cuuint32_t box[4] = {128u, 16u, 2u, 4u};
   const cuuint32_t elem[4] = {1u, 1u, 1u, 1u};
-  CUresult r = encode(&map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, const_cast<void*>(base), dims, strides, box, elem,
+  CUresult r = encode(out, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, const_cast<void*>(key.base), dims, strides, box, elem,
                       CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
     return fail(TK100_ERR_DRIVER, "[gpu.driver] cuTensorMapEncodeTiled (gate/up plane) failed with CUresult " +
                                       std::to_string(static_cast<int>(r)));
   }
+  return TK100_OK;
+}
+
+Status Context::swiglu_map(const void* base, uint64_t outputs, uint64_t row_bytes, CUtensorMap* out) {
+  const MapKey key{base, outputs, row_bytes, 16u, 2u};
+  auto pinned = pinned_maps_.find(key);
+  if (pinned != pinned_maps_.end()) {
+    *out = pinned->second;
+    return TK100_OK;
+  }
+  auto it = maps_.find(key);
+  if (it != maps_.end()) {
+    *out = it->second;
+    return TK100_OK;
+  }
+  CUtensorMap map;
+  TK100_TRY(encode_swiglu_map(key, &map));
   if (maps_.size() > 4096) maps_.clear();
   maps_.emplace(key, map);
   *out = map;
@@ -363,12 +385,6 @@ Status check_plane(Context& ctx, const char* what, const char* plane, const void
   }
   return TK100_OK;
 }
-
-#define TK100_TRY(expr)                  \
-  do {                                   \
-    Status _s = (expr);                  \
-    if (_s != TK100_OK) return _s;       \
-  } while (0)
 
 }  // namespace
 

@@ -163,9 +163,11 @@ class Context {
   // Maps of declared weight planes: encoded once by tk100_register_plane, never evicted.
   std::unordered_map<MapKey, CUtensorMap, MapKeyHash> pinned_maps_;
   Status encode_map(const MapKey& key, CUtensorMap* out);
+  Status encode_swiglu_map(const MapKey& key, CUtensorMap* out);
 
  public:
-  // Encodes the 128-row-box map of a weight-code plane ahead of its first launch.
+  // Encodes the maps of a weight-code plane ahead of its first launch: the 128-row box, and for a plane
+  // of the shape of gate/up weights the interleaved halves.
   Status register_plane(const void* base, uint64_t rows, uint64_t row_bytes);
   size_t pinned_map_count() const { return pinned_maps_.size(); }
   size_t transient_map_count() const { return maps_.size(); }
