@@ -68,6 +68,37 @@ def test_fp8_projection(tk, oracle, monkeypatch, out_rows, k, rows, tok, splits)
     assert c.device_status() == 0
 
 
+@pytest.mark.parametrize("out_rows,k,rows,kernel", [
+    (1040, 3072, 48, "fp8_projection_kernel<64"),    # three splits planned: one-CTA tiles up to 48 tokens
+    (1040, 3072, 49, "fp8_pair_persist_kernel"),
+    (1040, 2048, 48, "fp8_pair_persist_kernel"),     # two splits planned
+    (1040, 4096, 64, "fp8_projection_kernel<64"),    # four splits planned: up to 64
+    (1040, 4096, 65, "fp8_pair_persist_kernel"),
+    (768, 4096, 64, "fp8_pair_persist_kernel"),
+    (4096, 6144, 64, "fp8_projection_kernel<64"),    # three splits, but a long K
+    (4096, 3072, 33, "fp8_projection_kernel<64"),    # most rows of the rule
+    (4112, 3072, 33, "fp8_pair_persist_kernel"),
+])
+def test_fp8_projection_route_rules(tk, oracle, out_rows, k, rows, kernel):
+    """Both sides of each line between the pair kernel and the kernels it leaves a launch to."""
+    from tuiskollm_b200 import synth
+
+    c = tk.Context(device=0)
+    xb = synth.normal_bf16(64, rows, (rows, k))
+    w, s = synth.torch_fp8_weights(64, out_rows, out_rows, k, "cuda")
+    codes = torch.zeros((rows, k), dtype=torch.uint8, device="cuda")
+    scales = torch.zeros((rows,), dtype=torch.float32, device="cuda")
+    out = sentinel_plane((rows + 1, out_rows), torch.int16)
+    tk.ops.Fp8ProjectionOp(c).launch(None, rows, out_rows, k, dev(xb.view(np.int16)), codes, scales, w, s, out)
+    torch.cuda.synchronize()
+    assert c.last_kernel.startswith(kernel), c.last_kernel
+    oc, os_ = oracle.quantize_e4m3(xb)
+    exp = oracle.fp8_projection(oc, os_, host(w), _u16(s))
+    assert max_relative_error(_u16(out)[:rows], exp, 4 * float(np.abs(exp).mean())) <= 1e-2
+    assert_inactive_untouched(out, rows)
+    assert c.device_status() == 0
+
+
 @pytest.mark.parametrize("rows,tok,splits", [(33, 0, 0), (96, 0, 0), (129, 0, 0), (257, 0, 0), (300, 32, 0), (40, 0, 3)])
 def test_fp8_swiglu(tk, oracle, monkeypatch, rows, tok, splits):
     from tuiskollm_b200 import synth

@@ -439,6 +439,18 @@ PairPlan plan_pairs(const Context& ctx, int rows, int row_units, int nkb, bool n
   return best;  // an unsplit plan is always admitted
 }
 
+// FP8 projections of 33 to 64 tokens whose weight rows are few and whose K is long run better on the
+// one-CTA kernel: a cluster holds four pairs, so the plan's splits occupy at most 2 x 4 x 16 SMs with
+// one 256-row tile each, where eight splits of 128-row tiles occupy all (that kernel cannot place more
+// than 32 tiles of eight splits at once: 4608 rows, 41 tokens, K 5120 pairs 8.6, one CTA 11.9 us).
+// Pairs / one CTA, us: 41 tokens, K 5120: 1024 rows 6.4 / 5.4, 3072 rows 8.0 / 6.8, 4096 rows 8.2 / 7.9;
+// 64 tokens: 3072 rows 8.1 / 7.7, 4096 rows 8.3 / 8.8; K 2048 (two splits), 1024 rows, 41 tokens: 4.7 / 4.6.
+// (4096 rows plan three splits; K 17408, 49 tokens: 16.4 / 15.7.)
+bool better_on_one_cta_tiles(const PairPlan& plan, int rows, int out_rows, int k) {
+  if (out_rows > 4096 || plan.splits < 3) return false;
+  return rows <= 48 || (rows <= 64 && out_rows >= 1024 && (plan.splits == 4 || k >= 6144));
+}
+
 PairGemmParams pair_params(Context& ctx, const PairPlan& plan, int rows, int out_rows, int k, int row_units, bool nvfp4,
                            const void* out) {
   PairGemmParams q{};
@@ -835,20 +847,23 @@ Status Fp8ProjectionOp::launch(cudaStream_t stream, int rows, int out_rows, int 
       const bool may_split = tune.fp8_stream_k != 0 || (tune.fp8_persist < 0 && tune.fp8_pair == 1);
       const PairPlan plan = plan_pairs(ctx_, rows, row_units, nkb, false, static_cast<double>(out_rows) * columns,
                                        may_split);
-      CUtensorMap map_w, map_a;
-      TK100_TRY(ctx_.tensor_map(weight_codes, static_cast<uint64_t>(out_rows), static_cast<uint64_t>(columns), 128,
-                                &map_w));
-      TK100_TRY(ctx_.tensor_map(activation_codes, static_cast<uint64_t>(rows), static_cast<uint64_t>(columns),
-                                static_cast<uint32_t>(plan.tok_tile / 2), &map_a));
-      PairGemmParams q = pair_params(ctx_, plan, rows, out_rows, columns, row_units, false, output);
-      q.act_scales = activation_scales;
-      q.w_scales = weight_scales;
-      q.out = output;
-      ctx_.count_launch();
-      ctx_.note_route(tune.fp8_stream_k != 0 ? "fp8_pair_stream_k_kernel" : "fp8_pair_persist_kernel", plan.tok_tile,
-                      plan.workers, plan.splits, 1);
-      return ctx_.check(launch_pair_gemm(stream, false, false, plan.workers, map_w, map_a, map_w, map_a, q),
-                        "launching the persistent FP8 pair projection");
+      const bool by_rule = tune.fp8_persist < 0 && tune.fp8_stream_k == 0 && tune.pair_tok == 0 && tune.pair_splits == 0;
+      if (!by_rule || !better_on_one_cta_tiles(plan, rows, out_rows, columns)) {
+        CUtensorMap map_w, map_a;
+        TK100_TRY(ctx_.tensor_map(weight_codes, static_cast<uint64_t>(out_rows), static_cast<uint64_t>(columns), 128,
+                                  &map_w));
+        TK100_TRY(ctx_.tensor_map(activation_codes, static_cast<uint64_t>(rows), static_cast<uint64_t>(columns),
+                                  static_cast<uint32_t>(plan.tok_tile / 2), &map_a));
+        PairGemmParams q = pair_params(ctx_, plan, rows, out_rows, columns, row_units, false, output);
+        q.act_scales = activation_scales;
+        q.w_scales = weight_scales;
+        q.out = output;
+        ctx_.count_launch();
+        ctx_.note_route(tune.fp8_stream_k != 0 ? "fp8_pair_stream_k_kernel" : "fp8_pair_persist_kernel", plan.tok_tile,
+                        plan.workers, plan.splits, 1);
+        return ctx_.check(launch_pair_gemm(stream, false, false, plan.workers, map_w, map_a, map_w, map_a, q),
+                          "launching the persistent FP8 pair projection");
+      }
     }
   }
 
