@@ -78,6 +78,15 @@ def test_fp8_projection(tk, oracle, monkeypatch, out_rows, k, rows, tok, splits)
     (4096, 6144, 64, "fp8_projection_kernel<64"),    # three splits, but a long K
     (4096, 3072, 33, "fp8_projection_kernel<64"),    # most rows of the rule
     (4112, 3072, 33, "fp8_pair_persist_kernel"),
+    (5120, 256, 641, "fp8_pair_kernel"),             # 60 tiles in one wave, planned at 224 tokens
+    (5120, 256, 576, "fp8_pair_persist_kernel"),     # ... at 192
+    (5136, 256, 700, "fp8_pair_persist_kernel"),     # weight rows end inside a tile
+    (8192, 2176, 256, "fp8_pair_kernel"),            # two splits planned
+    (12288, 256, 256, "fp8_pair_kernel"),            # one wave where the plan takes two
+    (8192, 512, 630, "fp8_pair_kernel"),             # 96 tiles in two waves of 160 tokens: K up to 512
+    (8192, 640, 630, "fp8_pair_persist_kernel"),
+    (2560, 512, 2048, "fp8_pair_persist_kernel"),    # a second wave mostly empty
+    (8192, 256, 1281, "fp8_pair_persist_kernel"),    # more tiles than two waves hold
 ])
 def test_fp8_projection_route_rules(tk, oracle, out_rows, k, rows, kernel):
     """Both sides of each line between the pair kernel and the kernels it leaves a launch to."""

@@ -451,6 +451,32 @@ bool better_on_one_cta_tiles(const PairPlan& plan, int rows, int out_rows, int k
   return rows <= 48 || (rows <= 64 && out_rows >= 1024 && (plan.splits == 4 || k >= 6144));
 }
 
+// FP8 projections of a short K whose wide tiles fill their wave run better with one 256-token tile per
+// pair (fp8_pair.cu): there is no next tile's K loop to hide a wide tile's epilogue under, and two pairs
+// share two SMs there, so twice the `resident` pairs of the persistent kernel run at once.  The lines lie
+// where the two are equal on 1508 launches (256 to 14336 rows, 256 to 2048 tokens, K 256 to 5120): with
+// them 15 launches are more than 3 % (at most 9 %, K 256) slower than the faster of the two, without 312.
+// Persistent / one tile per pair, us: one wave, 5120 rows, 768 tokens: K 768 8.3 / 7.7, K 2176 11.7 /
+// 11.2; 12288 rows, 256 tokens, K 3072 15.9 / 14.3; two splits, 8192 rows, 256 tokens, K 2176 11.1 / 10.1;
+// two pairs per two SMs, 8192 rows, 1024 tokens: K 1024 12.7 / 11.4, K 2176 15.3 / 15.5; 2560 rows, 2048
+// tokens, K 768 (a second wave three quarters empty) 8.9 / 10.0; 160 tiles, 8192 rows, 1280 tokens, K 768
+// 13.9 / 16.9.
+bool better_on_single_pair_tiles(const PairPlan& plan, int rows, int out_rows, int k, int resident) {
+  if (out_rows % 256 != 0 || plan.splits > 2) return false;
+  const int units = out_rows / 256, tok = plan.tok_tile;
+  const int tiles = units * ((rows + 255) / 256);
+  if (plan.splits == 2) return tiles <= resident && tok == 256 && k <= 2176;
+  if (tiles <= resident) {
+    if (2 * tiles <= resident) return false;
+    return k <= (tok == 256 ? 3072 : tok == 224 ? 1024 : plan.tiles_m * units > resident ? 256 : 0);
+  }
+  if (tiles <= 2 * resident) {
+    const bool filled = rows * units >= 1.51 * resident * tok || k <= 256;  // 3/4 of two waves of `tok`
+    return filled && tok >= 160 && k <= (tok == 256 ? 1536 : 8 * (tok - 96));
+  }
+  return tok == 256 && k <= 256;
+}
+
 PairGemmParams pair_params(Context& ctx, const PairPlan& plan, int rows, int out_rows, int k, int row_units, bool nvfp4,
                            const void* out) {
   PairGemmParams q{};
@@ -836,6 +862,7 @@ Status Fp8ProjectionOp::launch(cudaStream_t stream, int rows, int out_rows, int 
   }
 
   // More than a few dozen tokens with a plain BF16 output: persistent CTA pairs.
+  bool one_tile_per_pair = false;
   {
     const Tuning& tune = ctx_.tuning();
     const bool wanted = tune.fp8_persist > 0 || tune.fp8_stream_k != 0 ||
@@ -848,7 +875,9 @@ Status Fp8ProjectionOp::launch(cudaStream_t stream, int rows, int out_rows, int 
       const PairPlan plan = plan_pairs(ctx_, rows, row_units, nkb, false, static_cast<double>(out_rows) * columns,
                                        may_split);
       const bool by_rule = tune.fp8_persist < 0 && tune.fp8_stream_k == 0 && tune.pair_tok == 0 && tune.pair_splits == 0;
-      if (!by_rule || !better_on_one_cta_tiles(plan, rows, out_rows, columns)) {
+      one_tile_per_pair = by_rule && rows >= tune.fp8_pair_min_rows &&
+                          better_on_single_pair_tiles(plan, rows, out_rows, columns, ctx_.pair_clusters(1));
+      if (!by_rule || !(one_tile_per_pair || better_on_one_cta_tiles(plan, rows, out_rows, columns))) {
         CUtensorMap map_w, map_a;
         TK100_TRY(ctx_.tensor_map(weight_codes, static_cast<uint64_t>(out_rows), static_cast<uint64_t>(columns), 128,
                                   &map_w));
@@ -867,7 +896,7 @@ Status Fp8ProjectionOp::launch(cudaStream_t stream, int rows, int out_rows, int 
     }
   }
 
-  // TK100_FP8_PERSIST=0: one pair tile (256 rows x 256 tokens) per CTA pair.
+  // A short K, or TK100_FP8_PERSIST=0: one pair tile (256 rows x 256 tokens) per CTA pair.
   {
     const Tuning& tune = ctx_.tuning();
     const int min_rows = tune.fp8_pair_min_rows;
@@ -880,7 +909,7 @@ Status Fp8ProjectionOp::launch(cudaStream_t stream, int rows, int out_rows, int 
     // there (measured 44.6 against 57.0 us).
     const bool long_k_few_tiles = pair_ctas < ctx_.sm_count() / 2 && columns >= 16384;
     if (tune.fp8_pair != 0 && rows >= min_rows && out_rows % 256 == 0 &&
-        ((pair_ctas >= 32 && !long_k_few_tiles) || tune.fp8_pair == 2) && output &&
+        ((pair_ctas >= 32 && !long_k_few_tiles) || tune.fp8_pair == 2 || one_tile_per_pair) && output &&
         !logits_f32 && !argmax_scratch && ctx_.forced_block_tok() == 0 && ctx_.forced_splits() == 0) {
       CUtensorMap map_w, map_a;
       TK100_TRY(ctx_.tensor_map(weight_codes, static_cast<uint64_t>(out_rows),
