@@ -191,6 +191,45 @@ def test_nvfp4_mlp(tk, oracle, monkeypatch, hidden, inter, rows, tok, splits):
         assert_inactive_untouched(plane, rows)
 
 
+@pytest.mark.parametrize("hidden,inter,rows,kernel", [
+    (5120, 6144, 33, "nvfp4_gemm_kernel"),      # three splits planned
+    (5120, 6144, 64, "nvfp4_gemm_kernel"),
+    (5120, 6144, 65, "nvfp4_persist_kernel"),
+    (5120, 4352, 33, "nvfp4_persist_kernel"),   # two
+    (1024, 2176, 80, "nvfp4_gemm_kernel"),      # few weight rows
+    (1024, 2176, 81, "nvfp4_persist_kernel"),
+    (1024, 2048, 64, "nvfp4_persist_kernel"),
+    (1280, 2176, 64, "nvfp4_persist_kernel"),
+])
+def test_nvfp4_down_route_rules(tk, oracle, hidden, inter, rows, kernel):
+    """Both sides of each line between the pair kernel and the one-CTA kernel, in both output types."""
+    from tuiskollm_b200 import synth
+
+    xb = synth.normal_bf16(65, rows, (rows, inter))
+    dn, dns, dnd = synth.torch_nvfp4_weights(65, 2, hidden, inter, "cuda")
+    div = float(np.float32(448.0 * 6.0 / 8.0))
+    c = tk.Context(device=0, hidden=hidden, intermediate=inter)
+    codes, scales = _nvfp4_planes(tk, rows, inter)
+    out = sentinel_plane((rows + 1, hidden), torch.int16)
+    part = sentinel_plane((rows + 1, hidden), torch.float32)
+    down = tk.Nvfp4DownOp(c)
+    kw = dict(activation_codes=codes, activation_scales=scales, input_global_divisor=div)
+    down.launch(None, rows, dev(xb.view(np.int16)), dn, dns, float(dnd), out, **kw)
+    assert c.last_kernel.startswith(kernel), c.last_kernel
+    down.launch_partial(None, rows, None, dn, dns, float(dnd), part, **kw)
+    assert c.last_kernel.startswith(kernel), c.last_kernel
+    torch.cuda.synchronize()
+    oc, osc = oracle.nvfp4_quantize(xb, div)
+    exp = oracle.nvfp4_w4a4_dot(oc, osc, div, host(dn), host(dns), float(dnd))
+    floor = 4 * float(np.abs(exp).mean())
+    assert max_relative_error(_u16(out)[:rows], exp, floor) <= 1e-2
+    got32 = host(part)[:rows]
+    assert (np.abs(got32 - exp) / np.maximum(np.abs(exp), floor)).max() <= 2e-3
+    for plane in (out, part):
+        assert_inactive_untouched(plane, rows)
+    assert c.device_status() == 0
+
+
 def test_quantised_output_planes_are_held_to_the_quantisers_alignment(tk):
     """More than 32 rows: what the quantiser launch refuses, the epilogue's quantisation refuses."""
     rows, hidden, inter = 40, 256, 256

@@ -477,6 +477,16 @@ bool better_on_single_pair_tiles(const PairPlan& plan, int rows, int out_rows, i
   return tok == 256 && k <= 256;
 }
 
+// NVFP4 down projections of 33 to 64 (80) tokens with a long K (few weight rows) run better on the one-CTA
+// kernel, which has twice the tiles and up to eight splits of each.  Pairs / one CTA, us:
+// 40 tokens: 512 x 8704 7.2 / 5.4, 1024 x 2176 5.1 / 4.6, 3072 x 8704 9.1 / 7.4, 5120 x 8704 10.1 / 8.9,
+// 5120 x 4352 (two splits) 7.2 / 8.6; 5120 x 8704: 64 tokens 10.2 / 9.8, 80 tokens 10.4 / 10.6;
+// 512 x 3072, 80 tokens 6.5 / 5.6.
+bool better_on_split_tiles(const PairPlan& plan, int rows, int out_rows, int k) {
+  if (out_rows <= 1024) return rows <= 80 && k >= 2176;
+  return rows <= 64 && plan.splits >= 3;
+}
+
 PairGemmParams pair_params(Context& ctx, const PairPlan& plan, int rows, int out_rows, int k, int row_units, bool nvfp4,
                            const void* out) {
   PairGemmParams q{};
@@ -1259,35 +1269,38 @@ Status Nvfp4MlpOp::launch(cudaStream_t stream, bool gate_up, int rows, int out_r
     const uint64_t chunks_per_tile = static_cast<uint64_t>(columns / 64);
     const PairPlan plan = plan_pairs(ctx_, rows, row_units, (columns + 255) / 256, true,
                                      static_cast<double>(w_rows) * columns * 9 / 16, !gate_up && tune.nvfp4_persist < 0);
-    CUtensorMap map_w, map_a, map_wsf, map_asf;
-    if (gate_up) {
-      TK100_TRY(ctx_.swiglu_map(weight_codes, static_cast<uint64_t>(out_rows), static_cast<uint64_t>(columns / 2), &map_w));
-      TK100_TRY(ctx_.swiglu_scale_map(weight_scales, static_cast<uint64_t>(out_rows), chunks_per_tile, &map_wsf));
-    } else {
-      TK100_TRY(ctx_.tensor_map(weight_codes, w_rows, static_cast<uint64_t>(columns / 2), 128, &map_w));
-      TK100_TRY(ctx_.scale_map(weight_scales, (w_rows / 128) * chunks_per_tile, &map_wsf));
+    const bool by_rule = tune.nvfp4_persist < 0 && tune.pair_tok == 0 && tune.pair_splits == 0;
+    if (gate_up || !by_rule || !better_on_split_tiles(plan, rows, out_rows, columns)) {
+      CUtensorMap map_w, map_a, map_wsf, map_asf;
+      if (gate_up) {
+        TK100_TRY(ctx_.swiglu_map(weight_codes, static_cast<uint64_t>(out_rows), static_cast<uint64_t>(columns / 2), &map_w));
+        TK100_TRY(ctx_.swiglu_scale_map(weight_scales, static_cast<uint64_t>(out_rows), chunks_per_tile, &map_wsf));
+      } else {
+        TK100_TRY(ctx_.tensor_map(weight_codes, w_rows, static_cast<uint64_t>(columns / 2), 128, &map_w));
+        TK100_TRY(ctx_.scale_map(weight_scales, (w_rows / 128) * chunks_per_tile, &map_wsf));
+      }
+      TK100_TRY(ctx_.tensor_map(activation_codes, static_cast<uint64_t>(rows), static_cast<uint64_t>(columns / 2),
+                                static_cast<uint32_t>(plan.tok_tile / 2), &map_a));
+      TK100_TRY(ctx_.scale_map(activation_scales, static_cast<uint64_t>((rows + 127) / 128) * chunks_per_tile, &map_asf));
+      PairGemmParams q = pair_params(ctx_, plan, rows, out_rows, columns, row_units, true, output);
+      q.out_scale = 1.0f / (weight_scale_divisor * input_global_divisor);
+      q.out = output;
+      q.out_f32 = output_f32;
+      if (next) {
+        // the planes the quantiser launch of the other routes takes at these sizes, and no others
+        const char* quantiser = "NVFP4 activation quantiser";
+        TK100_TRY(check_plane(ctx_, quantiser, "input", output, 32));
+        TK100_TRY(check_plane(ctx_, quantiser, "activation codes", next->codes, 128));
+        TK100_TRY(check_plane(ctx_, quantiser, "activation scales", next->scales, 128));
+        q.q_codes = next->codes;
+        q.q_scales = next->scales;
+        q.q_divisor = next->divisor;
+      }
+      ctx_.count_launch();
+      ctx_.note_route("nvfp4_persist_kernel", plan.tok_tile, plan.workers, plan.splits, 1);
+      return ctx_.check(launch_pair_gemm(stream, true, gate_up, plan.workers, map_w, map_a, map_wsf, map_asf, q),
+                        "launching the persistent NVFP4 projection");
     }
-    TK100_TRY(ctx_.tensor_map(activation_codes, static_cast<uint64_t>(rows), static_cast<uint64_t>(columns / 2),
-                              static_cast<uint32_t>(plan.tok_tile / 2), &map_a));
-    TK100_TRY(ctx_.scale_map(activation_scales, static_cast<uint64_t>((rows + 127) / 128) * chunks_per_tile, &map_asf));
-    PairGemmParams q = pair_params(ctx_, plan, rows, out_rows, columns, row_units, true, output);
-    q.out_scale = 1.0f / (weight_scale_divisor * input_global_divisor);
-    q.out = output;
-    q.out_f32 = output_f32;
-    if (next) {
-      // the planes the quantiser launch of the other routes takes at these sizes, and no others
-      const char* quantiser = "NVFP4 activation quantiser";
-      TK100_TRY(check_plane(ctx_, quantiser, "input", output, 32));
-      TK100_TRY(check_plane(ctx_, quantiser, "activation codes", next->codes, 128));
-      TK100_TRY(check_plane(ctx_, quantiser, "activation scales", next->scales, 128));
-      q.q_codes = next->codes;
-      q.q_scales = next->scales;
-      q.q_divisor = next->divisor;
-    }
-    ctx_.count_launch();
-    ctx_.note_route("nvfp4_persist_kernel", plan.tok_tile, plan.workers, plan.splits, 1);
-    return ctx_.check(launch_pair_gemm(stream, true, gate_up, plan.workers, map_w, map_a, map_wsf, map_asf, q),
-                      "launching the persistent NVFP4 projection");
   }
   // 256-token tiles (one CTA per SM, a third fewer operand bytes and issue slots per MAC) for
   // prefill shapes: the plain projection unsplit, and the gate/up pairs.
