@@ -6,7 +6,7 @@ import types
 import pytest
 import torch
 
-from tuiskollm_b200 import _lib, ops
+from tuiskollm_b200 import _lib, build, ops
 
 
 @pytest.fixture
@@ -89,6 +89,16 @@ def test_the_general_call_reports_as_before():
     assert info.value.code == "gpu.context"
     with pytest.raises(C.ArgumentError):
         _lib.native(ops._launch).tk100_rms_norm(c, 0, 1.5, 1, 2, 3)
+
+
+def test_a_binding_of_another_torch_or_interpreter_is_not_taken(monkeypatch):
+    build.build_binding()
+    assert not build.binding_is_stale()
+    monkeypatch.setattr(torch, "__version__", "0.0.1")
+    assert build.binding_is_stale()
+    monkeypatch.undo()
+    monkeypatch.setattr(build.sysconfig, "get_config_var", lambda name: ".other.so")
+    assert build.binding_is_stale()
 
 
 @pytest.mark.gpu

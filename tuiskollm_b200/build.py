@@ -1,5 +1,5 @@
 """Builds ``libtuisko_sm100.so`` in-tree with nvcc for sm_100a (the only target), and the CPython
-binding of its launches (``_native.so``) with the host compiler."""
+binding of its launches (``_native.<torch version><extension suffix>``) with the host compiler."""
 from __future__ import annotations
 
 import importlib.util
@@ -12,7 +12,6 @@ import sysconfig
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libtuisko_sm100.so")
-BINDING = os.path.join(HERE, "_native.so")
 BINDING_SOURCE = os.path.join(CSRC, "binding.cpp")
 SOURCES = ["norm_quant.cu", "fp8_proj.cu", "fp8_pair.cu", "fp8_mlp.cu", "gdn.cu", "materialize.cu", "nvfp4.cu", "nvfp4_pair.cu", "pair_gemm.cu", "peer_reduce.cu", "sampler.cu", "ops.cu", "static_entry.cu"]
 HEADERS = ["common.cuh", "ptx.cuh", "kernels.h", "ops.hpp", "../../include/tuisko_sm100.h"]
@@ -33,10 +32,19 @@ def is_stale() -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def binding_path() -> str:
+    """Named after what it is compiled against -- torch's C++ ABI and the interpreter's -- so that a copy
+    built for another of either is not taken for this one's."""
+    import torch
+
+    return os.path.join(HERE, "_native.%s%s" % (torch.__version__, sysconfig.get_config_var("EXT_SUFFIX")))
+
+
 def binding_is_stale() -> bool:
-    if not os.path.exists(BINDING):
+    path = binding_path()
+    if not os.path.exists(path):
         return True
-    t = os.path.getmtime(BINDING)
+    t = os.path.getmtime(path)
     deps = [BINDING_SOURCE, os.path.abspath(os.path.join(CSRC, "../../include/tuisko_sm100.h")),
             importlib.util.find_spec("torch").origin]  # compiled against this torch's headers
     return any(os.path.getmtime(d) > t for d in deps)
@@ -51,7 +59,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
 
 def build_binding(force: bool = False, verbose: bool = False) -> str:
     """The same for the launch binding."""
-    return _build_locked(BINDING, binding_is_stale, _compile_binding, force, verbose)
+    return _build_locked(binding_path(), binding_is_stale, _compile_binding, force, verbose)
 
 
 def _build_locked(path, stale, compile_it, force, verbose) -> str:
@@ -89,7 +97,8 @@ def _compile(verbose: bool) -> str:
 
 
 def _compile_binding(verbose: bool) -> str:
-    tmp = "%s.%d.tmp" % (BINDING, os.getpid())
+    path = binding_path()
+    tmp = "%s.%d.tmp" % (path, os.getpid())
     torch_dir = os.path.dirname(importlib.util.find_spec("torch").origin)
     cuda = os.path.dirname(os.path.dirname(os.path.realpath(nvcc_path())))
     cxx = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else os.environ.get("CXX", "g++")
@@ -98,7 +107,7 @@ def _compile_binding(verbose: bool) -> str:
                                os.path.join(torch_dir, "include/torch/csrc/api/include"),
                                sysconfig.get_paths()["include"], os.path.join(cuda, "include"))]
     cmd += ["-L" + os.path.join(torch_dir, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
-    return _run(cmd, tmp, BINDING, verbose)
+    return _run(cmd, tmp, path, verbose)
 
 
 def _run(cmd, tmp, path, verbose) -> str:
