@@ -101,6 +101,19 @@ def test_a_binding_of_another_torch_or_interpreter_is_not_taken(monkeypatch):
     assert build.binding_is_stale()
 
 
+def test_without_a_binding_launches_take_the_general_call(monkeypatch):
+    def fails(*_):
+        raise RuntimeError("no compiler")
+
+    monkeypatch.setattr(_lib, "_native", None)
+    monkeypatch.setattr(build, "build_binding", fails)
+    calls = []
+    with pytest.warns(RuntimeWarning, match="no compiler"):
+        native = _lib.native(lambda *a: calls.append(a))
+    native.tk100_rms_norm("context", None, 1, 2, 3, 4)
+    assert calls == [("tk100_rms_norm", "context", None, 1, 2, 3, 4)]
+
+
 @pytest.mark.gpu
 def test_tensors_and_streams(recorder):
     native, calls, general = recorder

@@ -6,8 +6,10 @@ that is impossible the import fails loudly.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import importlib.util
 import os
+import warnings
 
 from . import build as _build
 
@@ -115,16 +117,34 @@ def load() -> C.CDLL:
     return _lib
 
 
+class _GeneralLaunches:
+    """Stands in for the compiled binding: every launch takes the general call."""
+
+    def __init__(self, general):
+        self._general = general
+
+    def __getattr__(self, name):
+        return functools.partial(self._general, name)
+
+
 def native(general):
     """The compiled launch binding, bound to the loaded library's functions; ``general(name, context,
-    stream, *arguments)`` takes the calls it does not read itself."""
+    stream, *arguments)`` takes the calls it does not read itself.  Where the binding cannot be built
+    (no host compiler or torch headers), ``general`` takes all of them, after a warning: the launches
+    are the same, a call costs the host about 6 us more."""
     global _native
     if _native is None:
         lib = load()
-        path = _build.build_binding()
-        spec = importlib.util.spec_from_file_location("tuiskollm_b200._native", path)
-        module = importlib.util.module_from_spec(spec)
-        spec.loader.exec_module(module)
+        try:
+            path = _build.build_binding()
+            spec = importlib.util.spec_from_file_location("tuiskollm_b200._native", path)
+            module = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(module)
+        except (RuntimeError, OSError, ImportError) as exc:
+            warnings.warn("launches go through ctypes: the compiled binding is not available (%s)" % exc,
+                          RuntimeWarning, stacklevel=3)
+            _native = _GeneralLaunches(general)
+            return _native
         module.bind(lambda name: C.cast(getattr(lib, name), _vp).value, general)
         _native = module
     return _native
