@@ -97,9 +97,10 @@ TK100_API const char* tk100_last_error(const tk100_ctx* ctx);
 TK100_API tk100_status tk100_device_status(tk100_ctx* ctx, tk100_stream stream, uint32_t* word);
 /* Number of kernels this context has launched (for launch accounting). */
 TK100_API uint64_t tk100_launch_count(const tk100_ctx* ctx);
-/* Name of the kernel instantiation the last projection launch on this context took, e.g.
- * "fp8_projection_kernel<16,1> splits=1" (token tile, ring variant) -- for reports and route
- * tests; valid until the next call.  No counterpart in the reference. */
+/* Name of the kernel the last projection launch on this context took with two of its parameters and
+ * its K splits, e.g. "fp8_projection_kernel<16,1> splits=1" (token tile, ring variant) or
+ * "pair_gemm_kernel<160,40> splits=1 cluster" (token tile, resident clusters) -- for reports and
+ * route tests; valid until the next call.  No counterpart in the reference. */
 TK100_API const char* tk100_last_kernel(tk100_ctx* ctx);
 
 /* Declares a weight-code plane (`rows` x `row_bytes` bytes, 128-byte aligned: an FP8 plane has

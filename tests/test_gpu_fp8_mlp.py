@@ -88,7 +88,7 @@ def test_reference_fixture_fp8_swiglu(tk, ctx, oracle, swiglu_weights, rows):
     launch = lambda: op.launch(None, rows, x, planes.codes, planes.scales, w, s, planes.out)
     launch()
     torch.cuda.synchronize()
-    assert ctx.last_kernel.startswith("fp8_swiglu_kernel")
+    assert ctx.last_kernel.startswith("fp8_swiglu_kernel" if rows <= 32 else "pair_gemm_kernel"), ctx.last_kernel
     reps = check_quantiser(oracle, xb, planes, rows)
     got = _u16(planes.out)
     for t, (rsum, sc) in enumerate(reps):
@@ -141,13 +141,16 @@ def test_reference_fixture_gdn_output(tk, ctx, oracle, rows):
     assert ctx.device_status() == 0
 
 
-@pytest.mark.parametrize("rows", [1, 20, 33, 200, 300])
-def test_fp8_mlp_random_planes_match_oracle(tk, oracle, rows):
+@pytest.mark.parametrize("rows,persist", [(1, "-1"), (20, "-1"), (33, "-1"), (200, "-1"), (300, "-1"), (33, "0"), (200, "0"),
+                                          (300, "0")])
+def test_fp8_mlp_random_planes_match_oracle(tk, oracle, rows, persist, monkeypatch):
     """Seeded ~N(0,1) activations and ~N(0,0.02) weights on a small geometry, ragged token counts
-    (both token tiles, zero-filled tile tails): SwiGLU -> down through the two operators, each
-    stage against the f64 oracle of the codes it consumed, within 1e-2."""
+    (zero-filled tile tails): SwiGLU -> down through the two operators, each stage against the
+    f64 oracle of the codes it consumed, within 1e-2.  TK100_FP8_PERSIST=0 runs more than 32
+    tokens on the kernels' 128-token tiles instead of persistent pairs."""
     from tuiskollm_b200 import synth
 
+    monkeypatch.setenv("TK100_FP8_PERSIST", persist)
     hidden, inter = 1024, 1536
     c = tk.Context(device=0, hidden=hidden, intermediate=inter, max_rows=512)
     xb = synth.normal_bf16(51, rows, (rows, hidden))
@@ -157,6 +160,7 @@ def test_fp8_mlp_random_planes_match_oracle(tk, oracle, rows):
     p2 = Planes(rows + 1, inter, hidden)
     tk.Fp8SwiGluOp(c).launch(None, rows, dev(xb.view(np.int16)), p1.codes, p1.scales, dev(gu_c),
                              dev(gu_s.view(np.int16)), p1.out)
+    assert c.last_kernel.startswith("pair_gemm_kernel") == (rows > 32 and persist == "-1"), c.last_kernel
     tk.Fp8DownOp(c).launch(None, rows, p1.out, p2.codes, p2.scales, dev(dn_c), dev(dn_s.view(np.int16)),
                            p2.out)
     torch.cuda.synchronize()
@@ -197,9 +201,8 @@ def test_fp8_swiglu_rejected_launches(tk, ctx):
 
 @pytest.mark.parametrize("rows", [256, 512])
 def test_benchmarked_fp8_down_and_gdn_output_sampled_rows(tk, ctx, oracle, rows):
-    """The benchmarked batched shapes of the dense-FP8 down projection (K = 17408: at 256 tokens
-    the one-CTA kernel with K split over clusters, at 512 the CTA pairs) and of the GDN output
-    projection at full size: quantiser bit-exact, sampled output rows (first, middle and last
+    """The benchmarked batched shapes of the dense-FP8 down projection (K = 17408) and of the GDN
+    output projection at full size, on persistent CTA pairs: quantiser bit-exact, sampled output rows (first, middle and last
     128-row tile) of every token against the f64 oracle within 1e-2."""
     from tuiskollm_b200 import synth
 
@@ -214,6 +217,7 @@ def test_benchmarked_fp8_down_and_gdn_output_sampled_rows(tk, ctx, oracle, rows)
             tk.GdnOutputProjectionOp(ctx, columns).launch(None, rows, dev(xb.view(np.int16)), planes.codes,
                                                           planes.scales, w, s, planes.out)
         route = ctx.last_kernel
+        assert route.startswith("pair_gemm_kernel"), route
         torch.cuda.synchronize()
         oc, os_ = oracle.quantize_e4m3(xb)
         assert np.array_equal(host(planes.codes)[:rows], oc), route

@@ -114,16 +114,17 @@ def test_synthetic_configs_match_oracle(tk, ctx, oracle, kind, out_rows, rows):
 
 @pytest.mark.parametrize("out_rows,rows", [(512, 512), (768, 700), (256, 1030), (5120, 600)])
 def test_pair_route_matches_oracle_and_one_cta_route(tk, oracle, out_rows, rows, monkeypatch):
-    """Prefill token counts take the CTA-pair kernel (cta_group::2, 256-row x 256-token pair
-    tiles); ragged token counts exercise the zero-filled tails.  Against the oracle, and against
-    the one-CTA kernel, which splits K at these small sizes: the two may differ by one BF16
-    rounding step, no more."""
+    """The kernel with one 256-row x 256-token tile per CTA pair (cta_group::2; TK100_FP8_PERSIST=0
+    leaves larger launches to it); ragged token counts exercise the zero-filled tails.  Against
+    the oracle, and against the one-CTA kernel, which splits K at these small sizes: the two may
+    differ by one BF16 rounding step, no more."""
     from tuiskollm_b200 import synth
 
     hidden = 1024
     xb = synth.normal_bf16(43, rows, (rows, hidden))
     wc, ws = synth.fp8_weights(43, out_rows, out_rows, hidden)
     outs = {}
+    monkeypatch.setenv("TK100_FP8_PERSIST", "0")
     for route, env in (("pair", "2"), ("single", "0")):  # "2": also for launches of few CTAs
         monkeypatch.setenv("TK100_FP8_PAIR", env)
         ctx = tk.Context(device=0, hidden=hidden, max_rows=2048)
@@ -134,6 +135,8 @@ def test_pair_route_matches_oracle_and_one_cta_route(tk, oracle, out_rows, rows,
             dev(ws.view(np.int16)), planes.out)
         torch.cuda.synchronize()
         assert ctx.launch_count - launches == 2, route  # quantiser + one projection kernel
+        kernel = "fp8_pair_kernel" if route == "pair" else "fp8_projection_kernel"
+        assert ctx.last_kernel.startswith(kernel), ctx.last_kernel
         check_projection(oracle, xb, wc, ws, planes, rows, floor=0.25 * (hidden / 5120) ** 0.5)
         assert ctx.device_status() == 0, route
         outs[route] = _u16(planes.out)[:rows].copy()
@@ -145,7 +148,7 @@ def test_pair_route_matches_oracle_and_one_cta_route(tk, oracle, out_rows, rows,
 @pytest.mark.parametrize("out_rows,rows", [(8192, 512), (8192, 2048), (12288, 512), (12288, 2048)])
 def test_benchmarked_prefill_shapes_sampled_tiles(tk, ctx, oracle, out_rows, rows):
     """The prefill shapes the benchmark times (K = 5120, M = 512 / 2048, N = 8192 / 12288) run on
-    the CTA-pair kernel; the f64 oracle cannot do the whole product in seconds, so whole
+    persistent CTA pairs; the f64 oracle cannot do the whole product in seconds, so whole
     128 x 128 tiles are sampled -- first, last and two inner weight tiles x first, an inner and
     the last token tile -- after the activation codes and scales of ALL rows are checked bit for
     bit."""
@@ -158,7 +161,7 @@ def test_benchmarked_prefill_shapes_sampled_tiles(tk, ctx, oracle, out_rows, row
     tk.GdnInputProjectionOp(ctx, out_rows).launch(None, rows, x, planes.codes, planes.scales, w, s,
                                                   planes.out)
     torch.cuda.synchronize()
-    assert ctx.last_kernel.startswith(("fp8_pair_kernel", "fp8_pair_persist_kernel")), ctx.last_kernel
+    assert ctx.last_kernel.startswith("pair_gemm_kernel"), ctx.last_kernel
     xb = _u16(x)
     oc, os_ = oracle.quantize_e4m3(xb)
     assert np.array_equal(host(planes.codes)[:rows], oc)
@@ -418,7 +421,7 @@ def test_persistent_pair_route_matches_pair_route_bit_for_bit(tk, oracle, out_ro
             dev(ws.view(np.int16)), planes.out)
         torch.cuda.synchronize()
         assert c.device_status() == 0, route
-        assert c.last_kernel.startswith("fp8_pair_persist_kernel") == (route == "persistent"), c.last_kernel
+        assert c.last_kernel.startswith("pair_gemm_kernel" if route == "persistent" else "fp8_pair_kernel"), c.last_kernel
         planes.check_inactive(rows)
         if out_rows == 1024:
             check_projection(oracle, xb, wc, ws, planes, rows, floor=0.25 * (hidden / 5120) ** 0.5)
@@ -426,37 +429,39 @@ def test_persistent_pair_route_matches_pair_route_bit_for_bit(tk, oracle, out_ro
     assert np.array_equal(outs["persistent"], outs["pair"])
 
 
-@pytest.mark.parametrize("out_rows,hidden,rows", [(1024, 1024, 256), (1024, 2048, 700), (4096, 1024, 1300),
-                                                  (5120, 6144, 256), (8192, 5120, 300)])
-def test_stream_k_pair_route(tk, oracle, out_rows, hidden, rows, monkeypatch):
-    """TK100_FP8_STREAMK=1: the resident pairs share the launch's tiles x K steps evenly; a tile
-    whose K range is cut meets in fp32 scratch under a ticket and is summed in K order by whichever
-    CTA arrives last.  The result is the oracle's within the projection tolerance (a split sum is
-    not the unsplit sum's bits, so the pair route is compared within one BF16 step, and tiles that
-    no range cuts bit for bit by construction), ragged token tails included; launches repeat bit
-    for bit, eagerly and as graph replays, and scratch counters re-arm (three launches)."""
+@pytest.mark.parametrize("out_rows,hidden,rows,splits", [(1024, 2048, 256, 2), (1024, 2048, 700, 2), (2048, 4096, 300, 3),
+                                                         (5120, 6144, 256, 3), (8192, 5120, 256, 2)])
+def test_cluster_split_pair_route(tk, oracle, out_rows, hidden, rows, splits, monkeypatch):
+    """TK100_FP8_STREAMK=1: the pairs of a cluster split K and add their parts of a tile in split
+    order over distributed shared memory.  The result is the oracle's within the projection
+    tolerance (whole 128-column tiles of it at the larger sizes), and within one BF16 step of the
+    unsplit one-tile kernel's; launches repeat bit for bit, eagerly and as graph replays."""
     from tuiskollm_b200 import synth
 
     xb = synth.normal_bf16(53, rows, (rows, hidden))
     wc, ws = synth.fp8_weights(53, out_rows + hidden, out_rows, hidden)
+    x, w, s = dev(xb.view(np.int16)), dev(wc), dev(ws.view(np.int16))
     outs = {}
-    for route, env in (("stream_k", "1"), ("pair", "0")):
-        monkeypatch.setenv("TK100_FP8_PAIR", "2")
-        monkeypatch.setenv("TK100_FP8_STREAMK", env)
+    for route, switches in (("split", {"STREAMK": "1"}), ("pair", {"STREAMK": "0", "PERSIST": "0", "PAIR": "2"})):
+        for name in ("STREAMK", "PERSIST", "PAIR"):
+            monkeypatch.delenv("TK100_FP8_" + name, raising=False)
+        for name, value in switches.items():
+            monkeypatch.setenv("TK100_FP8_" + name, value)
+        monkeypatch.setenv("TK100_PAIR_SPLITS", str(splits) if route == "split" else "0")
         c = tk.Context(device=0, hidden=hidden, max_rows=4096)
         planes = Planes(rows + 2, hidden, out_rows)
         op = tk.GdnInputProjectionOp(c, out_rows)
-        x, w, s = dev(xb.view(np.int16)), dev(wc), dev(ws.view(np.int16))
         launch = lambda: op.launch(None, rows, x, planes.codes, planes.scales, w, s, planes.out)
         launch()
         torch.cuda.synchronize()
         assert c.device_status() == 0, route
-        assert c.last_kernel.startswith("fp8_pair_stream_k_kernel") == (route == "stream_k"), c.last_kernel
+        if route == "split":
+            assert c.last_kernel.startswith("pair_gemm_kernel") and f"splits={splits}" in c.last_kernel, c.last_kernel
+        else:
+            assert c.last_kernel.startswith("fp8_pair_kernel"), c.last_kernel
         planes.check_inactive(rows)
-        first = _u16(planes.out)[:rows].copy()
-        if route == "stream_k":
-            if out_rows * rows <= 1024 * 700:
-                check_projection(oracle, xb, wc, ws, planes, rows, floor=0.25 * (hidden / 5120) ** 0.5)
+        outs[route] = first = _u16(planes.out)[:rows].copy()
+        if route == "split":
             for _ in range(2):
                 planes.out.fill_(0x5A5A)
                 launch()
@@ -469,9 +474,14 @@ def test_stream_k_pair_route(tk, oracle, out_rows, hidden, rows, monkeypatch):
             torch.cuda.synchronize()
             assert np.array_equal(_u16(planes.out)[:rows], first)
             assert c.device_status() == 0
-        outs[route] = first
-    a = oracle.bf16_to_f32(outs["stream_k"].reshape(-1)).astype(np.float64)
+    oc, os_ = oracle.quantize_e4m3(xb)
+    tiles = range(out_rows // 128) if out_rows <= 1024 else sorted({0, out_rows // 256, out_rows // 128 - 1})
+    for t in tiles:
+        cols = slice(t * 128, (t + 1) * 128)
+        exp = oracle.fp8_projection(oc, os_, wc[cols], ws[cols])
+        assert max_relative_error(outs["split"][:, cols], exp, 0.25 * (hidden / 5120) ** 0.5) <= 1e-2, t
+    a = oracle.bf16_to_f32(outs["split"].reshape(-1)).astype(np.float64)
     b = oracle.bf16_to_f32(outs["pair"].reshape(-1)).astype(np.float64)
     # one BF16 step of the larger magnitude, plus the cancellation floor of a split fp32 sum
     assert np.all(np.abs(a - b) <= np.maximum(np.abs(a), np.abs(b)) * 2.0 ** -7 + 1e-3), np.abs(a - b).max()
-    assert (outs["stream_k"] == outs["pair"]).mean() > 0.9
+    assert (outs["split"] == outs["pair"]).mean() > 0.9

@@ -250,6 +250,7 @@ def test_pair_route_small_geometry(tk, oracle, rows, monkeypatch):
     dn_codes, dn_scales, dn_div = synth.nvfp4_weights(14, 2, hidden, inter)
     a_div = float(np.float32(448.0 * 6.0 / 5.0))
     results = {}
+    monkeypatch.setenv("TK100_PERSIST", "0")  # the other arm on one-CTA tiles, not on persistent pairs
     for route, min_rows in (("pair", "1"), ("single", "1000000")):
         monkeypatch.setenv("TK100_PAIR_MIN_ROWS", min_rows)
         monkeypatch.setenv("TK100_PAIR", "2")  # gate_up on pairs too (off by default)
@@ -260,6 +261,8 @@ def test_pair_route_small_geometry(tk, oracle, rows, monkeypatch):
                                      float(gu_div), mid, activation_codes=codes,
                                      activation_scales=scales, input_global_divisor=a_div)
         torch.cuda.synchronize()
+        kernel = "nvfp4_pair_kernel" if route == "pair" else "nvfp4_gemm_kernel"
+        assert ctx.last_kernel.startswith(kernel), ctx.last_kernel
         got_mid = _u16(mid)[:rows].copy()
         assert_inactive_untouched(mid, rows)
         m_div = float(np.float32(448.0 * 6.0 / 8.0))
@@ -290,8 +293,8 @@ def test_pair_route_small_geometry(tk, oracle, rows, monkeypatch):
 @pytest.mark.parametrize("rows", [1, 7, 32, 33, 130, 256])
 def test_gate_up_cluster_pairs_and_fused_kernel_agree(tk, oracle, rows, monkeypatch):
     """gate_up + SwiGLU on its two routes, ragged token counts included: clusters of a gate CTA
-    and an up CTA that swap accumulator halves over distributed shared memory (the default), and
-    one CTA that holds both tiles (TK100_SWIGLU_PAIRS=0).  Both against the W4A4 oracle; the
+    and an up CTA that swap accumulator halves over distributed shared memory (the default up to
+    32 tokens), and one CTA that holds both tiles (TK100_SWIGLU_PAIRS=0).  Both against the W4A4 oracle; the
     two agree to the bit (same products, same fp32 accumulation order per output)."""
     from tuiskollm_b200 import synth
 
@@ -528,9 +531,8 @@ def test_reduction_routes_of_the_mlp_agree_bit_for_bit(tk, oracle, rows, monkeyp
 
 @pytest.mark.parametrize("rows", [256, 300, 700, 1030])
 def test_persistent_pair_route_matches_plain_route_and_oracle(tk, oracle, rows, monkeypatch):
-    """Prefill token counts run on persistent CTA pairs (256-row x 256-token pair tiles, each pair
-    walking several tiles, gate/up halves exchanged through the partner's shared memory).  On a
-    small geometry with ragged token counts: every output within tolerance of the W4A4 oracle,
+    """Prefill token counts run on persistent CTA pairs (256-row pair tiles of up to 256 tokens, each
+    pair walking several tiles, gate and up rows of an output in one CTA).  On a small geometry with ragged token counts: every output within tolerance of the W4A4 oracle,
     inactive rows untouched, and the same bits as the one-CTA kernels (TK100_PERSIST=0) -- both
     add the K blocks in order into one fp32 accumulator."""
     from tuiskollm_b200 import synth
@@ -565,8 +567,9 @@ def test_persistent_pair_route_matches_plain_route_and_oracle(tk, oracle, rows, 
                                          input_global_divisor=m_div)
         torch.cuda.synchronize()
         assert c.device_status() == 0, route
-        assert r_gu.startswith("nvfp4_persist_kernel") == (route == "persistent"), (route, r_gu)
-        assert r_dn.startswith("nvfp4_persist_kernel") == (route == "persistent"), (route, r_dn)
+        kernel = "pair_gemm_kernel" if route == "persistent" else "nvfp4_gemm_kernel"
+        assert r_gu.startswith(kernel), (route, r_gu)
+        assert r_dn.startswith(kernel), (route, r_dn)
         for pl in (mid, out, part):
             assert_inactive_untouched(pl, rows)
         got[route] = (_u16(mid)[:rows].copy(), _u16(out)[:rows].copy(), host(part)[:rows].copy())
@@ -585,8 +588,8 @@ def test_persistent_pair_route_matches_plain_route_and_oracle(tk, oracle, rows, 
 
 
 def test_full_size_prefill_down_sampled_tiles(tk, ctx, oracle):
-    """Configuration 4's down projection at full size (M = 2048, 5120 x 17408: unsplit 128-token
-    tiles over 68 k-blocks): first, last and two inner weight tiles x first and last token tile
+    """Configuration 4's down projection at full size (M = 2048, 5120 x 17408: unsplit pair tiles
+    over 68 k-blocks): first, last and two inner weight tiles x first and last token tile
     against the W4A4 oracle, the activation quantiser bit for bit on those token tiles."""
     from tuiskollm_b200 import synth
 
@@ -652,6 +655,7 @@ def test_wide_tile_route_matches_plain_route_bit_for_bit(tk, rows, monkeypatch):
     dn_codes, dn_scales, dn_div = synth.nvfp4_weights(19, 2, hidden, inter)
     a_div, m_div = float(np.float32(448.0 * 6.0 / 5.0)), float(np.float32(448.0 * 6.0 / 8.0))
     got = {}
+    monkeypatch.setenv("TK100_PERSIST", "0")  # the plain arm on 128-token tiles, not on pairs
     for route, env in (("wide", "2"), ("plain", "0")):
         monkeypatch.setenv("TK100_NVFP4_WIDE", env)
         monkeypatch.setenv("TK100_NVFP4_WIDE_MIN_ROWS", "256")
@@ -672,8 +676,9 @@ def test_wide_tile_route_matches_plain_route_bit_for_bit(tk, rows, monkeypatch):
         r_dn = c.last_kernel
         torch.cuda.synchronize()
         assert c.device_status() == 0, route
-        assert r_gu.startswith("nvfp4_gemm_kernel<256") == (route == "wide"), (route, r_gu)
-        assert r_dn.startswith("nvfp4_gemm_kernel<256") == (route == "wide"), (route, r_dn)
+        kernel = "nvfp4_gemm_kernel<256" if route == "wide" else "nvfp4_gemm_kernel<128"
+        assert r_gu.startswith(kernel), (route, r_gu)
+        assert r_dn.startswith(kernel), (route, r_dn)
         for pl in (mid, out):
             assert_inactive_untouched(pl, rows)
         got[route] = (_u16(mid)[:rows].copy(), _u16(out)[:rows].copy())

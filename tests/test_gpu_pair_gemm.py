@@ -52,7 +52,7 @@ def test_fp8_projection(tk, oracle, monkeypatch, out_rows, k, rows, tok, splits)
     op = tk.ops.Fp8ProjectionOp(c)
     op.launch(None, rows, out_rows, k, dev(xb.view(np.int16)), codes, scales, w, s, out)
     torch.cuda.synchronize()
-    assert c.last_kernel.startswith("fp8_pair_persist_kernel"), c.last_kernel
+    assert c.last_kernel.startswith("pair_gemm_kernel"), c.last_kernel
     assert f"splits={splits if 1 <= splits <= 4 else 1}" in c.last_kernel, c.last_kernel
     assert c.device_status() == 0
     oc, os_ = oracle.quantize_e4m3(xb)
@@ -70,23 +70,23 @@ def test_fp8_projection(tk, oracle, monkeypatch, out_rows, k, rows, tok, splits)
 
 @pytest.mark.parametrize("out_rows,k,rows,kernel", [
     (1040, 3072, 48, "fp8_projection_kernel<64"),    # three splits planned: one-CTA tiles up to 48 tokens
-    (1040, 3072, 49, "fp8_pair_persist_kernel"),
-    (1040, 2048, 48, "fp8_pair_persist_kernel"),     # two splits planned
+    (1040, 3072, 49, "pair_gemm_kernel"),
+    (1040, 2048, 48, "pair_gemm_kernel"),     # two splits planned
     (1040, 4096, 64, "fp8_projection_kernel<64"),    # four splits planned: up to 64
-    (1040, 4096, 65, "fp8_pair_persist_kernel"),
-    (768, 4096, 64, "fp8_pair_persist_kernel"),
+    (1040, 4096, 65, "pair_gemm_kernel"),
+    (768, 4096, 64, "pair_gemm_kernel"),
     (4096, 6144, 64, "fp8_projection_kernel<64"),    # three splits, but a long K
     (4096, 3072, 33, "fp8_projection_kernel<64"),    # most rows of the rule
-    (4112, 3072, 33, "fp8_pair_persist_kernel"),
+    (4112, 3072, 33, "pair_gemm_kernel"),
     (5120, 256, 641, "fp8_pair_kernel"),             # 60 tiles in one wave, planned at 224 tokens
-    (5120, 256, 576, "fp8_pair_persist_kernel"),     # ... at 192
-    (5136, 256, 700, "fp8_pair_persist_kernel"),     # weight rows end inside a tile
+    (5120, 256, 576, "pair_gemm_kernel"),     # ... at 192
+    (5136, 256, 700, "pair_gemm_kernel"),     # weight rows end inside a tile
     (8192, 2176, 256, "fp8_pair_kernel"),            # two splits planned
     (12288, 256, 256, "fp8_pair_kernel"),            # one wave where the plan takes two
     (8192, 512, 630, "fp8_pair_kernel"),             # 96 tiles in two waves of 160 tokens: K up to 512
-    (8192, 640, 630, "fp8_pair_persist_kernel"),
-    (2560, 512, 2048, "fp8_pair_persist_kernel"),    # a second wave mostly empty
-    (8192, 256, 1281, "fp8_pair_persist_kernel"),    # more tiles than two waves hold
+    (8192, 640, 630, "pair_gemm_kernel"),
+    (2560, 512, 2048, "pair_gemm_kernel"),    # a second wave mostly empty
+    (8192, 256, 1281, "pair_gemm_kernel"),    # more tiles than two waves hold
 ])
 def test_fp8_projection_route_rules(tk, oracle, out_rows, k, rows, kernel):
     """Both sides of each line between the pair kernel and the kernels it leaves a launch to."""
@@ -123,7 +123,7 @@ def test_fp8_swiglu(tk, oracle, monkeypatch, rows, tok, splits):
     out = sentinel_plane((rows + 1, inter), torch.int16)
     tk.Fp8SwiGluOp(c).launch(None, rows, dev(xb.view(np.int16)), codes, scales, dev(wc), dev(ws.view(np.int16)), out)
     torch.cuda.synchronize()
-    assert c.last_kernel.startswith("fp8_swiglu_kernel_pairs"), c.last_kernel
+    assert c.last_kernel.startswith("pair_gemm_kernel"), c.last_kernel
     assert c.device_status() == 0
     oc, os_ = oracle.quantize_e4m3(xb)
     dots = oracle.fp8_projection(oc, os_, wc, ws)
@@ -163,7 +163,7 @@ def test_nvfp4_mlp(tk, oracle, monkeypatch, hidden, inter, rows, tok, splits):
                                         activation_codes=a_codes, activation_scales=a_scales,
                                         input_global_divisor=a_div, output_global_divisor=m_div,
                                         output_codes=m_codes, output_scales=m_scales)
-    assert c.last_kernel.startswith("nvfp4_persist_kernel") and "splits=1" in c.last_kernel, c.last_kernel
+    assert c.last_kernel.startswith("pair_gemm_kernel") and "splits=1" in c.last_kernel, c.last_kernel
     down = tk.Nvfp4DownOp(c)
     kw = dict(activation_codes=m_codes, activation_scales=m_scales, input_global_divisor=m_div)
     down.launch(None, rows, None, dev(dn), dev(dns), float(dnd), out, **kw)
@@ -194,12 +194,12 @@ def test_nvfp4_mlp(tk, oracle, monkeypatch, hidden, inter, rows, tok, splits):
 @pytest.mark.parametrize("hidden,inter,rows,kernel", [
     (5120, 6144, 33, "nvfp4_gemm_kernel"),      # three splits planned
     (5120, 6144, 64, "nvfp4_gemm_kernel"),
-    (5120, 6144, 65, "nvfp4_persist_kernel"),
-    (5120, 4352, 33, "nvfp4_persist_kernel"),   # two
+    (5120, 6144, 65, "pair_gemm_kernel"),
+    (5120, 4352, 33, "pair_gemm_kernel"),   # two
     (1024, 2176, 80, "nvfp4_gemm_kernel"),      # few weight rows
-    (1024, 2176, 81, "nvfp4_persist_kernel"),
-    (1024, 2048, 64, "nvfp4_persist_kernel"),
-    (1280, 2176, 64, "nvfp4_persist_kernel"),
+    (1024, 2176, 81, "pair_gemm_kernel"),
+    (1024, 2048, 64, "pair_gemm_kernel"),
+    (1280, 2176, 64, "pair_gemm_kernel"),
 ])
 def test_nvfp4_down_route_rules(tk, oracle, hidden, inter, rows, kernel):
     """Both sides of each line between the pair kernel and the one-CTA kernel, in both output types."""
@@ -250,4 +250,4 @@ def test_quantised_output_planes_are_held_to_the_quantisers_alignment(tk):
     op.launch_quantize(None, rows, None, w, ws, 1.0, mid, activation_codes=codes, activation_scales=scales,
                        input_global_divisor=1.0, output_global_divisor=1.0, output_codes=m_codes, output_scales=m_scales)
     torch.cuda.synchronize()
-    assert c.last_kernel.startswith("nvfp4_persist_kernel") and c.device_status() == 0
+    assert c.last_kernel.startswith("pair_gemm_kernel") and c.device_status() == 0

@@ -898,8 +898,7 @@ Status Fp8ProjectionOp::launch(cudaStream_t stream, int rows, int out_rows, int 
         q.w_scales = weight_scales;
         q.out = output;
         ctx_.count_launch();
-        ctx_.note_route(tune.fp8_stream_k != 0 ? "fp8_pair_stream_k_kernel" : "fp8_pair_persist_kernel", plan.tok_tile,
-                        plan.workers, plan.splits, 1);
+        ctx_.note_route("pair_gemm_kernel", plan.tok_tile, plan.workers, plan.splits, 1);
         return ctx_.check(launch_pair_gemm(stream, false, false, plan.workers, map_w, map_a, map_w, map_a, q),
                           "launching the persistent FP8 pair projection");
       }
@@ -1108,7 +1107,7 @@ Status Fp8SwiGluOp::launch(cudaStream_t stream, int rows, const uint16_t* input,
     q.w_scales = weight_scales;
     q.out = output;
     ctx_.count_launch();
-    ctx_.note_route("fp8_swiglu_kernel_pairs", plan.tok_tile, plan.workers, plan.splits, 1);
+    ctx_.note_route("pair_gemm_kernel", plan.tok_tile, plan.workers, plan.splits, 1);
     return ctx_.check(launch_pair_gemm(stream, false, true, plan.workers, map_w, map_a, map_w, map_a, q),
                       "launching the persistent FP8 SwiGLU");
   }
@@ -1297,7 +1296,7 @@ Status Nvfp4MlpOp::launch(cudaStream_t stream, bool gate_up, int rows, int out_r
         q.q_divisor = next->divisor;
       }
       ctx_.count_launch();
-      ctx_.note_route("nvfp4_persist_kernel", plan.tok_tile, plan.workers, plan.splits, 1);
+      ctx_.note_route("pair_gemm_kernel", plan.tok_tile, plan.workers, plan.splits, 1);
       return ctx_.check(launch_pair_gemm(stream, true, gate_up, plan.workers, map_w, map_a, map_wsf, map_asf, q),
                         "launching the persistent NVFP4 projection");
     }
