@@ -21,10 +21,10 @@ the peers over NVLink and merges (N > 1): two kernel launches per step.
             inside the timed region, one stream synchronisation per step (graph replay, and
             `e2e.eager` with every operator call made from the host)
   roofline  the projection kernel alone against the measured HBM copy bandwidth
-  configs   (N = 1) every other benchmark configuration as its own measured row: time, kernel and
-            fraction of its roofline; the rows in full (bytes, flops, nominal peaks, end-to-end and
-            CPU figures) go to stderr, one JSON line each, so that the line stays short enough for
-            a reader that keeps only the end of a run's output
+  configs   (N = 1) every other benchmark configuration as its own measured row: operator, M, N,
+            median time and fraction of its roofline; the rows in full (percentiles, kernel, bytes,
+            flops, peaks, end-to-end and CPU figures) go to stderr, one JSON line each, so that the
+            line stays short enough for a reader that keeps only the end of a run's output
 
 `--impl reference` times the CPU restatement of the reference's qualification oracle for
 the same workload on the host cores (the reference is Rust + cuda-oxide for sm_120 and can
@@ -490,14 +490,12 @@ class Protocol:
         return out
 
 
+LINE_ROW = ["op", "M", "N", "median_us", "frac"]
+
+
 def line_row(row):
-    """What the printed line carries of a configuration row."""
-    short = {k: row[k] for k in ("config", "op", "M", "N", "K") if k in row}
-    short["us"] = {k: round(row["us"][k], 3) for k in ("median", "p10", "p90")}
-    roofline = row["roofline"]
-    short["kernel"], short["bound"] = roofline["kernel"], roofline["bound"]
-    short["frac"] = round(roofline["frac"], 4)
-    return short
+    """What the printed line carries of a configuration row (LINE_ROW)."""
+    return [row["op"], row["M"], row.get("N", 0), round(row["us"]["median"], 2), round(row["roofline"]["frac"], 3)]
 
 
 def hbm_roofline(kernel, nbytes, us, peak, peak_kind):
@@ -1796,6 +1794,7 @@ def run_native(args):
                     r["kilocycles_at_median_sm_clock"] = r["us"]["median"] * row_clocks["sm_mhz"] / 1e3
             for r in rows:
                 print(json.dumps({"config_row": r}), file=sys.stderr, flush=True)
+            line["configs_columns"] = LINE_ROW
             line["configs"] = [line_row(r) for r in rows]
             if deviation is not None:
                 line["w4a4_vs_a16"] = deviation

@@ -36,8 +36,8 @@ def test_operations_per_sample_reach_the_floor():
 
 
 def test_printed_line_stays_short():
-    """A reader that keeps the last 32 KB of a run's output still finds the whole line: with the rows
-    in full (about 800 bytes each, 70 and more of them) it did not."""
+    """A reader that keeps the last 10 KB of a run's output still finds the whole line; with the rows in
+    full (about 800 bytes each, 70 and more of them) it would not.  The gate reads those from stderr."""
     import json
     import xtask
 
@@ -51,7 +51,9 @@ def test_printed_line_stays_short():
            "cpu_baseline": {"value": 1.0 / 3, "us_full_shape": 1e9 / 3, "sample": "x" * 160},
            "kilocycles_at_median_sm_clock": 1e3 / 3}
     assert len(json.dumps(row)) > 800
-    short = [bench.line_row(row) for _ in range(90)]
-    assert len(json.dumps(short)) < 24 << 10        # the rest of the line takes about 4 KB
-    line = {"config": {"rows": 1, "vocab": 248320}, "protocol": {"us_per_step": {"median": 186.0}}, "configs": short}
-    assert xtask.perf_rows(line)[("nvfp4_gate_up_swiglu_quantize", 2048, 16384)] == 148.123   # what the gate reads
+    short = [bench.line_row(row) for _ in range(75)]
+    assert all(len(r) == len(bench.LINE_ROW) for r in short)
+    assert len(json.dumps(short)) < 5 << 10        # the rest of the line takes about 4 KB
+    rows = xtask.full_rows("a warning\n" + json.dumps({"config_row": row}) + "\n")
+    line = {"config": {"rows": 1, "vocab": 248320}, "protocol": {"us_per_step": {"median": 186.0}}, "configs": rows}
+    assert xtask.perf_rows(line)[("nvfp4_gate_up_swiglu_quantize", 2048, 16384)] == row["us"]["median"]

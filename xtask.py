@@ -185,6 +185,11 @@ def perf_rows(line: dict):
     return rows
 
 
+def full_rows(stderr: str):
+    """The configuration rows in full, which bench.py prints to stderr, one JSON line each."""
+    return [json.loads(text)["config_row"] for text in stderr.splitlines() if text.startswith('{"config_row":')]
+
+
 def perf(mode: str, extra) -> int:
     cmd = [sys.executable, os.path.join(ROOT, "bench.py"), "--gpus", "1"] + list(extra)
     if mode == "smoke":
@@ -198,6 +203,7 @@ def perf(mode: str, extra) -> int:
         print(res.stdout)
         return res.returncode
     line = json.loads(res.stdout.strip().splitlines()[-1])
+    line["configs"] = full_rows(res.stderr)
     rows = perf_rows(line)
     if mode == "smoke":
         for k, v in rows.items():
