@@ -973,7 +973,7 @@ def config_rows(torch, tk, ctx, peak_gbs, peak_kind, lm, with_cpu=True):
         proto.add(case, graph.replay, 1)
         flops = 2.0 * m * HIDDEN * (synth.QKV_ROWS + synth.GDN_ROWS + 3 * inter)
         meta[case] = {"config": 1 if m == 1 else 5 if m == 256 else "metric", "op": "layer_slice",
-                      "M": m, "kernel": "5 kernels" if m <= 32 else "6 kernels",
+                      "M": m, "kernel": "5 kernels",
                       "kind": "slice", "flops": flops, "bytes": weight_bytes, "cpu": ("slice", m)}
         graph_e2e = capture(torch, slice_e2e_, 1)
         for _ in range(3):

@@ -389,9 +389,9 @@ TK100_API tk100_status tk100_peer_sum_bf16(tk100_ctx* ctx, tk100_stream stream, 
 
 /* tk100_nvfp4_gate_up_swiglu that also leaves the NVFP4 form of its output (codes
  * [rows, intermediate/2], swizzled block scales, definition at tk100_nvfp4_quantize_activation
- * with output_global_divisor) for tk100_nvfp4_down(input == NULL).  Up to 32 rows the
- * quantisation runs in the projection's epilogue instead of a launch of its own; beyond that
- * the call launches the quantiser after the projection.  Both planes are always written.  No
+ * with output_global_divisor) for tk100_nvfp4_down(input == NULL).  The quantisation runs in the
+ * projection's epilogue, at every row count; a TK100_* switch that selects another kernel beyond 32
+ * rows launches the quantiser after the projection.  Both planes are always written.  No
  * counterpart in the reference (its down kernel reads BF16). */
 TK100_API tk100_status tk100_nvfp4_gate_up_swiglu_quantize(
     tk100_ctx* ctx, tk100_stream stream, int rows, const uint16_t* input, uint8_t* activation_codes,

@@ -232,3 +232,46 @@ def test_batch_outside_the_admitted_range_is_refused(tk, ctx):
         with pytest.raises(tk.GpuError, match="outside the admitted range"):
             prep.launch(tk.GdnPrepareOp(ctx), batch)
 
+
+@pytest.mark.parametrize("batch", [1, 8])
+def test_dependent_launches_keep_the_order_of_a_layer(tk, batch, monkeypatch):
+    """Norm -> input projection -> prepare -> recurrence -> output projection, four times over the same
+    planes and state, with programmatic launches on and off: kernels that release their dependents
+    before they wait themselves must leave the bits of a serial stream."""
+    from tuiskollm_b200 import synth
+
+    slots, steps = 8, 4
+    bf16 = lambda n, *shape, std=1.0: synth.torch_normal_bf16(71, n, shape, "cuda", std=std)
+    w_in, ws_in = synth.torch_fp8_weights(71, 1, 16384, 5120, "cuda")
+    w_out, ws_out = synth.torch_fp8_weights(71, 2, 5120, 6144, "cuda")
+    branch, norm_w, control = bf16(3, steps, batch, 5120), bf16(4, 5120, std=0.1), bf16(5, 96, 5120, std=0.02)
+    a_log, dt_bias, conv_w, head_w = bf16(6, 48), bf16(7, 48), bf16(8, 10240, 4, std=0.5), bf16(9, 128)
+    rows = torch.arange(batch, dtype=torch.int32, device="cuda").flip(0)
+    results = []
+    for pdl in ("0", "1"):  # read when a context is made; the last one leaves it on
+        monkeypatch.setenv("TK100_PDL", pdl)
+        c = tk.Context(device=0)
+        x, history = bf16(10, batch, 5120), bf16(11, slots, 10240, 3)
+        state = torch.linspace(-0.1, 0.1, slots * 48 * 128 * 128, device="cuda").view(slots, 48, 128, 128).clone()
+        empty = lambda *shape, dtype=torch.bfloat16: torch.empty(shape, dtype=dtype, device="cuda")
+        residual, normed, projected = empty(batch, 5120), empty(batch, 5120), empty(batch, 16384)
+        convolved, mixed, out = empty(batch, 10240), empty(batch, 6144), empty(steps, batch, 5120)
+        codes, scales = empty(batch, 5120, dtype=torch.uint8), empty(batch, dtype=torch.float32)
+        codes2, scales2 = empty(batch, 6144, dtype=torch.uint8), empty(batch, dtype=torch.float32)
+        decay, beta = empty(batch, 48, dtype=torch.float32), empty(batch, 48, dtype=torch.float32)
+        norm, in_op, out_op = tk.ResidualNormOp(c), tk.GdnInputProjectionOp(c, 16384), tk.GdnOutputProjectionOp(c, 6144)
+        prepare, recurrence = tk.GdnPrepareOp(c), tk.GdnRecurrenceOp(c)
+        for i in range(steps):
+            norm.launch_quantize(None, batch, x, branch[i], norm_w, residual, normed, codes, scales)
+            in_op.launch(None, batch, None, codes, scales, w_in, ws_in, projected)
+            prepare.launch(None, batch, normed, control, a_log, dt_bias, projected, conv_w, rows, history, decay,
+                           beta, convolved)
+            recurrence.launch(None, batch, convolved, projected, decay, beta, head_w, rows, state, mixed)
+            out_op.launch(None, batch, mixed, codes2, scales2, w_out, ws_out, out[i])
+            x = residual if i == 0 else x
+        torch.cuda.synchronize()
+        assert c.device_status() == 0
+        results.append([t.clone() for t in (out, history, state, residual)])
+    for a, b in zip(*results):
+        assert torch.equal(a.view(torch.uint8), b.view(torch.uint8))
+    assert bool(torch.isfinite(results[0][0].float()).all())

@@ -230,6 +230,45 @@ def test_nvfp4_down_route_rules(tk, oracle, hidden, inter, rows, kernel):
     assert c.device_status() == 0
 
 
+def test_launches_on_two_streams_of_one_context_are_independent(tk):
+    """A split tile meets in the cluster's shared memory, not in the context's scratch: launches that
+    overlap on two streams leave the bits of launches one after the other."""
+    from tuiskollm_b200 import synth
+
+    out_rows, k, rows, count = 5120, 6144, 100, 12
+    c = tk.Context(device=0)
+    op = tk.ops.Fp8ProjectionOp(c)
+    planes = []
+    for i in range(2):
+        w, s = synth.torch_fp8_weights(66, i, out_rows, k, "cuda")
+        x = synth.torch_normal_bf16(66, 10 + i, (rows, k), "cuda")
+        codes = torch.empty((rows, k), dtype=torch.uint8, device="cuda")
+        scales = torch.empty((rows,), dtype=torch.float32, device="cuda")
+        op.quantize(None, rows, k, x, codes, scales)
+        planes.append((codes, scales, w, s, torch.empty((count, rows, out_rows), dtype=torch.int16, device="cuda")))
+
+    def launch(i, n):
+        codes, scales, w, s, out = planes[i]
+        op.launch(None, rows, out_rows, k, None, codes, scales, w, s, out[n])
+
+    want = []
+    for i in range(2):
+        launch(i, 0)
+        assert "splits=3" in c.last_kernel and c.last_kernel.startswith("pair_gemm_kernel"), c.last_kernel
+        want.append(planes[i][4][0].clone())
+        planes[i][4].zero_()
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    for n in range(count):
+        for i in range(2):
+            with torch.cuda.stream(streams[i]):
+                launch(i, n)
+    torch.cuda.synchronize()
+    for i in range(2):
+        assert bool((planes[i][4] == want[i]).all())
+    assert c.device_status() == 0
+
+
 def test_quantised_output_planes_are_held_to_the_quantisers_alignment(tk):
     """More than 32 rows: what the quantiser launch refuses, the epilogue's quantisation refuses."""
     rows, hidden, inter = 40, 256, 256

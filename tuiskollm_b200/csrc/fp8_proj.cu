@@ -316,7 +316,8 @@ __global__ void __launch_bounds__(kThreads, BLOCK_TOK <= 32 ? (DEEP == 1 ? 2 : (
       // The next kernel may start: with the accumulators all but complete its CTAs find slots as these
       // epilogues end, where during the stream they would hold slots and wait (norm + 8192 rows, one
       // token: 9.4 us with the trigger behind the set-up, 9.05 here, 10.2 without one; gated-delta-net
-      // layer: 33.1, 30.6 and 31.5 us, 32.5 with it two blocks earlier).
+      // layer: 33.1, 30.6 and 31.5 us a step in a chain of steps, 32.5 with it two blocks earlier; a
+      // layer replayed alone takes 34.8).
       pdl_trigger();
       umma_commit(&ctl->tmem_full);  // accumulator complete (also releases the epilogue on error)
       TK100_STAMP(p, 4);

@@ -401,9 +401,11 @@ struct PairPlan {
 };
 
 // Token tile and K splits of a pair_gemm launch: the cheapest by a count of SM cycles.  A stage of a pair
-// tile takes the longer of its MMAs (2 N cycles for 256 x N x 128 bytes) and of its delivery from L2
-// (about 56 bytes per cycle and SM measured on B200); a launch takes at least its weights at HBM rate
-// (about 3.9 KB per cycle).  Splitting K costs an exchange and wants at least 8 stages a split.
+// tile is counted as the longer of its MMAs (2 N cycles for 256 x N x 128 bytes) and of its bytes at 56 per
+// cycle and SM, a fit within 20 % of what a stage takes (FP8 337 / 364 / 433 / 511 / 674 cycles at 64 / 128 /
+// 160 / 192 / 256 tokens, NVFP4 649 / 709 at 128 / 256, operands in L2) and no rate of the machine: up to 68
+// arrive.  A launch takes at least its weights at HBM rate (about 3.9 KB per cycle).  Splitting K costs an
+// exchange and wants at least 8 stages a split.
 // A forced split count holds where it is admitted; where it is not (gate/up never splits) the plan is
 // chosen as without it.
 PairPlan plan_pairs(const Context& ctx, int rows, int row_units, int nkb, bool nvfp4, double weight_bytes,
@@ -411,7 +413,7 @@ PairPlan plan_pairs(const Context& ctx, int rows, int row_units, int nkb, bool n
   PairPlan best;
   const Tuning& tune = ctx.tuning();
   const int least = (rows + 255) / 256;
-  // NVFP4: whole 128-token scale tiles (a 64-token block-scaled pair MMA is not taken by the hardware)
+  // NVFP4: whole scale tiles of 128 tokens, the only sizes the kernel is written for
   const int grain = nvfp4 ? 128 : 32;
   for (int n = least; n < least + 4; ++n) {
     int tok = ((rows + n - 1) / n + grain - 1) / grain * grain;

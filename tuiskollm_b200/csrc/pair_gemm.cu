@@ -3,8 +3,7 @@
 //
 // A pair tile is 256 weight rows (128 per CTA, the UMMA "A" operand) x N tokens, N chosen per launch: a
 // multiple of 32 up to 256 for FP8 (a ragged token count costs at most 31 padded tokens a tile), 128 or
-// 256 for NVFP4 (whole scale tiles; a 64-token block-scaled pair MMA ended in a misaligned-address
-// error, so no other size is used).  Each
+// 256 for NVFP4: activation scales are stored, copied and addressed in whole tiles of 128 tokens.  Each
 // CTA loads its 128 weight rows and half of the tokens; one pair per two SMs stays resident and walks
 // its share of the tiles (token tiles fastest: the pairs that run together read the same weights).
 //

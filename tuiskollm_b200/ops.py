@@ -440,7 +440,7 @@ class Nvfp4SwiGluOp(_Nvfp4Op):
                         weight_scale_divisor, output, *, activation_codes, activation_scales,
                         input_global_divisor, output_global_divisor, output_codes, output_scales):
         """The same projection, also leaving the NVFP4 codes and block scales of its output for
-        ``Nvfp4DownOp.launch(input=None, ...)`` (in the projection's epilogue up to 32 rows)."""
+        ``Nvfp4DownOp.launch(input=None, ...)`` (in the projection's epilogue)."""
         c = self.ctx
         c._native.tk100_nvfp4_gate_up_swiglu_quantize(c, stream, batch, input, activation_codes,
                                                       activation_scales, input_global_divisor, weight_codes,
