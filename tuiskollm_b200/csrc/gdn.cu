@@ -87,8 +87,8 @@ __global__ void __launch_bounds__(kPrepThreads) gdn_prepare_kernel(GdnPreparePar
       w[c] = chunk < chunks ? ldg16(p.control_weights + static_cast<size_t>(row) * p.hidden + chunk * 8)
                             : make_uint4(0, 0, 0, 0);
     }
-    pdl_trigger();  // early: the output projection's weights can be on their way behind this chain
     pdl_wait();
+    pdl_trigger();
     // Two chunk columns at a time: all tokens' loads of a column pair are requested before the
     // first FMA on them, so a batch of 8 costs one round trip to L2 per pair, not eight.
     float acc[kGdnMaxBatch];
@@ -139,8 +139,8 @@ __global__ void __launch_bounds__(kPrepThreads) gdn_prepare_kernel(GdnPreparePar
   // Convolution: 8 adjacent channels of one token per thread.
   const int groups = p.qkv_rows / 8;
   const int index = (static_cast<int>(blockIdx.x) - control_ctas) * kPrepThreads + tid;
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
   if (index >= p.batch * groups) return;
   const int token = index / groups;
   const int channel = (index - token * groups) * 8;
@@ -237,8 +237,8 @@ __global__ void __cluster_dims__(SPLIT, 1, 1) __launch_bounds__(kRecThreads)
   // First half of the "every CTA of the cluster is running" barrier a remote shared-memory store
   // needs; the second half sits in front of the push, behind the state math.
   cluster_arrive();
-  pdl_trigger();
   pdl_wait();
+  pdl_trigger();
 
   const size_t state_row = p.state_rows[token];
   float* state = p.state + ((state_row * kValueHeads + value_head) * kHeadDim + row0) * kHeadDim;
