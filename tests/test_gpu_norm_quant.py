@@ -237,3 +237,23 @@ def test_quotients_of_every_scale_round_as_the_division(tk, oracle, cols, rows):
     oc, os_ = oracle.quantize_e4m3(clean)
     oc[:, 7] = 0x7F
     assert np.array_equal(host(scales), os_) and np.array_equal(host(codes), oc)
+
+
+@pytest.mark.parametrize("exponent", [-66, -60, 0, 96])
+def test_every_pair_of_significands_rounds_as_the_division(tk, oracle, exponent):
+    """E4M3 scales and codes come from products with a two-part reciprocal: all 128 significands a row maximum
+    can have (exponents on both sides of the range the products are used in) against all 128 of a value,
+    down to 2^-20 of the maximum."""
+    mant = 1.0 + np.arange(128) / 128.0
+    values = np.concatenate([mant * 2.0 ** -e for e in range(20)])
+    x = np.minimum(values[None, :], mant[:, None])
+    x[:, 1::2] *= -1.0
+    x[:, 0] = mant
+    bits = oracle.f32_to_bf16((x * 2.0 ** exponent).astype(np.float32))
+    codes, scales = (torch.zeros(bits.shape, dtype=torch.uint8, device="cuda"),
+                     torch.zeros((128,), dtype=torch.float32, device="cuda"))
+    c = tk.Context(device=0)
+    tk.ops.Fp8ProjectionOp(c).quantize(None, 128, bits.shape[1], dev(bits.view(np.int16)), codes, scales)
+    oc, os_ = oracle.quantize_e4m3(bits)
+    assert np.array_equal(host(scales), os_) and np.array_equal(host(codes), oc)
+    assert c.device_status() == 0

@@ -63,12 +63,14 @@ __device__ __forceinline__ uint32_t f32x2_to_bf16x2(F32x2 v) {
   return pack_bf16x2(f.x, f.y);
 }
 
-// max(|.|) of two packed BF16 pairs, NaNs ignored as by fmaxf (`acc` starts at 0).
+// max(|.|) of two packed BF16 pairs, NaNs ignored as by fmaxf (`acc` starts at 0).  The signs of the result
+// mean nothing; bf16x2_fold gives the bits of the larger magnitude.
 __device__ __forceinline__ uint32_t bf16x2_absmax(uint32_t acc, uint32_t w) {
   uint32_t r;
-  asm("max.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(acc), "r"(w & 0x7fff7fffu));
+  asm("max.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(acc), "r"(w));
   return r;
 }
+__device__ __forceinline__ uint32_t bf16x2_fold(uint32_t m) { return max(m & 0x7fffu, (m >> 16) & 0x7fffu); }
 
 // Two f32 -> two E4M3FN codes, round-to-nearest-even, saturating to +-448
 // (cvt.rn.satfinite.e4m3x2.f32); `lo` lands in the low byte.
@@ -107,58 +109,94 @@ __device__ __forceinline__ float silu_fp8_path(float v) {
   return __fdividef(v, 1.0f + ex);
 }
 
-// x / s by a residual step on the product with the correctly rounded reciprocal (P. Markstein, "Computation
-// of elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34 (1990)).  Operands
-// come negated: `negative` = -x, ninv = -__frcp_rn(s); that keeps the sign of a zero quotient, which the
-// residual of the plain form (0 - 0) would lose.  One step lands within one unit in the last place and
-// exactly on every quotient that fp32 holds; a second one rounds like the division.
-__device__ __forceinline__ F32x2 quotient_step(F32x2 q, F32x2 negative, F32x2 s, F32x2 ninv) {
-  return fma2(fma2(q, s, negative), ninv, q);
+// 1 / s as the sum hi + lo, hi slightly below it and lo > 0: rcp.approx is within one unit in the last
+// place, so three units less is below, and lo = (1 - hi s) hi restores what is missing to 2^-42.  A product
+// x hi + x lo, the second part rounded first, is then within 2^-42 of x / s before its one rounding, and keeps
+// the sign of a zero x (hence lo > 0).  Two operations per quotient, where a division takes about eight and
+// residual steps on a rounded reciprocal three to five; s must leave hi and lo normal (2^-100 .. 2^100).
+struct Reciprocal {
+  float hi, lo;
+};
+__device__ __forceinline__ Reciprocal reciprocal_parts(float s) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(s));
+  Reciprocal p;
+  p.hi = __uint_as_float(__float_as_uint(r) - 3u);
+  p.lo = __fmul_rn(__fmaf_rn(-p.hi, s, 1.0f), p.hi);
+  return p;
 }
+__device__ __forceinline__ F32x2 quotient(F32x2 x, F32x2 hi, F32x2 lo) { return fma2(x, hi, mul2(x, lo)); }
 
-// E4M3 codes of a packed BF16 pair divided by `scale` (e4m3_rn_satfinite of the IEEE quotient).  Two
-// residual steps; they need a scale whose residuals stay in the normal range (e4m3_scale_is_ordinary).
-__device__ __forceinline__ bool e4m3_scale_is_ordinary(float scale) { return scale >= 0x1p-80f && scale <= 0x1p120f; }
-__device__ __forceinline__ uint32_t e4m3_pair_ordinary(uint32_t w, F32x2 scale, F32x2 ninv) {
-  const F32x2 n = bf16x2_to_f32x2(w ^ 0x80008000u);
-  const float2 q = f32x2_parts(quotient_step(quotient_step(mul2(n, ninv), n, scale, ninv), n, scale, ninv));
+// E4M3 row quantiser: scale = amax / 448 (1 for a zero row), code = e4m3_rne_sat(x / scale), both quotients
+// rounded as the division rounds them.  amax has 128 significands (it is a BF16 value): for each of them and
+// each BF16 x <= amax the two-part products round like the division (all 128 x 128 pairs of significands
+// checked), so an ordinary amax takes them; beyond, where exponents run out, the division runs.
+__device__ __forceinline__ bool e4m3_amax_is_ordinary(float amax) { return amax >= 0x1p-60f && amax <= 0x1p97f; }
+__device__ __forceinline__ float e4m3_scale_ordinary(float amax) {
+  // 1 / 448 in two parts, the first three units in the last place below it
+  return __fmaf_rn(amax, 0x1.249244p-9f, __fmul_rn(amax, 0x1.49248cp-31f));
+}
+__device__ __forceinline__ float e4m3_scale(float amax) { return amax == 0.0f ? 1.0f : __fdiv_rn(amax, 448.0f); }
+__device__ __forceinline__ uint32_t e4m3_pair_ordinary(F32x2 x, F32x2 hi, F32x2 lo) {
+  const float2 q = f32x2_parts(quotient(x, hi, lo));
   return f32x2_to_e4m3x2(q.x, q.y);
 }
-__device__ __forceinline__ uint32_t e4m3_pair(uint32_t w, float scale) {
-  return f32x2_to_e4m3x2(__fdiv_rn(bf16x2_lo(w), scale), __fdiv_rn(bf16x2_hi(w), scale));
+__device__ __forceinline__ uint32_t e4m3_pair(F32x2 x, float scale) {
+  const float2 v = f32x2_parts(x);
+  return f32x2_to_e4m3x2(__fdiv_rn(v.x, scale), __fdiv_rn(v.y, scale));
+}
+
+// Four pairs of f32 -> eight E2M1 codes (cvt.rn.satfinite.e2m1x2.f32), first value in the lowest nibble.
+__device__ __forceinline__ uint32_t f32x8_to_e2m1x8(F32x2 a, F32x2 b, F32x2 c, F32x2 d) {
+  const float2 p = f32x2_parts(a), q = f32x2_parts(b), r = f32x2_parts(c), s = f32x2_parts(d);
+  uint32_t w;
+  asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\t"
+      "cvt.rn.satfinite.e2m1x2.f32 b0, %2, %1;\n\t"
+      "cvt.rn.satfinite.e2m1x2.f32 b1, %4, %3;\n\t"
+      "cvt.rn.satfinite.e2m1x2.f32 b2, %6, %5;\n\t"
+      "cvt.rn.satfinite.e2m1x2.f32 b3, %8, %7;\n\t"
+      "mov.b32 %0, {b0, b1, b2, b3};\n\t}"
+      : "=r"(w)
+      : "f"(p.x), "f"(p.y), "f"(q.x), "f"(q.y), "f"(r.x), "f"(r.y), "f"(s.x), "f"(s.y));
+  return w;
+}
+
+// Scale code of an NVFP4 block, e4m3_rne_sat((amax * divisor) / 6).  Six times an E4M3 rounding boundary has at
+// most 7 significant bits, so a quotient is on a boundary exactly or more than 1.3 half units in the last
+// place away from it: the two-part product decides every code as the division does.
+__device__ __forceinline__ uint32_t nvfp4_scale_code(float amax, float divisor) {
+  constexpr float hi = 0x1.55555p-3f, lo = 0x1.55555p-25f;  // 1 / 6 in two parts, the first below it
+  const float t = __fmul_rn(amax, divisor);
+  return f32x2_to_e4m3x2(__fmaf_rn(t, hi, __fmul_rn(t, lo)), 0.0f) & 0xffu;
 }
 
 // NVFP4 codes of N packed BF16 pairs of one block: code = e2m1_rne_sat((x * divisor) / s), signed zeros
 // when s == 0; two codes a byte, low nibble first.  s is a decoded E4M3 scale (4 significant bits) and an
 // E2M1 rounding boundary has 3, so a quotient is on a boundary exactly or more than 1.007 half units in
-// the last place away from it: one residual step decides every code as the division does.  An infinite
-// product keeps the division (its residual is NaN).
+// the last place away from it: the two-part product decides every code as the division does.
 template <int N>
-__device__ __forceinline__ void nvfp4_codes(const uint32_t (&w)[N], float block_max, float divisor, float s,
-                                            uint32_t (&packed)[N / 4]) {
-#pragma unroll
-  for (int j = 0; j < N / 4; ++j) packed[j] = 0u;
+__device__ __forceinline__ void nvfp4_codes(const F32x2 (&x)[N], float divisor, float s, uint32_t (&packed)[N / 4]) {
   if (s == 0.0f) {
 #pragma unroll
-    for (int j = 0; j < N; ++j) {
-      const uint32_t byte = ((w[j] & 0x8000u) ? 0x08u : 0u) | ((w[j] & 0x80000000u) ? 0x80u : 0u);
-      packed[j >> 2] |= byte << (8 * (j & 3));
-    }
-  } else if (__fmul_rn(block_max, divisor) <= 3.0e38f) {
-    const F32x2 ndiv = f32x2_splat(-divisor), ninv = f32x2_splat(-__frcp_rn(s)), s2 = f32x2_splat(s);
+    for (int j = 0; j < N / 4; ++j) {
+      packed[j] = 0u;
 #pragma unroll
-    for (int j = 0; j < N; ++j) {
-      const F32x2 n = mul2(bf16x2_to_f32x2(w[j]), ndiv);
-      const float2 q = f32x2_parts(quotient_step(mul2(n, ninv), n, s2, ninv));
-      packed[j >> 2] |= (f32x2_to_e2m1x2(q.x, q.y) & 0xffu) << (8 * (j & 3));
+      for (int i = 0; i < 4; ++i) {
+        const float2 v = f32x2_parts(x[4 * j + i]);
+        const uint32_t byte = ((__float_as_uint(v.x) >> 28) & 0x08u) | ((__float_as_uint(v.y) >> 24) & 0x80u);
+        packed[j] |= byte << (8 * i);
+      }
     }
-  } else {
+    return;
+  }
+  const Reciprocal r = reciprocal_parts(s);
+  const F32x2 div = f32x2_splat(divisor), hi = f32x2_splat(r.hi), lo = f32x2_splat(r.lo);
 #pragma unroll
-    for (int j = 0; j < N; ++j) {
-      const uint32_t byte = f32x2_to_e2m1x2(__fdiv_rn(__fmul_rn(bf16x2_lo(w[j]), divisor), s),
-                                            __fdiv_rn(__fmul_rn(bf16x2_hi(w[j]), divisor), s));
-      packed[j >> 2] |= (byte & 0xffu) << (8 * (j & 3));
-    }
+  for (int j = 0; j < N / 4; ++j) {
+    F32x2 q[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) q[i] = quotient(mul2(x[4 * j + i], div), hi, lo);
+    packed[j] = f32x8_to_e2m1x8(q[0], q[1], q[2], q[3]);
   }
 }
 
@@ -167,13 +205,16 @@ __device__ __forceinline__ void nvfp4_codes(const uint32_t (&w)[N], float block_
 // signed zeros when the scale underflows to 0.  Codes low nibble first.
 __device__ __forceinline__ uint2 nvfp4_quantize_block(const uint32_t (&w)[8], float divisor, uint32_t* scale_code) {
   uint32_t m = 0u;
+  F32x2 x[8];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) m = bf16x2_absmax(m, w[j]);
-  const float amax = fmaxf(bf16x2_lo(m), bf16x2_hi(m));
-  const uint32_t sc = f32x2_to_e4m3x2(__fdiv_rn(__fmul_rn(amax, divisor), 6.0f), 0.0f) & 0xffu;
+  for (int j = 0; j < 8; ++j) {
+    m = bf16x2_absmax(m, w[j]);
+    x[j] = bf16x2_to_f32x2(w[j]);
+  }
+  const uint32_t sc = nvfp4_scale_code(__uint_as_float(bf16x2_fold(m) << 16), divisor);
   *scale_code = sc;
   uint32_t packed[2];
-  nvfp4_codes(w, amax, divisor, e4m3_to_f32(sc), packed);
+  nvfp4_codes(x, divisor, e4m3_to_f32(sc), packed);
   return make_uint2(packed[0], packed[1]);
 }
 
@@ -187,22 +228,6 @@ __device__ __forceinline__ float warp_max(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
   return v;
-}
-
-// Block-wide sum / max with a fixed evaluation order (bit-reproducible across
-// launches): butterfly inside each warp, then every thread folds the per-warp
-// values in warp order.  `scratch` holds one float per warp.
-template <bool IS_MAX>
-__device__ __forceinline__ float block_reduce(float v, float* scratch) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int warps = (blockDim.x + 31) >> 5;
-  v = IS_MAX ? warp_max(v) : warp_sum(v);
-  __syncthreads();  // scratch may still be read from a previous reduction
-  if (lane == 0) scratch[warp] = v;
-  __syncthreads();
-  float r = scratch[0];
-  for (int i = 1; i < warps; ++i) r = IS_MAX ? fmaxf(r, scratch[i]) : r + scratch[i];
-  return r;
 }
 
 }  // namespace tk100

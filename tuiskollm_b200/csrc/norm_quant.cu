@@ -7,11 +7,13 @@
 // (tuisko-kernels-sm120/src/residual_norm.rs:155-226 followed by
 // tuisko-kernels-sm120/src/device/fp8_projection.rs:54-126).
 //
-// Reading and writing a row's 48 KB bounds it from a few hundred rows up (2048 rows with both quantised
-// forms: 98 MB, 15.3 us at the copy rate); below that its chain of two block reductions does.  With an
-// IEEE divide per value and code and unpacked fp32 rows, instruction issue came first: fp32 pairs, BF16
-// rows kept packed and quotients from one reciprocal per row or block took 2048 rows from 31.7 to
-// 23.9 us, 512 from 11.3 to 8.7, one row from 3.8 to 3.0.
+// Instruction issue bounds it beyond one wave of rows (2048 rows with both quantised forms: 12.7 M warp
+// instructions, two thirds of the issue slots, 21.3 us where the 98 MB take 15.3 at the copy rate); below that
+// its chain of load, two block reductions and store does.  So every quotient is two operations on fp32 pairs
+// (reciprocal_parts), maxima are packed BF16 and reduced as integers, a reduction has one barrier, and a row's
+// values stay widened.  With residual steps on a rounded reciprocal, IEEE divides per block and row and rows
+// unpacked at each use: 16.0 M instructions; 2048 rows 24.2 us, 512 7.0 (now 5.6), 300 6.5 (5.2), 33 4.1 (2.7),
+// one 3.0 (2.65).
 //
 // Numeric contract (bit-exact parts marked *):
 //   res  = bf16_rn(f32(x) + f32(branch))                                  *
@@ -22,6 +24,7 @@
 // The starred results are bit-exact functions of their inputs; `codes`/`scale`
 // are exact with respect to the normalised row this same kernel wrote.
 #include <cstdlib>
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -44,30 +47,67 @@ struct Nvfp4Out {
   float divisor;    // input global divisor
 };
 
+// Sum and max over the CTA, one barrier each.  The sum has a fixed order: a butterfly inside each warp, then
+// every thread adds the warps' values in warp order (the zeros behind the last do not change it).  The max is
+// over magnitudes as integers (bf16x2_fold).
+__device__ __forceinline__ float row_sum(float v, float* scratch) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int warps = (blockDim.x + 31) >> 5;
+  v = warp_sum(v);
+  if (lane == 0) scratch[warp] = v;
+  if (threadIdx.x >= warps && threadIdx.x < 32) scratch[threadIdx.x] = 0.0f;
+  __syncthreads();
+  float4 f = *reinterpret_cast<const float4*>(scratch);
+  float r = __fadd_rn(__fadd_rn(__fadd_rn(f.x, f.y), f.z), f.w);
+  for (int i = 4; i < warps; i += 4) {
+    f = *reinterpret_cast<const float4*>(scratch + i);
+    r = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(r, f.x), f.y), f.z), f.w);
+  }
+  return r;
+}
+__device__ __forceinline__ uint32_t row_max(uint32_t v, uint32_t* scratch) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int warps = (blockDim.x + 31) >> 5;
+  v = __reduce_max_sync(0xffffffffu, v);
+  if (lane == 0) scratch[warp] = v;
+  __syncthreads();
+  return __reduce_max_sync(0xffffffffu, lane < warps ? scratch[lane] : 0u);
+}
+
+// A pair of BF16 values that a thread keeps: in fp32, or packed where the registers do not allow that.
+__device__ __forceinline__ void keep_pair(F32x2& v, uint32_t w) { v = bf16x2_to_f32x2(w); }
+__device__ __forceinline__ void keep_pair(uint32_t& v, uint32_t w) { v = w; }
+__device__ __forceinline__ F32x2 pair_f32(F32x2 v) { return v; }
+__device__ __forceinline__ F32x2 pair_f32(uint32_t v) { return bf16x2_to_f32x2(v); }
+
 template <bool HAS_BRANCH, bool DO_NORM, bool DO_QUANT, int CHUNKS>
-__global__ void __launch_bounds__(1024)
+__global__ void __launch_bounds__(CHUNKS == 3 ? 704 : 1024)  // norm_geometry: three chunks on at most 704
     resnorm_quant_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ branch,
                          const uint16_t* __restrict__ weight, uint16_t* __restrict__ residual_out,
                          uint16_t* __restrict__ normalized_out, uint8_t* __restrict__ codes,
                          float* __restrict__ scales, int hidden, float eps, uint32_t* status,
                          const Nvfp4Out nv) {
-  __shared__ float scratch[32];
+  __shared__ __align__(16) float sums[32];
+  __shared__ uint32_t maxima[32];
   pdl_trigger();
   pdl_wait();  // x / branch may be the predecessor's output
   const int row = blockIdx.x;
   const int chunks_per_row = hidden >> 3;
   const size_t row_off = static_cast<size_t>(row) * hidden;
 
-  uint32_t v[CHUNKS][4];  // the row as packed BF16 pairs: rounded residual, later the normalised row
+  using Pair = std::conditional_t<CHUNKS <= 2, F32x2, uint32_t>;
+  Pair v[CHUNKS][4];  // the row: rounded residual, later the normalised row
   // The norm weight of this thread's columns is requested together with the row (one memory
   // latency less on the chain load -> reduce -> scale -> reduce -> store); with three or four
   // chunks per thread the registers do not allow it and the weight is loaded where it is used.
   constexpr bool EARLY_WEIGHT = DO_NORM && CHUNKS <= 2;
   Chunk wreg[EARLY_WEIGHT ? CHUNKS : 1];
   F32x2 sum = f32x2_splat(0.0f);
+  uint32_t m[CHUNKS];  // largest magnitudes of the row to quantise
 #pragma unroll
   for (int i = 0; i < CHUNKS; ++i) {
     const int c = threadIdx.x + i * blockDim.x;
+    m[i] = 0u;
     if (c < chunks_per_row) {
       if constexpr (EARLY_WEIGHT) wreg[i] = *reinterpret_cast<const Chunk*>(weight + c * 8);
       Chunk a = *reinterpret_cast<const Chunk*>(x + row_off + c * 8);
@@ -80,23 +120,24 @@ __global__ void __launch_bounds__(1024)
         a = r;  // the norm consumes the rounded residual
       }
 #pragma unroll
-      for (int j = 0; j < 4; ++j) v[i][j] = a.w[j];
-      if (DO_NORM) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const F32x2 f = bf16x2_to_f32x2(v[i][j]);
+      for (int j = 0; j < 4; ++j) {
+        keep_pair(v[i][j], a.w[j]);
+        if (DO_NORM) {
+          const F32x2 f = pair_f32(v[i][j]);
           sum = fma2(f, f, sum);
+        } else {
+          m[i] = bf16x2_absmax(m[i], a.w[j]);
         }
       }
     } else {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) v[i][j] = 0u;
+      for (int j = 0; j < 4; ++j) keep_pair(v[i][j], 0u);
     }
   }
 
   if (DO_NORM) {
     const float2 halves = f32x2_parts(sum);
-    const float total = block_reduce<false>(__fadd_rn(halves.x, halves.y), scratch);
+    const float total = row_sum(__fadd_rn(halves.x, halves.y), sums);
     const float mean = __fdiv_rn(total, static_cast<float>(hidden));
     const F32x2 inv_rms = f32x2_splat(__frsqrt_rn(__fadd_rn(mean, eps)));
     const F32x2 one = f32x2_splat(1.0f);
@@ -110,9 +151,9 @@ __global__ void __launch_bounds__(1024)
         Chunk o;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          o.w[j] = f32x2_to_bf16x2(mul2(mul2(bf16x2_to_f32x2(v[i][j]), inv_rms),
-                                        add2(one, bf16x2_to_f32x2(wv.w[j]))));
-          v[i][j] = o.w[j];  // keep the rounded value for the quantiser
+          o.w[j] = f32x2_to_bf16x2(mul2(mul2(pair_f32(v[i][j]), inv_rms), add2(one, bf16x2_to_f32x2(wv.w[j]))));
+          m[i] = bf16x2_absmax(m[i], o.w[j]);
+          keep_pair(v[i][j], o.w[j]);  // keep the rounded value for the quantiser
         }
         *reinterpret_cast<Chunk*>(normalized_out + row_off + c * 8) = o;
       }
@@ -126,16 +167,12 @@ __global__ void __launch_bounds__(1024)
 #pragma unroll
     for (int i = 0; i < CHUNKS; ++i) {
       const int c = threadIdx.x + i * blockDim.x;  // chunk index; block g = c / 2
-      uint32_t m = 0u;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) m = bf16x2_absmax(m, v[i][j]);
-      float bmax = fmaxf(bf16x2_lo(m), bf16x2_hi(m));
-      bmax = fmaxf(bmax, __shfl_xor_sync(0xffffffffu, bmax, 1));
+      const uint32_t block = bf16x2_absmax(m[i], __shfl_xor_sync(0xffffffffu, m[i], 1));
       if (c < chunks_per_row) {
-        const float raw = __fdiv_rn(__fmul_rn(bmax, nv.divisor), 6.0f);
-        const uint32_t sc = f32x2_to_e4m3x2(raw, 0.0f) & 0xffu;
+        const uint32_t sc = nvfp4_scale_code(__uint_as_float(bf16x2_fold(block) << 16), nv.divisor);
+        const F32x2 f[4] = {pair_f32(v[i][0]), pair_f32(v[i][1]), pair_f32(v[i][2]), pair_f32(v[i][3])};
         uint32_t packed[1];
-        nvfp4_codes(v[i], bmax, nv.divisor, e4m3_to_f32(sc), packed);
+        nvfp4_codes(f, nv.divisor, e4m3_to_f32(sc), packed);
         *reinterpret_cast<uint32_t*>(nv.codes + static_cast<size_t>(row) * (hidden >> 1) + c * 4) = packed[0];
         if ((c & 1) == 0) {
           const int g = c >> 1;
@@ -148,16 +185,10 @@ __global__ void __launch_bounds__(1024)
   }
 
   if (DO_QUANT) {
-    uint32_t m = 0u;
+    uint32_t all = m[0];
 #pragma unroll
-    for (int i = 0; i < CHUNKS; ++i) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) m = bf16x2_absmax(m, v[i][j]);
-    }
-    const float amax = block_reduce<true>(fmaxf(bf16x2_lo(m), bf16x2_hi(m)), scratch);
-    if (!(amax <= 3.0e38f) && threadIdx.x == 0) atomicOr(status, STATUS_NONFINITE_INPUT);
-    const float scale = (amax == 0.0f) ? 1.0f : __fdiv_rn(amax, 448.0f);
-    if (threadIdx.x == 0) scales[row] = scale;
+    for (int i = 1; i < CHUNKS; ++i) all = bf16x2_absmax(all, m[i]);
+    const float amax = __uint_as_float(row_max(bf16x2_fold(all), maxima) << 16);
     auto store_codes = [&](auto&& pair) {
 #pragma unroll
       for (int i = 0; i < CHUNKS; ++i) {
@@ -165,16 +196,24 @@ __global__ void __launch_bounds__(1024)
         if (c < chunks_per_row) {
           uint32_t q[4];
 #pragma unroll
-          for (int j = 0; j < 4; ++j) q[j] = pair(v[i][j]);
+          for (int j = 0; j < 4; ++j) q[j] = pair(pair_f32(v[i][j]));
           *reinterpret_cast<uint2*>(codes + row_off + c * 8) = make_uint2(q[0] | (q[1] << 16), q[2] | (q[3] << 16));
         }
       }
     };
-    if (e4m3_scale_is_ordinary(scale)) {
-      const F32x2 scale2 = f32x2_splat(scale), ninv = f32x2_splat(-__frcp_rn(scale));
-      store_codes([&](uint32_t w) { return e4m3_pair_ordinary(w, scale2, ninv); });
+    if (e4m3_amax_is_ordinary(amax)) {
+      const float scale = e4m3_scale_ordinary(amax);
+      const Reciprocal r = reciprocal_parts(scale);
+      const F32x2 hi = f32x2_splat(r.hi), lo = f32x2_splat(r.lo);
+      if (threadIdx.x == 0) scales[row] = scale;
+      store_codes([&](F32x2 p) { return e4m3_pair_ordinary(p, hi, lo); });
     } else {
-      store_codes([&](uint32_t w) { return e4m3_pair(w, scale); });
+      const float scale = e4m3_scale(amax);
+      if (threadIdx.x == 0) {
+        if (!(amax <= 3.0e38f)) atomicOr(status, STATUS_NONFINITE_INPUT);
+        scales[row] = scale;
+      }
+      store_codes([&](F32x2 p) { return e4m3_pair(p, scale); });
     }
   }
 }
@@ -253,9 +292,9 @@ cudaError_t launch_resnorm_quant(cudaStream_t stream, int rows, int hidden, cons
   if (!norm_geometry(hidden, &threads, &chunks)) return cudaErrorInvalidValue;
   // A row per CTA: with one 16-byte chunk per thread (640 threads for 5120 columns) three CTAs share an
   // SM, and rows beyond that wave run better on CTAs of half the threads and twice the chunks, more of
-  // which are in different phases at once.  One / two / four chunks, 5120 columns with both quantised
-  // forms: 301 rows 7.3 / 7.7 / 9.4 us, 512 rows 9.4 / 8.7 / 11.8, 1200 rows 17.2 / 16.0 / 19.1, 2048
-  // rows 25.7 / 23.9 / 25.6; two / four chunks, quantiser alone on 1024 rows of 6144: 4.8 / 4.3 us.
+  // which are in different phases at once.  Two / four chunks, 5120 columns with both quantised forms:
+  // 512 rows 5.6 / 10.6 us, 1200 rows 13.9 / 14.7, 2048 rows 21.3 / 22.7; one / two before the quotients
+  // got cheaper: 301 rows 7.3 / 7.7, 512 rows 9.4 / 8.7, 2048 rows 25.7 / 23.9.
   if (chunks <= 2) {
     static int sms = 0;
     if (sms == 0) {
