@@ -275,3 +275,33 @@ def test_dependent_launches_keep_the_order_of_a_layer(tk, batch, monkeypatch):
     for a, b in zip(*results):
         assert torch.equal(a.view(torch.uint8), b.view(torch.uint8))
     assert bool(torch.isfinite(results[0][0].float()).all())
+
+
+@pytest.mark.parametrize("batch", [1, 3, 6, 8])
+def test_recurrences_in_a_row_see_each_others_state(tk, ctx, batch):
+    """State goes in and out through asynchronous copies: steps launched back to back (each may start while the
+    one before runs) leave the bits of steps with a synchronisation between them, and no other slot changes."""
+    from tuiskollm_b200 import synth
+
+    slots, steps = 9, 6
+    bf16 = lambda i, *shape: synth.torch_normal_bf16(92, i, shape, "cuda")
+    qkv, projected, weight = bf16(1, batch, 10240), bf16(2, batch, 16384), bf16(3, 128)
+    decay = -torch.linspace(0.01, 0.5, batch * 48, device="cuda").view(batch, 48)
+    beta = torch.linspace(0.1, 0.9, batch * 48, device="cuda").view(batch, 48)
+    rows = (torch.arange(batch, dtype=torch.int32, device="cuda") * 2 + 1) % slots
+    start = torch.linspace(-0.1, 0.1, slots * 48 * 128 * 128, device="cuda").view(slots, 48, 128, 128)
+    op, got = tk.GdnRecurrenceOp(ctx), []
+    for wait in (True, False):
+        state, out = start.clone(), torch.empty((steps, batch, 6144), dtype=torch.bfloat16, device="cuda")
+        for i in range(steps):
+            op.launch(None, batch, qkv, projected, decay, beta, weight, rows, state, out[i])
+            if wait:
+                torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        got.append((state, out))
+    assert ctx.device_status() == 0
+    for a, b in zip(*got):
+        assert torch.equal(a.view(torch.uint8), b.view(torch.uint8))
+    others = [s for s in range(slots) if s not in rows.tolist()]
+    assert torch.equal(got[0][0][others], start[others])
+    assert not torch.equal(got[0][0][rows.long()], start[rows.long()])

@@ -11,12 +11,12 @@
 //     on 8 channels per thread (history, weights, input and output as 16-byte accesses).  Tokens and columns
 //     that do not exist are skipped (multiplied as zeros they were most of a one-token launch), products run
 //     on fp32 pairs and eight tokens' sums are reduced together: batch 1 3.0 -> 2.3 us, 8 4.5 -> 2.7;
-//   * the recurrence gives every (token, value head) a cluster of 4 CTAs, 32 state rows each:
-//     four times the CTAs in flight of a head-per-CTA grid at batch 1, every state byte loaded
-//     as part of an independent 16-byte request issued before any arithmetic, q/k normalised by
-//     each warp for itself (no block barrier in front of the state math), and the one value that
-//     couples the rows -- the mean square of the 128 recurrent outputs -- exchanged through
-//     distributed shared memory with a single cluster barrier.
+//   * the recurrence gives every (token, value head) a CTA.  Its 64 KB of state pass through shared memory
+//     as bulk copies that each warp issues, waits for and sends back for itself, so bytes in flight cost no
+//     registers; q and k are normalised by each warp for itself (no barrier in front of the state math), and
+//     the one value that couples the rows -- the mean square of the 128 recurrent outputs -- meets at a CTA
+//     barrier.  Prepare and recurrence in sequence, against clusters of 4 (batches above 4: 2) CTAs that held
+//     their rows in registers: batch 1 7.0 -> 6.4 us, 4 9.4 -> 9.3, 5 12.5 -> 9.5, 7 13.5 -> 12.2, 8 13.9 -> 12.6.
 #include "common.cuh"
 #include "kernels.h"
 #include "ptx.cuh"
@@ -225,8 +225,11 @@ constexpr int kHeadDim = 128;
 constexpr int kKeyHeads = 16;
 constexpr int kValueHeads = 48;
 constexpr int kQkWidth = kKeyHeads * kHeadDim;
-constexpr int kRecThreads = 256;
-constexpr int kRecWarps = kRecThreads / 32;
+constexpr int kRecWarps = 16;
+constexpr int kRecThreads = 32 * kRecWarps;
+constexpr int kRecRows = kHeadDim / kRecWarps;  // state rows of a warp
+constexpr int kRecGroup = 4;                    // rows whose reductions run side by side
+constexpr int kRecTileBytes = kHeadDim * kHeadDim * 4;
 constexpr float kRmsEpsilon = 1.0e-6f;
 constexpr float kDeltaScale = 0.08838835f;  // 1 / sqrt(128)
 
@@ -240,48 +243,46 @@ __device__ __forceinline__ float4 load_bf16x4(const uint16_t* p) {
   return make_float4(bf16x2_lo(w.x), bf16x2_hi(w.x), bf16x2_lo(w.y), bf16x2_hi(w.y));
 }
 
-// SPLIT = CTAs (one cluster) per (token, value head): 4 up to batch 4 (at most 768 CTAs of 32 state
-// rows), 2 beyond (at most 768 CTAs of 64 rows), so that every batch runs as one wave.
-template <int SPLIT>
-__global__ void __cluster_dims__(SPLIT, 1, 1) __launch_bounds__(kRecThreads)
-    gdn_recurrence_kernel(GdnRecurrenceParams p) {
-  constexpr int kRecSplit = SPLIT;
-  constexpr int kRowsPerCta = kHeadDim / kRecSplit;
-  constexpr int kRowsPerWarp = kRowsPerCta / kRecWarps;
-  // Every CTA of the cluster holds all partial sums of squares (pushed by their owners) and
-  // its own 32 recurrent outputs.
-  __shared__ float squares[kRecSplit * kRecWarps];
-  __shared__ float recurrent[kRowsPerCta];
+// One CTA per (token, value head); a warp owns kRecRows consecutive state rows.  It brings them to shared
+// memory with one bulk copy, updates them there and sends them back with another, so no register holds a
+// state byte in flight, and the value that couples the rows -- the mean square of the head's outputs --
+// meets at a CTA barrier.  Two CTAs share an SM: with registers for three, behind prepare, batches 4 and 5 took
+// 11.8 us instead of 9.4 (7 and 8 12.0 / 12.3 instead of 12.2 / 12.6), with eight warps a CTA the same.
+__global__ void __launch_bounds__(kRecThreads, 2) gdn_recurrence_kernel(GdnRecurrenceParams p) {
+  constexpr uint32_t kBytes = kRecRows * kHeadDim * 4;
+  extern __shared__ __align__(128) float tile[];  // the head's state
+  __shared__ float squares[kRecWarps];
+  __shared__ float recurrent[kHeadDim];
+  __shared__ uint64_t landed[kRecWarps];
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const uint32_t rank = cluster_cta_rank();
-  const int unit = blockIdx.x / kRecSplit;
-  const int token = unit / kValueHeads;
-  const int value_head = unit - token * kValueHeads;
+  const int token = blockIdx.x / kValueHeads;
+  const int value_head = blockIdx.x - token * kValueHeads;
   const int key_head = value_head / (kValueHeads / kKeyHeads);
-  const int row0 = static_cast<int>(rank) * kRowsPerCta + warp * kRowsPerWarp;
+  const int row0 = warp * kRecRows;
+  float* rows = tile + row0 * kHeadDim;
 
-  // First half of the "every CTA of the cluster is running" barrier a remote shared-memory store
-  // needs; the second half sits in front of the push, behind the state math.
-  cluster_arrive();
+  if (lane == 0) {
+    mbar_init(&landed[warp], 1);
+    fence_mbar_init();
+  }
   pdl_wait();
   pdl_trigger();
 
   const size_t state_row = p.state_rows[token];
   float* state = p.state + ((state_row * kValueHeads + value_head) * kHeadDim + row0) * kHeadDim;
-  // All state bytes of this warp in flight before anything depends on them.
-  float4 old_state[kRowsPerWarp];
-#pragma unroll
-  for (int i = 0; i < kRowsPerWarp; ++i)
-    old_state[i] = *reinterpret_cast<const float4*>(state + i * kHeadDim + lane * 4);
+  if (lane == 0) {
+    mbar_arrive_expect_tx(&landed[warp], kBytes);
+    bulk_load_1d(rows, state, kBytes, &landed[warp], l2_policy_evict_last());
+  }
+  __syncwarp();
 
   const uint16_t* token_qkv = p.qkv + static_cast<size_t>(token) * p.qkv_rows;
   float4 q = load_bf16x4(token_qkv + key_head * kHeadDim + lane * 4);
   float4 k = load_bf16x4(token_qkv + kQkWidth + key_head * kHeadDim + lane * 4);
-  const uint16_t* value_row = token_qkv + 2 * kQkWidth + value_head * kHeadDim + row0;
-  float value[kRowsPerWarp];
-#pragma unroll
-  for (int i = 0; i < kRowsPerWarp; ++i) value[i] = bf16_bits_to_f32(__ldg(value_row + i));
+  // lane i holds the value of the warp's row i
+  const uint16_t* values = token_qkv + 2 * kQkWidth + value_head * kHeadDim + row0;
+  const float my_value = lane < kRecRows ? bf16_bits_to_f32(__ldg(values + lane)) : 0.0f;
   const int control = token * kValueHeads + value_head;
   const float decay = ex2_approx(__ldg(p.log_decay + control) * kLog2e);
   const float beta = __ldg(p.beta + control);
@@ -292,73 +293,72 @@ __global__ void __cluster_dims__(SPLIT, 1, 1) __launch_bounds__(kRecThreads)
   q.x *= q_norm; q.y *= q_norm; q.z *= q_norm; q.w *= q_norm;
   k.x *= k_norm; k.y *= k_norm; k.z *= k_norm; k.w *= k_norm;
 
-  float state_key[kRowsPerWarp];
-#pragma unroll
-  for (int i = 0; i < kRowsPerWarp; ++i) state_key[i] = dot4(old_state[i], k);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-    for (int i = 0; i < kRowsPerWarp; ++i) state_key[i] += __shfl_xor_sync(0xffffffffu, state_key[i], o);
-  }
-  float rec[kRowsPerWarp];
-#pragma unroll
-  for (int i = 0; i < kRowsPerWarp; ++i) {
-    const float update = beta * (value[i] - decay * state_key[i]);
-    float4 s;
-    s.x = fmaf(old_state[i].x, decay, k.x * update);
-    s.y = fmaf(old_state[i].y, decay, k.y * update);
-    s.z = fmaf(old_state[i].z, decay, k.z * update);
-    s.w = fmaf(old_state[i].w, decay, k.w * update);
-    // Four-CTA clusters (batches up to 4) keep the new rows and store them behind the push below;
-    // with two-CTA clusters the registers that takes cost the sixth resident CTA per SM, and the
-    // 768 CTAs of batch 8 would no longer run as one wave.
-    if constexpr (kRecSplit == 4) old_state[i] = s;
-    else *reinterpret_cast<float4*>(state + i * kHeadDim + lane * 4) = s;
-    rec[i] = dot4(s, q);
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-    for (int i = 0; i < kRowsPerWarp; ++i) rec[i] += __shfl_xor_sync(0xffffffffu, rec[i], o);
-  }
+  const bool ok = mbar_wait(&landed[warp], 0, p.status);
   float square = 0.0f;
 #pragma unroll
-  for (int i = 0; i < kRowsPerWarp; ++i) {
-    rec[i] *= kDeltaScale;
-    square = fmaf(rec[i], rec[i], square);
-  }
-  if (lane < kRowsPerWarp) {
-    float mine = rec[0];
+  for (int i0 = 0; i0 < kRecRows; i0 += kRecGroup) {
+    float4 s[kRecGroup];
+    float sum[kRecGroup];
 #pragma unroll
-    for (int i = 1; i < kRowsPerWarp; ++i) mine = lane == i ? rec[i] : mine;
-    recurrent[warp * kRowsPerWarp + lane] = mine;
-  }
-  // Lane r pushes this warp's sum of squares into CTA r of the cluster.  Four-CTA clusters store
-  // the new state rows between the two halves of the barrier: its release half would otherwise
-  // wait for those global stores before it lets the peers see the sums (batch 1: 4.9 -> 4.6 us).
-  cluster_wait();
-  if (lane < kRecSplit)
-    st_dsmem_f32(mapa_u32(smem_u32(&squares[rank * kRecWarps + warp]), lane), square);
-  cluster_arrive();
-  if constexpr (kRecSplit == 4) {
+    for (int i = 0; i < kRecGroup; ++i) {
+      s[i] = *reinterpret_cast<const float4*>(rows + (i0 + i) * kHeadDim + lane * 4);
+      sum[i] = dot4(s[i], k);
+    }
 #pragma unroll
-    for (int i = 0; i < kRowsPerWarp; ++i)
-      *reinterpret_cast<float4*>(state + i * kHeadDim + lane * 4) = old_state[i];
+    for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+      for (int i = 0; i < kRecGroup; ++i) sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], o);
+    }
+#pragma unroll
+    for (int i = 0; i < kRecGroup; ++i) {
+      const float update = beta * (__shfl_sync(0xffffffffu, my_value, i0 + i) - decay * sum[i]);
+      s[i].x = fmaf(s[i].x, decay, k.x * update);
+      s[i].y = fmaf(s[i].y, decay, k.y * update);
+      s[i].z = fmaf(s[i].z, decay, k.z * update);
+      s[i].w = fmaf(s[i].w, decay, k.w * update);
+      *reinterpret_cast<float4*>(rows + (i0 + i) * kHeadDim + lane * 4) = s[i];
+      sum[i] = dot4(s[i], q);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+      for (int i = 0; i < kRecGroup; ++i) sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], o);
+    }
+#pragma unroll
+    for (int i = 0; i < kRecGroup; ++i) {
+      sum[i] *= kDeltaScale;
+      square = fmaf(sum[i], sum[i], square);
+      if (lane == i) recurrent[row0 + i0 + i] = sum[i];
+    }
   }
-  cluster_wait();
+  // The new rows leave while the head's outputs are finished.
+  fence_proxy_async_smem();
+  __syncwarp();
+  if (lane == 0) {
+    if (ok) {
+      bulk_store_1d(state, rows, kBytes);
+      bulk_store_commit();
+    }
+    squares[warp] = square;
+  }
+  __syncthreads();
 
-  if (tid < kRowsPerCta) {
+  if (tid < kHeadDim) {
     float total = 0.0f;
 #pragma unroll
-    for (int i = 0; i < kRecSplit * kRecWarps; ++i) total += squares[i];
+    for (int i = 0; i < kRecWarps; ++i) total += squares[i];
     const float inverse_rms = rsqrt_approx(total / static_cast<float>(kHeadDim) + kRmsEpsilon);
-    const int row = static_cast<int>(rank) * kRowsPerCta + tid;
-    const float normalized = recurrent[tid] * inverse_rms * bf16_bits_to_f32(__ldg(p.norm_weight + row));
+    const float normalized = recurrent[tid] * inverse_rms * bf16_bits_to_f32(__ldg(p.norm_weight + tid));
     const float gate = bf16_bits_to_f32(__ldg(
-        p.projected + static_cast<size_t>(token) * p.input_rows + p.qkv_rows + value_head * kHeadDim + row));
+        p.projected + static_cast<size_t>(token) * p.input_rows + p.qkv_rows + value_head * kHeadDim + tid));
     const float silu = __fdiv_rn(gate, 1.0f + ex2_approx(-gate * kLog2e));
-    p.output[static_cast<size_t>(token) * (kValueHeads * kHeadDim) + value_head * kHeadDim + row] =
+    p.output[static_cast<size_t>(token) * (kValueHeads * kHeadDim) + value_head * kHeadDim + tid] =
         static_cast<uint16_t>(f32_to_bf16_bits(normalized * silu));
+  }
+  if (lane == 0) {
+    bulk_store_wait();  // shared memory stays until the rows are in global memory
+    // a wait that gave up: give the copy in flight time to land before shared memory is released
+    for (int i = 0; i < 64 && !ok; ++i) __nanosleep(1000);
   }
 }
 
@@ -376,13 +376,12 @@ cudaError_t launch_gdn_prepare(cudaStream_t stream, const GdnPrepareParams& p) {
   return launch_kernel(gdn_prepare_kernel, dim3(grid), dim3(kPrepThreads), 0, stream, p);
 }
 
+cudaError_t gdn_prepare() {
+  return cudaFuncSetAttribute(gdn_recurrence_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRecTileBytes);
+}
+
 cudaError_t launch_gdn_recurrence(cudaStream_t stream, const GdnRecurrenceParams& p) {
-  // The cluster shape is compiled into the kernel (__cluster_dims__).
-  if (p.batch <= 4)
-    return launch_kernel(gdn_recurrence_kernel<4>, dim3(p.batch * kValueHeads * 4), dim3(kRecThreads),
-                         0, stream, p);
-  return launch_kernel(gdn_recurrence_kernel<2>, dim3(p.batch * kValueHeads * 2), dim3(kRecThreads), 0,
-                       stream, p);
+  return launch_kernel(gdn_recurrence_kernel, dim3(p.batch * kValueHeads), dim3(kRecThreads), kRecTileBytes, stream, p);
 }
 
 }  // namespace tk100

@@ -127,9 +127,11 @@ struct GdnRecurrenceParams {
   const uint32_t* state_rows;   // [batch]
   float* state;                 // [state rows, 48, 128, 128] FP32, updated in place
   uint16_t* output;             // [batch, 48 * 128] BF16
+  uint32_t* status;
 };
 // True for the one geometry the kernels are written for (16 key heads, 48 value heads of 128).
 bool gdn_geometry_ok(int hidden, int control_rows, int qkv_rows, int input_rows);
+cudaError_t gdn_prepare();  // sets the dynamic shared-memory attribute once
 cudaError_t launch_gdn_prepare(cudaStream_t stream, const GdnPrepareParams& p);
 cudaError_t launch_gdn_recurrence(cudaStream_t stream, const GdnRecurrenceParams& p);
 

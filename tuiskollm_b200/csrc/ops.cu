@@ -131,6 +131,11 @@ Status Context::create(const tk100_config& in, Context** out, std::string* error
     delete ctx;
     return TK100_ERR_MODULE;
   }
+  if ((e = gdn_prepare()) != cudaSuccess) {
+    *error = std::string("[gpu.module] preparing the GDN recurrence: ") + cudaGetErrorString(e);
+    delete ctx;
+    return TK100_ERR_MODULE;
+  }
   if ((e = fp8_projection_prepare()) != cudaSuccess) {
     *error = std::string("[gpu.module] preparing the FP8 projection routes: ") +
              cudaGetErrorString(e);
@@ -708,6 +713,7 @@ Status GdnRecurrenceOp::launch(cudaStream_t stream, int batch, const uint16_t* q
   TK100_TRY(check_plane(ctx_, what, "state", state, 16));
   TK100_TRY(check_plane(ctx_, what, "output", output, 16));
   GdnRecurrenceParams p{};
+  p.status = ctx_.status_word();
   p.batch = batch;
   p.qkv_rows = kGdnQkvRows;
   p.input_rows = kGdnInputRows;
