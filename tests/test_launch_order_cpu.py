@@ -36,3 +36,14 @@ def _kernels(source):
 def test_every_kernel_waits_for_its_predecessor(source):
     for name, body in _kernels(source):
         assert "pdl_wait()" in body, f"{source}: {name} never waits for the kernel in front of it"
+
+
+def test_a_wait_that_guards_state_has_one_verdict_per_warp():
+    """The recurrence updates its state in place, so rows go back only if all of them had arrived.  Each lane
+    updates columns of every row of its warp and one lane sends the rows: were the verdict of the bounded wait
+    that lane's own, another lane that gave up first would have its columns stored over the state.  Read from
+    the source: lanes part only while a wait is running out."""
+    body = dict(_kernels("gdn.cu"))["gdn_recurrence_kernel"]
+    waits = re.findall(r"mbar_wait\w*\(", body)
+    assert waits and len(re.findall(r"__all_sync\(0xffffffffu, mbar_wait\(", body)) == len(waits)
+    assert re.search(r"if \(ok\) \{\s*bulk_store_1d\(", body)

@@ -293,7 +293,8 @@ __global__ void __launch_bounds__(kRecThreads, 2) gdn_recurrence_kernel(GdnRecur
   q.x *= q_norm; q.y *= q_norm; q.z *= q_norm; q.w *= q_norm;
   k.x *= k_norm; k.y *= k_norm; k.z *= k_norm; k.w *= k_norm;
 
-  const bool ok = mbar_wait(&landed[warp], 0, p.status);
+  // One verdict for the warp: every lane updates columns of all its rows, and lane 0 alone sends them back.
+  const bool ok = __all_sync(0xffffffffu, mbar_wait(&landed[warp], 0, p.status));
   float square = 0.0f;
 #pragma unroll
   for (int i0 = 0; i0 < kRecRows; i0 += kRecGroup) {
