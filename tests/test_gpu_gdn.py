@@ -305,3 +305,27 @@ def test_recurrences_in_a_row_see_each_others_state(tk, ctx, batch):
     others = [s for s in range(slots) if s not in rows.tolist()]
     assert torch.equal(got[0][0][others], start[others])
     assert not torch.equal(got[0][0][rows.long()], start[rows.long()])
+
+
+def test_both_routes_of_the_recurrence_agree(tk, ctx):
+    """Up to three tokens (a head per SM) the state rows go through registers, beyond through shared memory:
+    a token's state and outputs have the same bits in a batch of either side."""
+    from tuiskollm_b200 import synth
+
+    most = 4
+    bf16 = lambda i, *shape: synth.torch_normal_bf16(93, i, shape, "cuda")
+    qkv, projected, weight = bf16(1, most, 10240), bf16(2, most, 16384), bf16(3, 128)
+    decay = -torch.linspace(0.01, 0.5, most * 48, device="cuda").view(most, 48)
+    beta = torch.linspace(0.1, 0.9, most * 48, device="cuda").view(most, 48)
+    rows = torch.tensor([2, 0, 4, 1], dtype=torch.int32, device="cuda")
+    start = torch.linspace(-0.1, 0.1, 5 * 48 * 128 * 128, device="cuda").view(5, 48, 128, 128)
+    op, got = tk.GdnRecurrenceOp(ctx), []
+    for batch in (1, 3, 4):
+        state, out = start.clone(), torch.zeros((most, 6144), dtype=torch.bfloat16, device="cuda")
+        op.launch(None, batch, qkv, projected, decay, beta, weight, rows, state, out)
+        torch.cuda.synchronize()
+        got.append((batch, state, out))
+    for batch, state, out in got[:-1]:
+        slots = rows[:batch].long()
+        assert torch.equal(state[slots].view(torch.int32), got[-1][1][slots].view(torch.int32))
+        assert torch.equal(out[:batch].view(torch.int16), got[-1][2][:batch].view(torch.int16))

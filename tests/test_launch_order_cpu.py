@@ -46,4 +46,4 @@ def test_a_wait_that_guards_state_has_one_verdict_per_warp():
     body = dict(_kernels("gdn.cu"))["gdn_recurrence_kernel"]
     waits = re.findall(r"mbar_wait\w*\(", body)
     assert waits and len(re.findall(r"__all_sync\(0xffffffffu, mbar_wait\(", body)) == len(waits)
-    assert re.search(r"if \(ok\) \{\s*bulk_store_1d\(", body)
+    assert re.search(r"\bok\) \{\s*bulk_store_1d\(", body)

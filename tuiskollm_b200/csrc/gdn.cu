@@ -11,12 +11,11 @@
 //     on 8 channels per thread (history, weights, input and output as 16-byte accesses).  Tokens and columns
 //     that do not exist are skipped (multiplied as zeros they were most of a one-token launch), products run
 //     on fp32 pairs and eight tokens' sums are reduced together: batch 1 3.0 -> 2.3 us, 8 4.5 -> 2.7;
-//   * the recurrence gives every (token, value head) a CTA.  Its 64 KB of state pass through shared memory
-//     as bulk copies that each warp issues, waits for and sends back for itself, so bytes in flight cost no
-//     registers; q and k are normalised by each warp for itself (no barrier in front of the state math), and
-//     the one value that couples the rows -- the mean square of the 128 recurrent outputs -- meets at a CTA
-//     barrier.  Prepare and recurrence in sequence, against clusters of 4 (batches above 4: 2) CTAs that held
-//     their rows in registers: batch 1 7.0 -> 6.4 us, 4 9.4 -> 9.3, 5 12.5 -> 9.5, 7 13.5 -> 12.2, 8 13.9 -> 12.6.
+//   * the recurrence gives every (token, value head) a CTA, whose warps own its state rows.  Where every head has
+//     an SM to itself (batches up to 3) the rows pass through registers; beyond that through shared memory, as bulk
+//     copies that each warp issues, waits for and sends back for itself, so bytes in flight cost no registers.  q
+//     and k are normalised by each warp for itself (no barrier in front of the state math), and the one value that
+//     couples the rows -- the mean square of the 128 recurrent outputs -- meets at a CTA barrier.
 #include "common.cuh"
 #include "kernels.h"
 #include "ptx.cuh"
@@ -243,14 +242,15 @@ __device__ __forceinline__ float4 load_bf16x4(const uint16_t* p) {
   return make_float4(bf16x2_lo(w.x), bf16x2_hi(w.x), bf16x2_lo(w.y), bf16x2_hi(w.y));
 }
 
-// One CTA per (token, value head); a warp owns kRecRows consecutive state rows.  It brings them to shared
-// memory with one bulk copy, updates them there and sends them back with another, so no register holds a
-// state byte in flight, and the value that couples the rows -- the mean square of the head's outputs --
-// meets at a CTA barrier.  Two CTAs share an SM: with registers for three, behind prepare, batches 4 and 5 took
-// 11.8 us instead of 9.4 (7 and 8 12.0 / 12.3 instead of 12.2 / 12.6), with eight warps a CTA the same.
-__global__ void __launch_bounds__(kRecThreads, 2) gdn_recurrence_kernel(GdnRecurrenceParams p) {
+// One CTA per (token, value head); a warp owns kRecRows consecutive state rows.  THROUGH_SHARED: it brings them to
+// shared memory with one bulk copy, updates them there and sends them back with another, so no register holds a
+// state byte in flight and two CTAs share an SM.  Otherwise the rows go through registers: no barrier and no trip
+// through shared memory on the chain, but one CTA per SM, so it is taken where every head has an SM to itself.
+// The value that couples the rows, the mean square of the head's outputs, meets at a CTA barrier.
+template <bool THROUGH_SHARED>
+__global__ void __launch_bounds__(kRecThreads, THROUGH_SHARED ? 2 : 1) gdn_recurrence_kernel(GdnRecurrenceParams p) {
   constexpr uint32_t kBytes = kRecRows * kHeadDim * 4;
-  extern __shared__ __align__(128) float tile[];  // the head's state
+  extern __shared__ __align__(128) float tile[];  // THROUGH_SHARED: the head's state
   __shared__ float squares[kRecWarps];
   __shared__ float recurrent[kHeadDim];
   __shared__ uint64_t landed[kRecWarps];
@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(kRecThreads, 2) gdn_recurrence_kernel(GdnRecur
   const int row0 = warp * kRecRows;
   float* rows = tile + row0 * kHeadDim;
 
-  if (lane == 0) {
+  if (THROUGH_SHARED && lane == 0) {
     mbar_init(&landed[warp], 1);
     fence_mbar_init();
   }
@@ -271,11 +271,17 @@ __global__ void __launch_bounds__(kRecThreads, 2) gdn_recurrence_kernel(GdnRecur
 
   const size_t state_row = p.state_rows[token];
   float* state = p.state + ((state_row * kValueHeads + value_head) * kHeadDim + row0) * kHeadDim;
-  if (lane == 0) {
-    mbar_arrive_expect_tx(&landed[warp], kBytes);
-    bulk_load_1d(rows, state, kBytes, &landed[warp], l2_policy_evict_last());
+  float4 old[THROUGH_SHARED ? 1 : kRecRows];
+  if constexpr (THROUGH_SHARED) {
+    if (lane == 0) {
+      mbar_arrive_expect_tx(&landed[warp], kBytes);
+      bulk_load_1d(rows, state, kBytes, &landed[warp], l2_policy_evict_last());
+    }
+    __syncwarp();
+  } else {
+#pragma unroll
+    for (int i = 0; i < kRecRows; ++i) old[i] = *reinterpret_cast<const float4*>(state + i * kHeadDim + lane * 4);
   }
-  __syncwarp();
 
   const uint16_t* token_qkv = p.qkv + static_cast<size_t>(token) * p.qkv_rows;
   float4 q = load_bf16x4(token_qkv + key_head * kHeadDim + lane * 4);
@@ -287,6 +293,14 @@ __global__ void __launch_bounds__(kRecThreads, 2) gdn_recurrence_kernel(GdnRecur
   const float decay = ex2_approx(__ldg(p.log_decay + control) * kLog2e);
   const float beta = __ldg(p.beta + control);
 
+  // The first kHeadDim threads finish the outputs; what they need for that is asked for before the state math.
+  float weight = 0.0f, gate = 0.0f;
+  if (tid < kHeadDim) {
+    weight = bf16_bits_to_f32(__ldg(p.norm_weight + tid));
+    gate = bf16_bits_to_f32(__ldg(
+        p.projected + static_cast<size_t>(token) * p.input_rows + p.qkv_rows + value_head * kHeadDim + tid));
+  }
+
   // L2 normalisation of q and k over the head (device/gdn_recurrence.rs:79-105); each warp for itself.
   const float q_norm = rsqrt_approx(warp_sum(dot4(q, q)) + kRmsEpsilon);
   const float k_norm = rsqrt_approx(warp_sum(dot4(k, k)) + kRmsEpsilon);
@@ -294,7 +308,8 @@ __global__ void __launch_bounds__(kRecThreads, 2) gdn_recurrence_kernel(GdnRecur
   k.x *= k_norm; k.y *= k_norm; k.z *= k_norm; k.w *= k_norm;
 
   // One verdict for the warp: every lane updates columns of all its rows, and lane 0 alone sends them back.
-  const bool ok = __all_sync(0xffffffffu, mbar_wait(&landed[warp], 0, p.status));
+  bool ok = true;
+  if constexpr (THROUGH_SHARED) ok = __all_sync(0xffffffffu, mbar_wait(&landed[warp], 0, p.status));
   float square = 0.0f;
 #pragma unroll
   for (int i0 = 0; i0 < kRecRows; i0 += kRecGroup) {
@@ -302,7 +317,8 @@ __global__ void __launch_bounds__(kRecThreads, 2) gdn_recurrence_kernel(GdnRecur
     float sum[kRecGroup];
 #pragma unroll
     for (int i = 0; i < kRecGroup; ++i) {
-      s[i] = *reinterpret_cast<const float4*>(rows + (i0 + i) * kHeadDim + lane * 4);
+      if constexpr (THROUGH_SHARED) s[i] = *reinterpret_cast<const float4*>(rows + (i0 + i) * kHeadDim + lane * 4);
+      else s[i] = old[i0 + i];
       sum[i] = dot4(s[i], k);
     }
 #pragma unroll
@@ -317,7 +333,7 @@ __global__ void __launch_bounds__(kRecThreads, 2) gdn_recurrence_kernel(GdnRecur
       s[i].y = fmaf(s[i].y, decay, k.y * update);
       s[i].z = fmaf(s[i].z, decay, k.z * update);
       s[i].w = fmaf(s[i].w, decay, k.w * update);
-      *reinterpret_cast<float4*>(rows + (i0 + i) * kHeadDim + lane * 4) = s[i];
+      *reinterpret_cast<float4*>((THROUGH_SHARED ? rows : state) + (i0 + i) * kHeadDim + lane * 4) = s[i];
       sum[i] = dot4(s[i], q);
     }
 #pragma unroll
@@ -332,15 +348,15 @@ __global__ void __launch_bounds__(kRecThreads, 2) gdn_recurrence_kernel(GdnRecur
       if (lane == i) recurrent[row0 + i0 + i] = sum[i];
     }
   }
+  if (lane == 0) squares[warp] = square;
   // The new rows leave while the head's outputs are finished.
-  fence_proxy_async_smem();
-  __syncwarp();
-  if (lane == 0) {
-    if (ok) {
+  if constexpr (THROUGH_SHARED) {
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0 && ok) {
       bulk_store_1d(state, rows, kBytes);
       bulk_store_commit();
     }
-    squares[warp] = square;
   }
   __syncthreads();
 
@@ -349,14 +365,12 @@ __global__ void __launch_bounds__(kRecThreads, 2) gdn_recurrence_kernel(GdnRecur
 #pragma unroll
     for (int i = 0; i < kRecWarps; ++i) total += squares[i];
     const float inverse_rms = rsqrt_approx(total / static_cast<float>(kHeadDim) + kRmsEpsilon);
-    const float normalized = recurrent[tid] * inverse_rms * bf16_bits_to_f32(__ldg(p.norm_weight + tid));
-    const float gate = bf16_bits_to_f32(__ldg(
-        p.projected + static_cast<size_t>(token) * p.input_rows + p.qkv_rows + value_head * kHeadDim + tid));
+    const float normalized = recurrent[tid] * inverse_rms * weight;
     const float silu = __fdiv_rn(gate, 1.0f + ex2_approx(-gate * kLog2e));
     p.output[static_cast<size_t>(token) * (kValueHeads * kHeadDim) + value_head * kHeadDim + tid] =
         static_cast<uint16_t>(f32_to_bf16_bits(normalized * silu));
   }
-  if (lane == 0) {
+  if (THROUGH_SHARED && lane == 0) {
     bulk_store_wait();  // shared memory stays until the rows are in global memory
     // a wait that gave up: give the copy in flight time to land before shared memory is released
     for (int i = 0; i < 64 && !ok; ++i) __nanosleep(1000);
@@ -378,11 +392,16 @@ cudaError_t launch_gdn_prepare(cudaStream_t stream, const GdnPrepareParams& p) {
 }
 
 cudaError_t gdn_prepare() {
-  return cudaFuncSetAttribute(gdn_recurrence_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRecTileBytes);
+  return cudaFuncSetAttribute(gdn_recurrence_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRecTileBytes);
 }
 
-cudaError_t launch_gdn_recurrence(cudaStream_t stream, const GdnRecurrenceParams& p) {
-  return launch_kernel(gdn_recurrence_kernel, dim3(p.batch * kValueHeads), dim3(kRecThreads), kRecTileBytes, stream, p);
+cudaError_t launch_gdn_recurrence(cudaStream_t stream, const GdnRecurrenceParams& p, int sm_count) {
+  const dim3 grid(p.batch * kValueHeads), block(kRecThreads);
+  // Registers / shared memory, prepare and recurrence in sequence: batch 1 5.9 / 6.5 us, 2 6.4 / 8.5, 3 7.0 / 9.0,
+  // 4 10.3 / 9.6, 8 14.9 / 13.4 (the recurrence alone 3.6 / 4.2, 3.8 / 4.3, 4.2 / 4.5, 7.4 / 6.8, 11.9 / 10.7).
+  if (static_cast<int>(grid.x) <= sm_count)
+    return launch_kernel(gdn_recurrence_kernel<false>, grid, block, 0, stream, p);
+  return launch_kernel(gdn_recurrence_kernel<true>, grid, block, kRecTileBytes, stream, p);
 }
 
 }  // namespace tk100

@@ -133,7 +133,7 @@ struct GdnRecurrenceParams {
 bool gdn_geometry_ok(int hidden, int control_rows, int qkv_rows, int input_rows);
 cudaError_t gdn_prepare();  // sets the dynamic shared-memory attribute once
 cudaError_t launch_gdn_prepare(cudaStream_t stream, const GdnPrepareParams& p);
-cudaError_t launch_gdn_recurrence(cudaStream_t stream, const GdnRecurrenceParams& p);
+cudaError_t launch_gdn_recurrence(cudaStream_t stream, const GdnRecurrenceParams& p, int sm_count);
 
 // --------------------------------------------------------------- materialize.cu
 constexpr int kMaterializeMaxPlanes = 3;

@@ -726,7 +726,7 @@ Status GdnRecurrenceOp::launch(cudaStream_t stream, int batch, const uint16_t* q
   p.state = state;
   p.output = output;
   ctx_.count_launch();
-  return ctx_.check(launch_gdn_recurrence(stream, p), "launching GDN recurrence");
+  return ctx_.check(launch_gdn_recurrence(stream, p, ctx_.sm_count()), "launching GDN recurrence");
 }
 
 Status ResidualNormOp::launch_plain(cudaStream_t stream, int batch, const uint16_t* input,
