@@ -275,7 +275,9 @@ __global__ void __launch_bounds__(kRecThreads, THROUGH_SHARED ? 2 : 1) gdn_recur
   if constexpr (THROUGH_SHARED) {
     if (lane == 0) {
       mbar_arrive_expect_tx(&landed[warp], kBytes);
-      bulk_load_1d(rows, state, kBytes, &landed[warp], l2_policy_evict_last());
+      // No L2 policy: the rows are not read again before the next token.  Over eight layers in turn (920 MB of
+      // weights, up to 25 MB of state each) evict_first and evict_last gave the same times within 1.5 %.
+      bulk_load_1d(rows, state, kBytes, &landed[warp]);
     }
     __syncwarp();
   } else {
