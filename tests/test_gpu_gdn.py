@@ -133,6 +133,31 @@ def test_prepare_random_planes(tk, ctx):
         assert np.array_equal(history, want_history)
 
 
+@pytest.mark.parametrize("hidden", [128, 2560, 2688, 5248, 7808, 10240])
+def test_prepare_of_other_widths(tk, hidden):
+    """The control mat-vec walks pairs of 2560-column steps: a row shorter than one step, a pair whose second
+    step is absent or partial, a second pair that is partial (its second step absent or partial) or whole."""
+    from oracle import tuisko_oracle as O
+    rng = np.random.default_rng(hidden)
+    normal = lambda std, *shape: O.f32_to_bf16(rng.normal(0, std, shape).astype(np.float32)).reshape(shape)
+    f = dict(input=normal(1.0, MAX_BATCH, hidden), control_weights=normal(0.02, 96, hidden),
+             a_log=O.f32_to_bf16(rng.uniform(-3, 1, 48).astype(np.float32)), dt_bias=normal(1.0, 48),
+             projected=normal(1.5, MAX_BATCH, 16384), convolution_weights=normal(0.5, 10240, 4),
+             history=normal(1.5, MAX_BATCH, 10240, 3), state_rows=np.arange(MAX_BATCH, dtype=np.uint32))
+    planes = PreparePlanes(f)
+    op = tk.GdnPrepareOp(tk.Context(device=0, hidden=hidden))
+    for batch in (1, 3, 8):
+        planes.reset()
+        planes.launch(op, batch)
+        log_decay, beta, _, _ = planes.observe()
+        want_decay, want_beta = G.gdn_controls(f["input"][:batch], f["control_weights"], f["a_log"], f["dt_bias"])
+        # as for the random planes above; one missing 16-byte chunk of a row moves a sum by about 0.06
+        assert (np.abs(log_decay[:batch] - want_decay) <= 0.002 * np.maximum(1.0, np.abs(want_decay))).all()
+        assert np.abs(beta[:batch] - want_beta).max() <= 0.002
+        for p in (planes.log_decay, planes.beta):
+            assert_inactive_untouched(p, batch)
+
+
 class RecurrencePlanes:
     def __init__(self, f):
         self.f = f

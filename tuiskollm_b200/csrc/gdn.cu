@@ -129,6 +129,7 @@ __global__ void __launch_bounds__(kPrepThreads) gdn_prepare_kernel(GdnPreparePar
       const float sum = warp_sum(acc[0]);
       if (lane == 0) partial[warp][0] = sum;
     } else {
+      static_assert(kGdnMaxBatch == 8, "the exchanges below are for eight sums");
       // Eight sums over 32 lanes in nine exchanges: at offsets 16, 8 and 4 a lane hands half of its tokens to
       // its partner, and lane l ends with token l / 4.
 #pragma unroll
@@ -393,7 +394,7 @@ cudaError_t launch_gdn_prepare(cudaStream_t stream, const GdnPrepareParams& p) {
   return launch_kernel(gdn_prepare_kernel, dim3(grid), dim3(kPrepThreads), 0, stream, p);
 }
 
-cudaError_t gdn_prepare() {
+cudaError_t gdn_recurrence_prepare() {
   return cudaFuncSetAttribute(gdn_recurrence_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRecTileBytes);
 }
 

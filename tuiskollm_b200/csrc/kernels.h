@@ -131,7 +131,7 @@ struct GdnRecurrenceParams {
 };
 // True for the one geometry the kernels are written for (16 key heads, 48 value heads of 128).
 bool gdn_geometry_ok(int hidden, int control_rows, int qkv_rows, int input_rows);
-cudaError_t gdn_prepare();  // sets the dynamic shared-memory attribute once
+cudaError_t gdn_recurrence_prepare();  // sets its kernel's dynamic shared-memory attribute once
 cudaError_t launch_gdn_prepare(cudaStream_t stream, const GdnPrepareParams& p);
 cudaError_t launch_gdn_recurrence(cudaStream_t stream, const GdnRecurrenceParams& p, int sm_count);
 
