@@ -257,3 +257,48 @@ def test_every_pair_of_significands_rounds_as_the_division(tk, oracle, exponent)
     oc, os_ = oracle.quantize_e4m3(bits)
     assert np.array_equal(host(scales), os_) and np.array_equal(host(codes), oc)
     assert c.device_status() == 0
+
+
+@pytest.mark.parametrize("cols,ctas", [(2048, 8), (2560, 6), (5120, 3), (6144, 4), (10240, 2)])
+def test_quantiser_on_both_sides_of_a_wave(tk, ctx, oracle, cols, ctas):
+    """Rows beyond one wave of CTAs (`ctas` to an SM) are quantised by four chunks a thread: the last count of one
+    side, the first of the other, and a ragged one further on."""
+    from tuiskollm_b200 import synth
+
+    wave = torch.cuda.get_device_properties(0).multi_processor_count * ctas
+    bits = synth.normal_bf16(79, cols, (min(wave + 37, 2048), cols))
+    want_codes, want_scales = oracle.quantize_e4m3(bits)
+    x = dev(bits.view(np.int16))
+    for rows in sorted({min(wave, 2048), min(wave + 1, 2048), bits.shape[0]}):
+        codes = sentinel_plane((rows + 1, cols), torch.uint8)
+        scales = sentinel_plane((rows + 1,), torch.float32)
+        tk.Fp8ProjectionOp(ctx).quantize(None, rows, cols, x, codes, scales)
+        torch.cuda.synchronize()
+        assert np.array_equal(host(codes)[:rows], want_codes[:rows])
+        assert np.array_equal(host(scales)[:rows], want_scales[:rows])
+        assert_inactive_untouched(codes, rows)
+        assert_inactive_untouched(scales, rows)
+
+
+@pytest.mark.parametrize("hidden,ctas", [(2560, 6), (8192, 4)])
+def test_norm_on_both_sides_of_a_wave(tk, oracle, hidden, ctas):
+    """The fused producer doubles its chunks beyond a wave, from one to two and from two to four."""
+    from tuiskollm_b200 import synth
+
+    wave = torch.cuda.get_device_properties(0).multi_processor_count * ctas
+    xb, bb = (synth.normal_bf16(80, i, (wave + 1, hidden)) for i in (1, 2))
+    wb = synth.normal_bf16(80, 3, (hidden,), std=0.1)
+    want_res, want_norm = oracle.residual_rms_norm(xb, bb, wb, 1e-6)
+    x, branch, weight = (dev(a.view(np.int16)) for a in (xb, bb, wb))
+    op = tk.ResidualNormOp(tk.Context(device=0, hidden=hidden))
+    for rows in (wave, wave + 1):
+        residual, normed = (sentinel_plane((rows + 1, hidden), torch.int16) for _ in range(2))
+        codes, scales = sentinel_plane((rows + 1, hidden), torch.uint8), sentinel_plane((rows + 1,), torch.float32)
+        op.launch_quantize(None, rows, x, branch, weight, residual, normed, codes, scales)
+        torch.cuda.synchronize()
+        assert np.array_equal(_u16(residual)[:rows], want_res[:rows])
+        check_close(_u16(normed)[:rows], oracle.bf16_to_f32(want_norm[:rows]).astype(np.float64), 1 / 64, 0.005)
+        oc, os_ = oracle.quantize_e4m3(_u16(normed)[:rows])
+        assert np.array_equal(host(codes)[:rows], oc) and np.array_equal(host(scales)[:rows], os_)
+        for plane in (residual, normed, codes, scales):
+            assert_inactive_untouched(plane, rows)

@@ -290,11 +290,15 @@ cudaError_t launch_resnorm_quant(cudaStream_t stream, int rows, int hidden, cons
   const Nvfp4Out nv{nvfp4_codes, nvfp4_scales, nvfp4_divisor};
   int threads = 0, chunks = 0;
   if (!norm_geometry(hidden, &threads, &chunks)) return cudaErrorInvalidValue;
-  // A row per CTA: with one 16-byte chunk per thread (640 threads for 5120 columns) three CTAs share an
-  // SM, and rows beyond that wave run better on CTAs of half the threads and twice the chunks, more of
-  // which are in different phases at once.  Two / four chunks, 5120 columns with both quantised forms:
-  // 512 rows 5.6 / 10.6 us, 1200 rows 13.9 / 14.7, 2048 rows 21.3 / 22.7; one / two before the quotients
-  // got cheaper: 301 rows 7.3 / 7.7, 512 rows 9.4 / 8.7, 2048 rows 25.7 / 23.9.
+  const bool has_branch = branch != nullptr;
+  const bool do_norm = normalized_out != nullptr;
+  const bool do_quant = codes != nullptr;
+  // A row per CTA.  Rows beyond one wave of CTAs run better on more of them with fewer threads and more chunks,
+  // which are in different phases at once.  The quantiser alone takes four chunks there: 6144 columns (384 threads
+  // x 2, four CTAs per SM at 40 registers), two / four chunks: 600 rows 4.6 / 3.8 us, 740 5.4 / 4.1, 2048 10.8 / 7.9;
+  // 5120 columns, one / two / four: 600 rows 4.1 / 4.5 / 3.6, 2048 9.4 / 10.0 / 6.8.  With the norm the chunks
+  // double; 5120 columns, one / two / four: 512 rows 7.0 / 6.5 / 8.7, 800 9.2 / 9.5 / 10.5, 1024 rows and
+  // more equal; 10240 columns, two / four: 600 rows 13.9 / 15.1, 1024 21.8 / 20.5, 2048 38.9 / 36.9.
   if (chunks <= 2) {
     static int sms = 0;
     if (sms == 0) {
@@ -304,15 +308,14 @@ cudaError_t launch_resnorm_quant(cudaStream_t stream, int rows, int hidden, cons
         sms = 148;
       }
     }
-    const int half = (((hidden >> 3) + 2 * chunks - 1) / (2 * chunks) + 31) & ~31;
-    if (rows > sms * (2048 / threads) && half >= 128) {
-      chunks *= 2;
-      threads = half;
+    const int resident = !do_norm && chunks == 2 ? 1536 : 2048;  // threads of an SM
+    const int wide = do_norm ? 2 * chunks : 4;
+    const int narrow = (((hidden >> 3) + wide - 1) / wide + 31) & ~31;
+    if (rows > sms * (resident / threads) && narrow >= (do_norm ? 128 : 64)) {
+      chunks = wide;
+      threads = narrow;
     }
   }
-  const bool has_branch = branch != nullptr;
-  const bool do_norm = normalized_out != nullptr;
-  const bool do_quant = codes != nullptr;
 #define TK100_CASE(B, N, Q)                                                                      \
   if (has_branch == B && do_norm == N && do_quant == Q)                                          \
   return launch_chunks<B, N, Q>(stream, rows, hidden, threads, chunks, x, branch, weight,        \
