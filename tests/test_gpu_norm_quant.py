@@ -205,9 +205,9 @@ def test_rejected_launches_report_gpu_launch(tk, ctx):
 
 @pytest.mark.parametrize("cols,rows", [(256, 64), (5120, 3), (5120, 500)])
 def test_quotients_of_every_scale_round_as_the_division(tk, oracle, cols, rows):
-    """E4M3 and NVFP4 codes come from residual steps on one reciprocal per row or block: rows whose scale
-    runs through the whole BF16 range (the E4M3 route leaves the reciprocal for the division below 2^-80),
-    quotients on the rounding boundaries, signed zeros, and a NaN that must not disturb its neighbours."""
+    """E4M3 and NVFP4 codes come from products with a two-part reciprocal per row or block: rows whose maximum
+    runs through the whole BF16 range (the E4M3 route divides below 2^-60 and above 2^97), quotients on the
+    rounding boundaries, signed zeros, and a NaN that must not disturb its neighbours' E4M3 codes."""
     rng = np.random.default_rng(cols + rows)
     exps = rng.integers(-130, 120, rows)
     x = rng.standard_normal((rows, cols)) * np.exp2(exps.astype(np.float64))[:, None]
@@ -239,11 +239,11 @@ def test_quotients_of_every_scale_round_as_the_division(tk, oracle, cols, rows):
     assert np.array_equal(host(scales), os_) and np.array_equal(host(codes), oc)
 
 
-@pytest.mark.parametrize("exponent", [-66, -60, 0, 96])
+@pytest.mark.parametrize("exponent", [-66, -60, 0, 96, 97, 110])
 def test_every_pair_of_significands_rounds_as_the_division(tk, oracle, exponent):
     """E4M3 scales and codes come from products with a two-part reciprocal: all 128 significands a row maximum
-    can have (exponents on both sides of the range the products are used in) against all 128 of a value,
-    down to 2^-20 of the maximum."""
+    can have (exponents inside and on both sides of the range the products are used in; at 97 the power of two
+    alone is still inside) against all 128 of a value, down to 2^-20 of the maximum."""
     mant = 1.0 + np.arange(128) / 128.0
     values = np.concatenate([mant * 2.0 ** -e for e in range(20)])
     x = np.minimum(values[None, :], mant[:, None])
@@ -257,6 +257,72 @@ def test_every_pair_of_significands_rounds_as_the_division(tk, oracle, exponent)
     oc, os_ = oracle.quantize_e4m3(bits)
     assert np.array_equal(host(scales), os_) and np.array_equal(host(codes), oc)
     assert c.device_status() == 0
+
+
+def _nonfinite_columns(bits):
+    """NaN in a low and in a high half of a pair, infinities in blocks of their own, and a block of NaN alone."""
+    bits[..., 5] = 0x7FC0
+    bits[..., 22] = 0xFFC0
+    bits[..., 40] = 0x7F80
+    bits[..., 57] = 0xFF80
+    bits[..., 64:80] = 0x7FC0
+    return bits
+
+
+@pytest.mark.parametrize("cols", [256, 5120])
+def test_nonfinite_values_stay_in_their_place(tk, oracle, cols):
+    """NVFP4: a NaN is left out of its block's maximum and codes as the largest magnitude, an infinity saturates
+    the block's scale and its own code; neighbours code as without them.  E4M3: an infinity makes the row's
+    scale infinite and sets the status bit, a NaN alone does not."""
+    from tuiskollm_b200 import _lib, synth
+
+    rows = 3
+    bits = _nonfinite_columns(synth.normal_bf16(77, 1, (rows, cols)))
+    nan = (bits & 0x7FFF) > 0x7F80
+    c = tk.Context(device=0)
+    c4 = torch.zeros((rows, cols // 2), dtype=torch.uint8, device="cuda")
+    s4 = torch.zeros((tk.ops.nvfp4_scale_plane_bytes(rows, cols),), dtype=torch.uint8, device="cuda")
+    tk.Nvfp4SwiGluOp(c).quantize(None, rows, cols, dev(bits.view(np.int16)), 448.0, c4, s4)
+    qc, qs = oracle.nvfp4_quantize(np.where(nan, 0, bits).astype(np.uint16), 448.0)
+    nibbles = np.stack([qc & 15, qc >> 4], axis=-1).reshape(rows, cols)
+    nibbles[nan] = 7
+    nibbles[:, 64:80] = 0  # no finite value: scale 0, zeros with the sign of the value
+    got = host(c4)
+    assert np.array_equal(np.stack([got & 15, got >> 4], axis=-1).reshape(rows, cols), nibbles)
+    assert np.array_equal(host(s4), qs)
+
+    codes, scales = (torch.zeros((rows, cols), dtype=torch.uint8, device="cuda"),
+                     torch.zeros((rows,), dtype=torch.float32, device="cuda"))
+    tk.ops.Fp8ProjectionOp(c).quantize(None, rows, cols, dev(bits.view(np.int16)), codes, scales)
+    assert c.device_status() == _lib.DEVICE_NONFINITE_INPUT
+    nonfinite = (bits & 0x7F80) == 0x7F80
+    want = np.where(nonfinite, 0x7F, (bits >> 8) & 0x80).astype(np.uint8)
+    assert np.isinf(host(scales)).all() and np.array_equal(host(codes), want)
+
+
+def test_nonfinite_values_behind_the_norm(tk, oracle):
+    """The fused producer's two quantised forms of a row with NaN and infinities (from the norm weight) are those
+    of the stand-alone quantisers on the row that it wrote."""
+    from tuiskollm_b200 import synth
+
+    rows, hidden = 3, 5120
+    x, branch = (dev(synth.normal_bf16(78, i, (rows, hidden)).view(np.int16)) for i in (1, 2))
+    weight = dev(_nonfinite_columns(synth.normal_bf16(78, 3, (hidden,), std=0.1)).view(np.int16))
+    c = tk.Context(device=0)
+    i16 = lambda: torch.zeros((rows, hidden), dtype=torch.int16, device="cuda")
+    forms = lambda: (torch.zeros((rows, hidden), dtype=torch.uint8, device="cuda"),
+                     torch.zeros((rows,), dtype=torch.float32, device="cuda"),
+                     torch.zeros((rows, hidden // 2), dtype=torch.uint8, device="cuda"),
+                     torch.zeros((tk.ops.nvfp4_scale_plane_bytes(rows, hidden),), dtype=torch.uint8, device="cuda"))
+    residual, normed, got, want = i16(), i16(), forms(), forms()
+    tk.ResidualNormOp(c).launch_quantize_nvfp4(None, rows, x, branch, weight, residual, normed, got[0], got[1],
+                                               448.0, got[2], got[3])
+    tk.ops.Fp8ProjectionOp(c).quantize(None, rows, hidden, normed, want[0], want[1])
+    tk.Nvfp4SwiGluOp(c).quantize(None, rows, hidden, normed, 448.0, want[2], want[3])
+    row = _u16(normed)
+    assert ((row[:, 5] & 0x7FFF) > 0x7F80).all() and ((row[:, 40] & 0x7FFF) == 0x7F80).all()
+    for a, b in zip(got, want):
+        assert torch.equal(a.view(torch.uint8), b.view(torch.uint8))
 
 
 @pytest.mark.parametrize("cols,ctas", [(2048, 8), (2560, 6), (5120, 3), (6144, 4), (10240, 2)])
