@@ -9,18 +9,16 @@
 //
 // Instruction issue bounds it beyond one wave of rows (2048 rows with both quantised forms: 12.7 M warp
 // instructions, two thirds of the issue slots, 21.3 us where the 98 MB take 15.3 at the copy rate); below that
-// its chain of load, two block reductions and store does.  So every quotient is two operations on fp32 pairs
-// (reciprocal_parts), maxima are packed BF16 and reduced as integers, a reduction has one barrier, and a row's
-// values stay widened.  With residual steps on a rounded reciprocal, IEEE divides per block and row and rows
-// unpacked at each use: 16.0 M instructions; 2048 rows 24.2 us, 512 7.0 (now 5.6), 300 6.5 (5.2), 33 4.1 (2.7),
-// one 3.0 (2.65).
+// its chain of load, two block reductions and store does (one row 2.6 us).  So every quotient is two operations
+// on fp32 pairs (reciprocal_parts), maxima are packed BF16 and reduced as integers, a reduction has one barrier,
+// and a row's values stay widened.
 //
 // Numeric contract (bit-exact parts marked *):
 //   res  = bf16_rn(f32(x) + f32(branch))                                  *
 //   r    = 1/sqrt(sum(res^2)/H + eps), fp32, fixed summation order
 //   y    = bf16_rn(res * r * (1 + w)), evaluated left to right in fp32
-//   amax = max |y|; scale = amax == 0 ? 1 : amax / 448   (IEEE fp32 divide)   *
-//   code = e4m3_rn_satfinite(y / scale)                  (IEEE fp32 quotient) *
+//   amax = max |y|; scale = amax == 0 ? 1 : amax / 448   (as the fp32 divide rounds) *
+//   code = e4m3_rn_satfinite(y / scale)                  (likewise)          *
 // The starred results are bit-exact functions of their inputs; `codes`/`scale`
 // are exact with respect to the normalised row this same kernel wrote.
 #include <cstdlib>
