@@ -68,6 +68,34 @@ def test_fp8_projection(tk, oracle, monkeypatch, out_rows, k, rows, tok, splits)
     assert c.device_status() == 0
 
 
+@pytest.mark.parametrize("tok,splits", [(64, 1), (160, 1), (256, 1), (160, 2), (256, 3), (224, 4)])
+def test_one_tile_per_pair_has_the_bits_of_one_cta_tiles(tk, monkeypatch, tok, splits):
+    """One tile per pair, more stages than the ring holds (which then reaches over the epilogue's transposition
+    space), every place of a split's own values in the sum: the kernel of one-CTA tiles cuts K at the same places
+    and adds the parts in the same order, so every output bit agrees."""
+    from tuiskollm_b200 import synth
+
+    out_rows, k, rows = 768, 5120, tok - 3
+    xb = synth.normal_bf16(66, tok, (rows, k))
+    w, s = synth.torch_fp8_weights(66, 1, out_rows, k, "cuda")
+    outs = []
+    for env in ({"TK100_PAIR_TOK": tok, "TK100_PAIR_SPLITS": splits}, {"TK100_SPLITS": splits, "TK100_BLOCK_TOK": 64}):
+        for name in ("TK100_PAIR_TOK", "TK100_PAIR_SPLITS", "TK100_SPLITS", "TK100_BLOCK_TOK"):
+            monkeypatch.setenv(name, str(env.get(name, 0)))
+        c = tk.Context(device=0)
+        codes = torch.zeros((rows, k), dtype=torch.uint8, device="cuda")
+        scales = torch.zeros((rows,), dtype=torch.float32, device="cuda")
+        out = sentinel_plane((rows + 1, out_rows), torch.int16)
+        tk.ops.Fp8ProjectionOp(c).launch(None, rows, out_rows, k, dev(xb.view(np.int16)), codes, scales, w, s, out)
+        torch.cuda.synchronize()
+        kernel = "pair_gemm_kernel" if "TK100_PAIR_TOK" in env else "fp8_projection_kernel<64"
+        assert c.last_kernel.startswith(kernel) and f"splits={splits}" in c.last_kernel, c.last_kernel
+        assert c.device_status() == 0
+        assert_inactive_untouched(out, rows)
+        outs.append(out[:rows])
+    assert torch.equal(outs[0], outs[1])
+
+
 @pytest.mark.parametrize("out_rows,k,rows,kernel", [
     (1040, 3072, 48, "fp8_projection_kernel<64"),    # three splits planned: one-CTA tiles up to 48 tokens
     (1040, 3072, 49, "pair_gemm_kernel"),

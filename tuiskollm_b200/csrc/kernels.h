@@ -331,7 +331,8 @@ struct PairGemmParams {
   uint32_t* status;
 };
 int pair_gemm_stage_bytes(bool nvfp4, int tok_tile);
-int pair_gemm_stages(int stage_bytes);
+// one_tile: no pair has a second tile, so the ring may take the epilogue's transposition space too.
+int pair_gemm_stages(int stage_bytes, bool one_tile);
 // max_clusters[s], s = 1..kPairGemmMaxSplits: clusters of 2 s CTAs resident at once.
 cudaError_t pair_gemm_prepare(int* max_clusters);
 // `workers` clusters of `p.splits` pairs.

@@ -506,7 +506,9 @@ PairGemmParams pair_params(Context& ctx, const PairPlan& plan, int rows, int out
   q.row_units = row_units;
   q.splits = plan.splits;
   q.stage_bytes = pair_gemm_stage_bytes(nvfp4, plan.tok_tile);
-  q.stages = pair_gemm_stages(q.stage_bytes);
+  // FP8 with one tile per pair has the transposition space for a stage more (5120 x 17408, 301 tokens 30.9 -> 30.3 us,
+  // 12288 x 5120, 256 tokens 20.1 -> 19.9); NVFP4 was slower with it (down, 100 tokens 15.1 -> 15.4).
+  q.stages = pair_gemm_stages(q.stage_bytes, !nvfp4 && plan.tiles_m * row_units <= plan.workers);
   q.chunks_per_tile = k / 64;
   q.vector_out = aligned(out, 16) ? 1 : 0;
   q.status = ctx.status_word();
