@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 import torch
 
-from gpu_util import assert_inactive_untouched, dev, host, max_relative_error, sentinel_plane
+from gpu_util import assert_inactive_untouched, dev, graph_replay, host, max_relative_error, sentinel_plane
 
 pytestmark = pytest.mark.gpu
 
@@ -256,6 +256,55 @@ def test_nvfp4_down_route_rules(tk, oracle, hidden, inter, rows, kernel):
     for plane in (out, part):
         assert_inactive_untouched(plane, rows)
     assert c.device_status() == 0
+
+
+@pytest.mark.parametrize("rows,inter,split", [
+    (1000, 6208, True),    # 80 tiles: a round of whole ones, 14 left over; a last stage of one step
+    (1930, 4160, True),    # 160 tiles: two rounds, then split ones on the other accumulator's turn
+    (1000, 3840, False),   # fewer than eight stages a split
+    (700, 6208, False),    # 60 tiles in one round
+])
+def test_nvfp4_down_whole_tiles_then_split_ones(tk, oracle, monkeypatch, rows, inter, split):
+    """Tiles left over by the rounds of whole tiles are split over the pairs of a cluster.  Against the unsplit
+    plan: K / 64 accumulations on either side, each within 2^-23 of a partial sum, and partial sums within twice the
+    largest result."""
+    from tuiskollm_b200 import synth
+
+    hidden = 5120
+    xb = synth.normal_bf16(67, rows, (rows, inter))
+    dn, dns, dnd = synth.torch_nvfp4_weights(67, 2, hidden, inter, "cuda")
+    div = float(np.float32(448.0 * 6.0 / 8.0))
+    codes, scales = _nvfp4_planes(tk, rows, inter)
+    kw = dict(activation_codes=codes, activation_scales=scales, input_global_divisor=div)
+    got = []
+    for forced in (0, 1):
+        monkeypatch.setenv("TK100_PAIR_SPLITS", str(forced))
+        c = tk.Context(device=0, hidden=hidden, intermediate=inter)
+        out = sentinel_plane((rows + 1, hidden), torch.int16)
+        part = sentinel_plane((rows + 1, hidden), torch.float32)
+        down = tk.Nvfp4DownOp(c)
+        down.launch(None, rows, dev(xb.view(np.int16)), dn, dns, float(dnd), out, **kw)
+        assert c.last_kernel.startswith("pair_gemm_kernel"), c.last_kernel
+        assert ("splits=1" in c.last_kernel) == (forced == 1 or not split), c.last_kernel
+        down.launch_partial(None, rows, None, dn, dns, float(dnd), part, **kw)
+        torch.cuda.synchronize()
+        first = out.clone()
+        replay = graph_replay(lambda: down.launch(None, rows, None, dn, dns, float(dnd), out, **kw))
+        replay.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, first)
+        assert_inactive_untouched(out, rows)
+        assert_inactive_untouched(part, rows)
+        assert c.device_status() == 0
+        assert np.array_equal(oracle.f32_to_bf16(host(part)[:rows]), _u16(out)[:rows])
+        got.append(host(part)[:rows].astype(np.float64))
+    bound = 2 * 2 * (inter / 64) * 2.0 ** -23 * np.abs(got[1]).max()
+    assert np.abs(got[0] - got[1]).max() <= bound
+    oc, osc = oracle.nvfp4_quantize(xb, div)
+    tile = 128 * (inter // 16)  # scales of the last 128 weight rows
+    exp = oracle.nvfp4_w4a4_dot(oc, osc, div, host(dn)[-128:], host(dns).reshape(-1)[-tile:], float(dnd))
+    floor = 4 * float(np.abs(exp).mean())
+    assert (np.abs(got[0][:, -128:] - exp) / np.maximum(np.abs(exp), floor)).max() <= 2e-3
 
 
 def test_launches_on_two_streams_of_one_context_are_independent(tk):

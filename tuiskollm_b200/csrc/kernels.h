@@ -317,6 +317,7 @@ struct PairGemmParams {
   int tiles_m;          // token tiles
   int row_units;        // pair tiles along the weights: 256 rows, or 128 outputs with SwiGLU
   int splits;           // pairs per cluster that split K (1: persistent over the tiles)
+  int rounds;           // with splits: whole tiles of every pair in front of the cluster's split one (NVFP4 projection)
   int stages, stage_bytes;
   int chunks_per_tile;  // NVFP4: 512-byte scale chunks per 128-row tile (k / 64)
   int vector_out;       // `out` is 16-byte aligned

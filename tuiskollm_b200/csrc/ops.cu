@@ -402,6 +402,7 @@ constexpr int kPairMinRows = 33;
 
 struct PairPlan {
   int tok_tile = 0, tiles_m = 0, splits = 1, workers = 0;
+  int rounds = 0;        // with splits: whole tiles of every pair in front of the split ones
   double cycles = 1e30;  // estimate; only compared with other plans
 };
 
@@ -429,15 +430,24 @@ PairPlan plan_pairs(const Context& ctx, int rows, int row_units, int nkb, bool n
     for (int s = 1; s <= kPairGemmMaxSplits; ++s) {
       if (forced && tune.pair_splits > 0 && s != tune.pair_splits) continue;
       const int clusters = ctx.pair_clusters(s);
-      if (clusters <= 0 || (s > 1 && (!may_split || nkb / s < 8 || tiles > clusters))) continue;
-      const long long waves = s > 1 ? 1 : (tiles + clusters - 1) / clusters;
-      const double body = static_cast<double>(waves) * ((nkb + s - 1) / s) * stage;
+      if (clusters <= 0 || (s > 1 && (!may_split || nkb / s < 8))) continue;
+      // Rounds of whole tiles on all pairs, then at most one tile a cluster, its K split.  Both in one launch for
+      // NVFP4 only, whose stage costs nearly the same at 128 tokens as at 256, so that no narrower tile fills the
+      // last round: down, two rounds -> one and a third, 800 tokens 48.6 -> 39.6 us, 1024 49.2 -> 40.1; three
+      // -> two and a half, 2048 tokens 73.4 -> 68.1.  FP8 takes narrower tiles instead (5120 x 6144, 1024
+      // tokens 31 us, split behind whole tiles 36; 5120 x 17408 70 and 69).
+      const long long pairs = static_cast<long long>(s) * clusters;
+      const long long rounds = s > 1 ? tiles / pairs : (tiles + pairs - 1) / pairs;
+      const long long left = s > 1 ? tiles - rounds * pairs : 0;
+      if (s > 1 && (left == 0 || left > clusters || (rounds > 0 && !nvfp4))) continue;
+      const double body = static_cast<double>(rounds * nkb + (left > 0 ? (nkb + s - 1) / s : 0)) * stage;
       const double cycles = std::max(body, weight_bytes / 3900.0) + 4.0 * tok + (s > 1 ? 1500.0 : 0.0);
       if (cycles < best.cycles) {
         best.tok_tile = tok;
         best.tiles_m = tiles_m;
         best.splits = s;
         best.workers = static_cast<int>(std::min<long long>(tiles, clusters));
+        best.rounds = static_cast<int>(s > 1 ? rounds : 0);
         best.cycles = cycles;
       }
     }
@@ -491,7 +501,7 @@ bool better_on_single_pair_tiles(const PairPlan& plan, int rows, int out_rows, i
 // 512 x 3072, 80 tokens 6.5 / 5.6.
 bool better_on_split_tiles(const PairPlan& plan, int rows, int out_rows, int k) {
   if (out_rows <= 1024) return rows <= 80 && k >= 2176;
-  return rows <= 64 && plan.splits >= 3;
+  return rows <= 64 && plan.splits >= 3 && plan.rounds == 0;
 }
 
 PairGemmParams pair_params(Context& ctx, const PairPlan& plan, int rows, int out_rows, int k, int row_units, bool nvfp4,
@@ -505,6 +515,7 @@ PairGemmParams pair_params(Context& ctx, const PairPlan& plan, int rows, int out
   q.tiles_m = plan.tiles_m;
   q.row_units = row_units;
   q.splits = plan.splits;
+  q.rounds = plan.rounds;
   q.stage_bytes = pair_gemm_stage_bytes(nvfp4, plan.tok_tile);
   // FP8 with one tile per pair has the transposition space for a stage more (5120 x 17408, 301 tokens 30.9 -> 30.3 us,
   // 12288 x 5120, 256 tokens 20.1 -> 19.9); NVFP4 was slower with it (down, 100 tokens 15.1 -> 15.4).

@@ -24,10 +24,10 @@
 // need anyway (stmatrix.trans; with 2-byte shared stores and a scale load per value the epilogue of a
 // 256-token tile took 6.1 us instead of ~2).
 //
-// Few tiles (T tiles on P pairs, T <= P / 2): the S pairs of a cluster split K; each CTA parks the
-// token batches other splits finish in its own ring, one cluster barrier, and every split adds its
-// batches over distributed shared memory in split order (fixed, so bit-reproducible).  No global
-// scratch, so launches on several streams of one context stay independent.
+// Few tiles (T tiles on P pairs, T <= P / 2), or with NVFP4 few left over by rounds of whole tiles: the S pairs
+// of a cluster split K of one; each CTA parks the token batches other splits finish in its own ring, one cluster
+// barrier, and every split adds its batches over distributed shared memory in split order (fixed, so
+// bit-reproducible).  No global scratch, so launches on several streams of one context stay independent.
 //
 // No load is shared through multicast: every CTA fetches its own operands.
 #include <type_traits>
@@ -110,6 +110,23 @@ __global__ void __launch_bounds__(block_threads(NV, SWIGLU), 1)
   const int tiles = p.tiles_m * p.row_units;
   const int k0 = static_cast<int>(static_cast<long long>(split) * p.nkb / splits);
   const int k1 = static_cast<int>(static_cast<long long>(split + 1) * p.nkb / splits);
+  // NVFP4 projections: behind `rounds` rounds of whole tiles on all pairs the cluster's pairs split K of one more.
+  constexpr bool TAILS = NV && !SWIGLU;
+  const int rounds = TAILS ? p.rounds : 0;
+  const int whole = rounds * workers * splits;
+  // The n-th tile of this pair: index and blocks of K.
+  auto tile_at = [&](int n, int& t, int& first_kb, int& last_kb) {
+    first_kb = k0;
+    last_kb = k1;
+    if (TAILS && n < rounds) {
+      t = static_cast<int>(blockIdx.x >> 1) + n * workers * splits;
+      first_kb = 0;
+      last_kb = p.nkb;
+      return true;
+    }
+    t = TAILS && splits > 1 ? whole + worker : worker + n * workers;
+    return t < tiles && (!TAILS || splits == 1 || n == rounds);
+  };
   const int stages = p.stages;
   const uint32_t stage_bytes = static_cast<uint32_t>(p.stage_bytes);
   const uint32_t off_b = kWTile;
@@ -191,28 +208,27 @@ __global__ void __launch_bounds__(block_threads(NV, SWIGLU), 1)
         }
       };
       bool ok = true, first = true;
-      int s = 0;
+      int s = 0, t = 0, kb = 0, kb_end = 0;
       uint32_t phase = 0;
-      for (int t = worker; t < tiles && ok; t += workers) {
+      for (int n = 0; ok && tile_at(n, t, kb, kb_end); ++n) {
         const int unit = t / p.tiles_m;
         const int tok0 = (t - unit * p.tiles_m) * tok_tile;
-        int kb = k0;
         if (first) {
           // First pass over the ring: the weights do not depend on the predecessor kernel and are
           // requested before pdl_wait(), the tokens of the same stages follow it.
-          const int pre = min(stages, k1 - k0);
+          const int pre = min(stages, kb_end - kb);
           for (int i = 0; i < pre; ++i) {
             if (rank == 0) mbar_arrive_expect_tx(&ctl->full[i], bytes);
-            load_w(i, k0 + i, unit);
+            load_w(i, kb + i, unit);
           }
           pdl_wait();
-          for (int i = 0; i < pre; ++i) load_b(i, k0 + i, tok0);
+          for (int i = 0; i < pre; ++i) load_b(i, kb + i, tok0);
           first = false;
           kb += pre;
           s = pre == stages ? 0 : pre;
           phase = pre == stages ? 1u : 0u;
         }
-        for (; kb < k1; ++kb) {
+        for (; kb < kb_end; ++kb) {
           ok = mbar_wait(&ctl->empty[s], phase ^ 1u, p.status);
           if (!ok) break;
           if (rank == 0) mbar_arrive_expect_tx(&ctl->full[s], bytes);
@@ -242,9 +258,9 @@ __global__ void __launch_bounds__(block_threads(NV, SWIGLU), 1)
       const uint64_t desc_sfb0 = umma_desc_noswizzle_rows16(base0 + off_sfb);
       const uint32_t stage_step = stage_bytes >> 4;
       bool ok = true;
-      int s = 0, n = 0;
+      int s = 0, t = 0, kb0 = 0, kb_end = 0;
       uint32_t phase = 0, sf_parity = 0;
-      for (int t = worker; t < tiles && ok; t += workers, ++n) {
+      for (int n = 0; ok && tile_at(n, t, kb0, kb_end); ++n) {
         const int b = n & 1;
         // the columns this tile accumulates into have been read: overlapping accumulators wait for
         // the shared columns of the tile before, disjoint ones for the tile two before
@@ -255,7 +271,7 @@ __global__ void __launch_bounds__(block_threads(NV, SWIGLU), 1)
           tc_fence_after_sync();
         }
         const uint32_t acc = tmem + static_cast<uint32_t>(b) * acc_stride;
-        for (int kb = k0; kb < k1; ++kb) {
+        for (int kb = kb0; kb < kb_end; ++kb) {
           ok = mbar_wait(&ctl->full[s], phase, p.status);
           if (!ok) break;
           tc_fence_after_sync();
@@ -274,13 +290,13 @@ __global__ void __launch_bounds__(block_threads(NV, SWIGLU), 1)
                 tmem_cp_32x128b_warpx4_pair(slot + 4, desc_sfb + k4 * 32);
                 if (tok_tile > kRows) tmem_cp_32x128b_warpx4_pair(slot + 8, desc_sfb + 128 + k4 * 32);
                 umma_nvfp4_pair(acc, desc_w + 2 * k4, desc_b + 2 * k4, idesc, slot, slot + 4,
-                                (kb > k0 || k4 > 0) ? 1u : 0u);
+                                (kb > kb0 || k4 > 0) ? 1u : 0u);
               }
             }
           } else {
 #pragma unroll
             for (int k4 = 0; k4 < 4; ++k4) {
-              umma_f8f6f4_pair(acc, desc_w + 2 * k4, desc_b + 2 * k4, idesc, (kb > k0 || k4 > 0) ? 1u : 0u);
+              umma_f8f6f4_pair(acc, desc_w + 2 * k4, desc_b + 2 * k4, idesc, (kb > kb0 || k4 > 0) ? 1u : 0u);
             }
           }
           umma_commit_pair(&ctl->empty[s], both);
@@ -439,8 +455,8 @@ __global__ void __launch_bounds__(block_threads(NV, SWIGLU), 1)
     // parked batches: [batch][quadrant][four 16-byte pieces of both fragments][lane]
     const uint32_t parked = smem_u32(smem) + static_cast<uint32_t>(quad * 4096 + lane * 16);
     constexpr uint32_t kParkedBatch = 16384;
-    int n = 0;
-    for (int t = worker; t < tiles; t += workers, ++n) {
+    int t = 0, kb0 = 0, kb_end = 0;
+    for (int n = 0; tile_at(n, t, kb0, kb_end); ++n) {
       const int unit = t / p.tiles_m;
       const int tok0 = (t - unit * p.tiles_m) * tok_tile;
       const int b = n & 1;
@@ -451,11 +467,12 @@ __global__ void __launch_bounds__(block_threads(NV, SWIGLU), 1)
       float ws[4];
       float2 as[4];
       row_scales(unit, ws);
-      if (splits == 1) token_scales(tok0 + batch_of(part) * kBatch, as);
+      const bool shared = !SWIGLU && splits > 1 && n == rounds;  // the tile whose K the cluster's pairs split
+      if (!shared) token_scales(tok0 + batch_of(part) * kBatch, as);
       if (!mbar_wait(&ctl->acc_full[b], (n >> 1) & 1, p.status)) break;
       tc_fence_after_sync();
       const uint32_t taddr = tmem + (static_cast<uint32_t>(quad * 32) << 16) + static_cast<uint32_t>(b) * acc_stride;
-      if (!SWIGLU && splits > 1) {
+      if (shared) {
         // park the batches other splits finish over the ring, whose loads and reads are all done
         for (int o = part; o < batches; o += PARTS) {
           if (o % splits == split || tok0 + o * kBatch >= p.rows) continue;
@@ -469,7 +486,7 @@ __global__ void __launch_bounds__(block_threads(NV, SWIGLU), 1)
             sts128(parked + o * kParkedBatch + j * 512, make_uint4(v[0], v[1], v[2], v[3]));
           }
         }
-        break;  // one tile per cluster; finished behind the cluster barrier below
+        break;  // the cluster's last tile; finished behind the barrier below
       }
       const int due = overlap ? overlap_batches : batches;  // columns the next tile waits for
       if (part >= due) {
@@ -499,12 +516,14 @@ __global__ void __launch_bounds__(block_threads(NV, SWIGLU), 1)
     if (!SWIGLU && splits > 1) {
       cluster_arrive();
       cluster_wait();
-      if (worker < tiles) {
-        const int unit = worker / p.tiles_m;
-        const int tok0 = (worker - unit * p.tiles_m) * tok_tile;
+      t = whole + worker;
+      if (t < tiles) {
+        const int unit = t / p.tiles_m;
+        const int tok0 = (t - unit * p.tiles_m) * tok_tile;
         float ws[4];
         row_scales(unit, ws);
-        const uint32_t taddr = tmem + (static_cast<uint32_t>(quad * 32) << 16);
+        const uint32_t taddr =
+            tmem + (static_cast<uint32_t>(quad * 32) << 16) + static_cast<uint32_t>(rounds & 1) * acc_stride;
         // This split's batches are split, split + splits, ...; the quadrant's warps alternate.  All that the S - 1
         // other splits parked of a batch is requested before the first sum (instead of one split after the other;
         // three splits, 256 tokens: NVFP4 down 18.4 -> 18.0 us, FP8 5120 x 6144 16.1 -> 15.8).  The sums run in split
