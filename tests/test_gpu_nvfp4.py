@@ -684,3 +684,50 @@ def test_wide_tile_route_matches_plain_route_bit_for_bit(tk, rows, monkeypatch):
         got[route] = (_u16(mid)[:rows].copy(), _u16(out)[:rows].copy())
     assert np.array_equal(got["wide"][0], got["plain"][0]), "gate/up + SwiGLU"
     assert np.array_equal(got["wide"][1], got["plain"][1]), "down"
+
+
+@pytest.mark.parametrize("rows", [1, 2, 3, 4, 5, 8, 9, 13, 16, 17, 29, 32])
+@pytest.mark.parametrize("divisor", [448.0 * 6.0 / 8.0, 2.0 ** -24])
+def test_gate_up_quarters_of_the_tokens(tk, oracle, monkeypatch, rows, divisor):
+    """Up to 32 tokens the four warps that hold a row of the gate and the up tile finish a quarter of the tokens each,
+    in groups of 1, 2, 4 or 8: every count, the quantised form bit for bit that of the rounded outputs (a small divisor
+    leaves every scale 0 and every code a signed zero), and the bits of the exchange that pushes halves."""
+    from tuiskollm_b200 import synth
+
+    hidden, inter = 512, 384
+    xb = synth.normal_bf16(71, rows, (rows, hidden))
+    if rows > 2:
+        xb[rows // 2] = 0  # a token whose outputs are zeros
+    gu, gus, gud = synth.nvfp4_weights(71, 1, 2 * inter, hidden)
+    a_div, m_div = float(np.float32(448.0)), float(np.float32(divisor))
+    got = []
+    for mode in ("3", "2"):
+        monkeypatch.setenv("TK100_CLUSTER", mode)
+        c = tk.Context(device=0, hidden=hidden, intermediate=inter)
+        codes = torch.zeros((rows, hidden // 2), dtype=torch.uint8, device="cuda")
+        scales = torch.zeros((tk.ops.nvfp4_scale_plane_bytes(rows, hidden),), dtype=torch.uint8, device="cuda")
+        m_codes = sentinel_plane((rows + 1, inter // 2), torch.uint8)
+        m_scales = torch.zeros((tk.ops.nvfp4_scale_plane_bytes(rows, inter),), dtype=torch.uint8, device="cuda")
+        mid = sentinel_plane((rows + 1, inter), torch.int16)
+        tk.Nvfp4SwiGluOp(c).launch_quantize(None, rows, dev(xb.view(np.int16)), dev(gu), dev(gus), float(gud), mid,
+                                            activation_codes=codes, activation_scales=scales,
+                                            input_global_divisor=a_div, output_global_divisor=m_div,
+                                            output_codes=m_codes, output_scales=m_scales)
+        torch.cuda.synchronize()
+        assert c.last_kernel.startswith("nvfp4_gemm_kernel<32") or mode == "2", c.last_kernel
+        assert c.device_status() == 0
+        assert_inactive_untouched(mid, rows)
+        assert_inactive_untouched(m_codes, rows)
+        got.append((mid, m_codes, m_scales))
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+    oc, osc = oracle.nvfp4_quantize(xb, a_div)
+    dots = oracle.nvfp4_w4a4_dot(oc, osc, a_div, gu, gus, float(gud))
+    exp = oracle.silu_mul(dots[:, :inter], dots[:, inter:])
+    out = host(got[0][0].view(torch.int16)).view(np.uint16)[:rows]
+    assert max_relative_error(out, exp, 4 * float(np.abs(exp).mean())) <= 1e-2
+    mc, msc = oracle.nvfp4_quantize(out, m_div)
+    assert np.array_equal(host(got[0][1])[:rows], mc)
+    assert np.array_equal(host(got[0][2]), msc)
+    if divisor < 1e-3:
+        assert not msc.any() and mc.any()

@@ -1408,7 +1408,7 @@ Status Nvfp4MlpOp::launch(cudaStream_t stream, bool gate_up, int rows, int out_r
   // Decode shapes quantise in the epilogue of the CTA that finishes the tokens (saves a launch:
   // M = 1 23.2 -> 22.1 us); from 128-token tiles on that epilogue work is not hidden and the
   // quantiser kernel after the projection is faster (M = 2048: 351 against 419 us).
-  const bool in_epilogue = next && as_pairs && block_tok == 32;
+  const bool in_epilogue = next && as_pairs && block_tok == 32 && p.cluster != 2;
   if (in_epilogue) {
     p.q_codes = next->codes;
     p.q_scales = next->scales;
