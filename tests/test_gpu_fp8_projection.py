@@ -267,6 +267,31 @@ def test_split_k_reduction_routes_agree_bit_for_bit(tk, oracle, rows, monkeypatc
     assert max_relative_error(outs["2"][:, sample], exp, 0.25) <= 1e-2
 
 
+@pytest.mark.parametrize("splits", [2, 3, 4, 5])
+@pytest.mark.parametrize("rows", [1, 7, 9, 16, 17, 32])
+def test_tokens_of_a_split_tile_in_groups_of_four_and_two(tk, rows, splits, monkeypatch):
+    """Up to four splits with more than four tokens each are finished four at a time, others two: the same bits as the tiles that meet in
+    global scratch, for every remainder of a group and an output row count that ends inside a tile."""
+    from tuiskollm_b200 import synth
+
+    hidden, out_rows = 1280, 400
+    w, s = synth.torch_fp8_weights(47, splits, out_rows, hidden, "cuda")
+    x = synth.torch_normal_bf16(47, rows, (rows, hidden), "cuda")
+    outs = []
+    monkeypatch.setenv("TK100_SPLITS", str(splits))
+    for mode in ("3", "0"):
+        monkeypatch.setenv("TK100_CLUSTER", mode)
+        c = tk.Context(device=0)
+        planes = Planes(rows + 1, hidden, out_rows)
+        tk.Fp8ProjectionOp(c).launch(None, rows, out_rows, hidden, x, planes.codes, planes.scales, w, s, planes.out)
+        torch.cuda.synchronize()
+        assert f"splits={splits}" in c.last_kernel and ("cluster" in c.last_kernel) == (mode == "3"), c.last_kernel
+        planes.check_inactive(rows)
+        assert c.device_status() == 0
+        outs.append(_u16(planes.out)[:rows].copy())
+    assert np.array_equal(outs[0], outs[1])
+
+
 def test_fused_producer_feeds_projection(tk, ctx, oracle):
     """Decode slice of the first benchmark configuration: residual add + RMSNorm + quantise in
     one kernel, then the QKV projection reads the codes it wrote (input == NULL)."""

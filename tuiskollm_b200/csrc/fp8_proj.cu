@@ -172,7 +172,8 @@ __device__ __forceinline__ void exchange_and_merge(int tid, int nthreads, int ro
   }
 }
 
-template <int BLOCK_TOK, int DEEP>  // DEEP: 0 normal ring, 1 deep, 2 wide
+// DEEP: 0 normal ring, 1 deep, 2 wide.  FEW: at most four splits meet in a cluster.
+template <int BLOCK_TOK, int DEEP, bool FEW = false>
 __global__ void __launch_bounds__(kThreads, BLOCK_TOK <= 32 ? (DEEP == 1 ? 2 : (DEEP == 2 ? 4 : 3))
                                                             : (BLOCK_TOK <= 128 ? 2 : 1))
     fp8_projection_kernel(const __grid_constant__ CUtensorMap tmap_w,
@@ -688,25 +689,28 @@ __global__ void __launch_bounds__(kThreads, BLOCK_TOK <= 32 ? (DEEP == 1 ? 2 : (
       if (!TK100_DBG(p, DBG_NO_EPILOGUE)) {
         const uint32_t rank = cluster_cta_rank();
         const uint32_t my_addr = smem_u32(reinterpret_cast<float*>(smem) + row_in_tile);
+        // Sixteen loads in flight per round trip over distributed shared memory: FEW takes four tokens at a time, else
+        // two (fp8_few_splits).
+        constexpr int TOKENS = FEW ? 4 : 2, SPLITS = FEW ? 4 : kMaxSplits;
 #pragma unroll 1
-        for (int j0 = static_cast<int>(rank); j0 < valid_tok; j0 += 2 * p.splits) {
-          float v[2][kMaxSplits];
+        for (int j0 = static_cast<int>(rank); j0 < valid_tok; j0 += TOKENS * p.splits) {
+          float v[TOKENS][SPLITS];
 #pragma unroll
-          for (int u = 0; u < 2; ++u) {
+          for (int u = 0; u < TOKENS; ++u) {
             const int j = j0 + u * p.splits;
 #pragma unroll
-            for (int s = 0; s < kMaxSplits; ++s) {
+            for (int s = 0; s < SPLITS; ++s) {
               v[u][s] = (j < valid_tok && s < p.splits)
                             ? ld_dsmem_f32(my_addr + j * kTileRows * 4, static_cast<uint32_t>(s))
                             : 0.0f;
             }
           }
 #pragma unroll
-          for (int u = 0; u < 2; ++u) {
+          for (int u = 0; u < TOKENS; ++u) {
             const int j = j0 + u * p.splits;
             float acc = 0.0f;
 #pragma unroll
-            for (int s = 0; s < kMaxSplits; ++s) {
+            for (int s = 0; s < SPLITS; ++s) {
               if (s < p.splits) acc = __fadd_rn(acc, v[u][s]);
             }
             if (j < valid_tok) emit(j, acc);
@@ -872,6 +876,14 @@ __global__ void __launch_bounds__(256)
   exchange_and_merge(threadIdx.x, blockDim.x, rows, world, rank, keys, peers, s_step, out, status);
 }
 
+// Up to four splits and more than four tokens for each to finish: four tokens a round trip instead of two.  Behind a
+// norm, 16384 rows (three splits) 16 / 32 tokens 18.1 / 20.6 -> 17.8 / 19.6 us, 12288 (four) 32 tokens 16.3 -> 15.7.
+// An instantiation of its own, and not with fewer tokens: both loops in one kernel cost launches of six and eight
+// splits 0.2 us, and a layer of few tokens that runs both kernels 0.4 (GDN layer, one token 32.9 -> 33.3).
+bool fp8_few_splits(const Fp8ProjParams& p) {
+  return p.cluster == 1 && p.splits > 1 && p.splits <= 4 && p.rows > 4 * p.splits;
+}
+
 template <int BLOCK_TOK>
 cudaError_t launch_one(cudaStream_t stream, const CUtensorMap& tmap_w, const CUtensorMap& tmap_a,
                        const Fp8ProjParams& p) {
@@ -888,6 +900,11 @@ cudaError_t launch_one(cudaStream_t stream, const CUtensorMap& tmap_w, const CUt
     return launch_kernel_cluster(fp8_projection_kernel<BT, 2>, grid, dim3(kThreads),
                                  smem_bytes_for<BT, 2>(), stream, dim3(1, 1, cluster_z), tmap_w, tmap_a, p);
   }
+  if (BLOCK_TOK <= 32 && fp8_few_splits(p)) {
+    constexpr int BT = BLOCK_TOK <= 32 ? BLOCK_TOK : 32;
+    return launch_kernel_cluster(fp8_projection_kernel<BT, 0, true>, grid, dim3(kThreads), smem_bytes_for<BT, 0>(),
+                                 stream, dim3(1, 1, cluster_z), tmap_w, tmap_a, p);
+  }
   return launch_kernel_cluster(fp8_projection_kernel<BLOCK_TOK, 0>, grid, dim3(kThreads),
                                smem_bytes_for<BLOCK_TOK, 0>(), stream, dim3(1, 1, cluster_z), tmap_w, tmap_a,
                                p);
@@ -899,6 +916,10 @@ cudaError_t prepare_one() {
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(smem_bytes_for<BLOCK_TOK, 0>()));
   if (e != cudaSuccess || BLOCK_TOK > 32) return e;
+  constexpr int BF = BLOCK_TOK <= 32 ? BLOCK_TOK : 32;
+  e = cudaFuncSetAttribute(fp8_projection_kernel<BF, 0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           static_cast<int>(smem_bytes_for<BF, 0>()));
+  if (e != cudaSuccess) return e;
   e = cudaFuncSetAttribute(fp8_projection_kernel<BLOCK_TOK, 1>,
                            cudaFuncAttributeMaxDynamicSharedMemorySize,
                            static_cast<int>(smem_bytes_for<BLOCK_TOK, 1>()));
