@@ -230,3 +230,30 @@ def test_benchmarked_fp8_down_and_gdn_output_sampled_rows(tk, ctx, oracle, rows)
         assert max_relative_error(got, exp, 4 * float(np.abs(exp).mean())) <= 1e-2, route
         planes.check_inactive(rows)
     assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("rows", [1, 2, 3, 4, 5, 8, 9, 15, 16, 17, 24, 31, 32])
+def test_fp8_swiglu_halves_of_the_tokens(tk, oracle, rows):
+    """Up to 32 tokens the two warps that hold a row finish half of the tokens each, in groups of 1, 2, 4 or 8: every
+    count, a token's outputs bit for bit those of a launch of its own, and against the f64 oracle."""
+    from tuiskollm_b200 import synth
+
+    hidden, inter = 640, 256
+    c = tk.Context(device=0, hidden=hidden, intermediate=inter)
+    xb = synth.normal_bf16(53, rows, (rows, hidden))
+    gu_c, gu_s = synth.fp8_weights(53, 1, 2 * inter, hidden)
+    w, s = dev(gu_c), dev(gu_s.view(np.int16))
+    op, p = tk.Fp8SwiGluOp(c), Planes(rows + 1, hidden, inter)
+    op.launch(None, rows, dev(xb.view(np.int16)), p.codes, p.scales, w, s, p.out)
+    assert c.last_kernel.startswith("fp8_swiglu_kernel"), c.last_kernel
+    one = Planes(2, hidden, inter)
+    for t in range(rows):
+        op.launch(None, 1, dev(xb[t:t + 1].view(np.int16)), one.codes, one.scales, w, s, one.out)
+        torch.cuda.synchronize()
+        assert torch.equal(one.out[0], p.out[t]), t
+    p.check_inactive(rows)
+    oc, os_ = oracle.quantize_e4m3(xb)
+    proj = oracle.fp8_projection(oc, os_, gu_c, gu_s)
+    exp = oracle.silu_mul(proj[:, :inter], proj[:, inter:])
+    assert max_relative_error(_u16(p.out)[:rows], exp, 4 * float(np.abs(exp).mean())) <= 1e-2
+    assert c.device_status() == 0
