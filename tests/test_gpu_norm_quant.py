@@ -368,3 +368,45 @@ def test_norm_on_both_sides_of_a_wave(tk, oracle, hidden, ctas):
         assert np.array_equal(host(codes)[:rows], oc) and np.array_equal(host(scales)[:rows], os_)
         for plane in (residual, normed, codes, scales):
             assert_inactive_untouched(plane, rows)
+
+
+@pytest.mark.parametrize("hidden", [5120, 17408])
+@pytest.mark.parametrize("with_branch", [True, False])
+def test_rows_that_get_an_sm_each_or_share_it_in_twos(tk, hidden, with_branch):
+    """Shared memory asked for to spread the rows over the SMs changes nothing but their place: every plane has the
+    bits of launches of four rows, which do not ask for it, on both sides of each line, and nothing behind them."""
+    from tuiskollm_b200 import ops, synth
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    c = tk.Context(device=0, hidden=hidden)
+    most = 2 * sms + 4
+    x, branch = (synth.torch_normal_bf16(95, i, (most, hidden), "cuda") for i in (1, 2))
+    weight = synth.torch_normal_bf16(95, 3, (hidden,), "cuda", std=0.1)
+    op = tk.ResidualNormOp(c)
+
+    def planes(rows):
+        return ([sentinel_plane((rows + 1, hidden), torch.int16) for _ in range(2)] +
+                [sentinel_plane((rows + 1, hidden), torch.uint8), sentinel_plane((rows + 1,), torch.float32),
+                 sentinel_plane((rows + 1, hidden // 2), torch.uint8),
+                 torch.zeros((ops.nvfp4_scale_plane_bytes(rows, hidden),), dtype=torch.uint8, device="cuda")])
+
+    def launch(rows, first, out):
+        op.launch_quantize_nvfp4(None, rows, x[first:first + rows], branch[first:first + rows] if with_branch else None,
+                                 weight, out[0], out[1], out[2], out[3], 448.0, out[4], out[5])
+
+    want = planes(most)
+    for first in range(0, most, 4):
+        four = planes(4)
+        launch(4, first, four)
+        for w, f in zip(want[:5], four[:5]):
+            w[first:first + 4] = f[:4]
+    for rows in (4, 5, sms, sms + 1, 3 * sms // 2, 3 * sms // 2 + 1, 2 * sms, 2 * sms + 1):
+        got = planes(rows)
+        launch(rows, 0, got)
+        torch.cuda.synchronize()
+        for i, (w, g) in enumerate(zip(want[:5], got[:5])):
+            if i == 0 and not with_branch:
+                continue  # no residual plane is written
+            assert torch.equal(w[:rows].view(torch.uint8), g[:rows].view(torch.uint8)), (rows, i)
+            assert_inactive_untouched(g, rows)
+    assert c.device_status() == 0

@@ -216,14 +216,22 @@ __global__ void __launch_bounds__(CHUNKS == 3 ? 704 : 1024)  // norm_geometry: t
   }
 }
 
+// Shared memory that a norm asks for and does not use, so that its rows get an SM each (from one and a half rows per SM:
+// two share one).  Left alone, the CTAs pile up three to an SM where the kernel in front frees one first, and CTAs of the
+// projection behind join them, whose weight tiles then fill the SM's way to L2 in front of the rows.
+// Without / with it, us: the norm itself (E4M3) 16 rows 2.16 / 2.01, 48 3.47 / 2.59, 100 4.10 / 2.93; with a projection
+// behind it, 16 rows 8192 x 5120 10.8 / 10.4, 16384 x 5120 17.8 / 16.9, 5120 x 6144 10.2 / 9.0, 32 rows 12.9 / 12.4,
+// 19.5 / 18.5, 11.6 / 10.6; equal up to four rows.  Two an SM: 256 rows 4.67 / 4.29, 296 4.83 / 4.40, but 200 3.97 / 4.09.
+constexpr int kOneAnSm = 160 * 1024, kTwoAnSm = 100 * 1024;
+
 template <bool HAS_BRANCH, bool DO_NORM, bool DO_QUANT>
 cudaError_t launch_chunks(cudaStream_t stream, int rows, int hidden, int threads, int chunks,
                           const uint16_t* x, const uint16_t* branch, const uint16_t* weight,
                           uint16_t* residual_out, uint16_t* normalized_out, uint8_t* codes,
-                          float* scales, float eps, uint32_t* status, const Nvfp4Out& nv) {
+                          float* scales, float eps, uint32_t* status, const Nvfp4Out& nv, int spread_bytes) {
 #define TK100_LAUNCH(C)                                                                       \
   launch_kernel(resnorm_quant_kernel<HAS_BRANCH, DO_NORM, DO_QUANT, C>, dim3(rows), dim3(threads), \
-                0, stream, x, branch, weight, residual_out, normalized_out, codes, scales, hidden, \
+                spread_bytes, stream, x, branch, weight, residual_out, normalized_out, codes, scales, hidden, \
                 eps, status, nv)
   switch (chunks) {
     case 1: return TK100_LAUNCH(1);
@@ -258,6 +266,22 @@ bool pdl_enabled() { return g_pdl; }
 uint32_t debug_flags() { return g_debug; }
 
 unsigned long long* debug_stamps() { return g_stamps; }
+
+cudaError_t norm_prepare() {
+  cudaError_t e = cudaSuccess;
+  auto allow = [&](auto kernel) {
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kOneAnSm);
+  };
+  allow(resnorm_quant_kernel<true, true, true, 1>);
+  allow(resnorm_quant_kernel<true, true, true, 2>);
+  allow(resnorm_quant_kernel<true, true, true, 3>);
+  allow(resnorm_quant_kernel<true, true, true, 4>);
+  allow(resnorm_quant_kernel<false, true, true, 1>);
+  allow(resnorm_quant_kernel<false, true, true, 2>);
+  allow(resnorm_quant_kernel<false, true, true, 3>);
+  allow(resnorm_quant_kernel<false, true, true, 4>);
+  return e;
+}
 
 bool norm_geometry(int hidden, int* threads, int* chunks) {
   if (hidden <= 0 || (hidden & 7) != 0) return false;
@@ -297,15 +321,20 @@ cudaError_t launch_resnorm_quant(cudaStream_t stream, int rows, int hidden, cons
   // 5120 columns, one / two / four: 600 rows 4.1 / 4.5 / 3.6, 2048 9.4 / 10.0 / 6.8.  With the norm the chunks
   // double; 5120 columns, one / two / four: 512 rows 7.0 / 6.5 / 8.7, 800 9.2 / 9.5 / 10.5, 1024 rows and
   // more equal; 10240 columns, two / four: 600 rows 13.9 / 15.1, 1024 21.8 / 20.5, 2048 38.9 / 36.9.
-  if (chunks <= 2) {
-    static int sms = 0;
-    if (sms == 0) {
-      int device = 0;
-      if (cudaGetDevice(&device) != cudaSuccess ||
-          cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
-        sms = 148;
-      }
+  static int sms = 0;
+  if (sms == 0) {
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
+      sms = 148;
     }
+  }
+  int spread_bytes = 0;
+  if (do_norm && do_quant) {
+    if (rows >= 5 && rows <= sms) spread_bytes = kOneAnSm;
+    else if (2 * rows > 3 * sms && rows <= 2 * sms) spread_bytes = kTwoAnSm;
+  }
+  if (chunks <= 2) {
     const int resident = !do_norm && chunks == 2 ? 1536 : 2048;  // threads of an SM
     const int wide = do_norm ? 2 * chunks : 4;
     const int narrow = (((hidden >> 3) + wide - 1) / wide + 31) & ~31;
@@ -317,7 +346,7 @@ cudaError_t launch_resnorm_quant(cudaStream_t stream, int rows, int hidden, cons
 #define TK100_CASE(B, N, Q)                                                                      \
   if (has_branch == B && do_norm == N && do_quant == Q)                                          \
   return launch_chunks<B, N, Q>(stream, rows, hidden, threads, chunks, x, branch, weight,        \
-                                residual_out, normalized_out, codes, scales, eps, status, nv)
+                                residual_out, normalized_out, codes, scales, eps, status, nv, spread_bytes)
   TK100_CASE(true, true, true);
   TK100_CASE(true, true, false);
   TK100_CASE(false, true, true);
