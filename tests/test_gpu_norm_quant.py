@@ -1,5 +1,7 @@
 """GPU parity: fused residual-add + RMSNorm + per-token E4M3 quantisation against the CPU
 oracle, following qual/src/residual_norm.rs (exact batches, sentinels, graph replay)."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -370,11 +372,18 @@ def test_norm_on_both_sides_of_a_wave(tk, oracle, hidden, ctas):
             assert_inactive_untouched(plane, rows)
 
 
-@pytest.mark.parametrize("hidden", [5120, 17408])
+def _tiled_scale_offsets(rows, hidden):
+    """Byte of each (row, block) in a scale plane: tiles of 128 rows x 4 blocks, 16 bytes per row of a tile's quarter."""
+    r = torch.arange(rows, device="cuda")[:, None]
+    g = torch.arange(hidden // 16, device="cuda")[None, :]
+    return ((r >> 7) * (hidden // 64) + (g >> 2)) * 512 + (r & 31) * 16 + ((r & 127) >> 5) * 4 + (g & 3)
+
+
+@pytest.mark.parametrize("hidden", [2048, 5120, 6144, 17408])
 @pytest.mark.parametrize("with_branch", [True, False])
-def test_rows_that_get_an_sm_each_or_share_it_in_twos(tk, hidden, with_branch):
-    """Shared memory asked for to spread the rows over the SMs changes nothing but their place: every plane has the
-    bits of launches of four rows, which do not ask for it, on both sides of each line, and nothing behind them."""
+def test_rows_in_clusters_have_the_bits_of_rows_alone(tk, hidden, with_branch):
+    """A cluster changes nothing but a row's place: every plane has the bits of launches of four rows, which have none,
+    on both sides of each line and with one to three rows in the last cluster, and nothing behind the rows."""
     from tuiskollm_b200 import ops, synth
 
     sms = torch.cuda.get_device_properties(0).multi_processor_count
@@ -394,13 +403,15 @@ def test_rows_that_get_an_sm_each_or_share_it_in_twos(tk, hidden, with_branch):
         op.launch_quantize_nvfp4(None, rows, x[first:first + rows], branch[first:first + rows] if with_branch else None,
                                  weight, out[0], out[1], out[2], out[3], 448.0, out[4], out[5])
 
+    offsets = _tiled_scale_offsets(most, hidden)
     want = planes(most)
     for first in range(0, most, 4):
         four = planes(4)
         launch(4, first, four)
         for w, f in zip(want[:5], four[:5]):
             w[first:first + 4] = f[:4]
-    for rows in (4, 5, sms, sms + 1, 3 * sms // 2, 3 * sms // 2 + 1, 2 * sms, 2 * sms + 1):
+        want[5][offsets[first:first + 4]] = four[5][offsets[:4]]
+    for rows in (4, 12, 13, 14, 15, 16, 29, 32, 33, sms, sms + 1, 3 * sms // 2 + 1, 2 * sms + 1):
         got = planes(rows)
         launch(rows, 0, got)
         torch.cuda.synchronize()
@@ -409,4 +420,40 @@ def test_rows_that_get_an_sm_each_or_share_it_in_twos(tk, hidden, with_branch):
                 continue  # no residual plane is written
             assert torch.equal(w[:rows].view(torch.uint8), g[:rows].view(torch.uint8)), (rows, i)
             assert_inactive_untouched(g, rows)
+        scales = torch.zeros_like(got[5])  # zero behind the rows
+        scales[offsets[:rows]] = want[5][offsets[:rows]]
+        assert torch.equal(scales, got[5]), rows
     assert c.device_status() == 0
+
+
+class _KernelNode(ctypes.Structure):
+    _fields_ = [("func", ctypes.c_void_p), ("grid", ctypes.c_uint * 3), ("block", ctypes.c_uint * 3),
+                ("shared_bytes", ctypes.c_uint), ("params", ctypes.c_void_p), ("extra", ctypes.c_void_p),
+                ("kern", ctypes.c_void_p), ("ctx", ctypes.c_void_p)]
+
+
+def test_norms_hold_no_shared_memory_that_they_do_not_use(tk, ctx):
+    """Beside a kernel of another stream that has most of an SM's shared memory a norm must find room: its launch asks
+    for none beyond the few bytes of its reductions (those are static), whatever the number of rows."""
+    from tuiskollm_b200 import synth
+
+    driver = ctypes.CDLL("libcuda.so.1")
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    most, hidden = 2 * sms, 5120
+    x, branch = (synth.torch_normal_bf16(96, i, (most, hidden), "cuda") for i in (1, 2))
+    weight = synth.torch_normal_bf16(96, 3, (hidden,), "cuda", std=0.1)
+    residual, normed = (torch.zeros((most, hidden), dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    codes = torch.zeros((most, hidden), dtype=torch.uint8, device="cuda")
+    scales = torch.zeros((most,), dtype=torch.float32, device="cuda")
+    op = tk.ResidualNormOp(ctx)
+    for rows in (1, 4, 5, 12, 13, 30, 32, 33, 100, sms, sms + 1, most):
+        graph = torch.cuda.CUDAGraph(keep_graph=True)
+        with torch.cuda.graph(graph):
+            op.launch_quantize(None, rows, x, branch, weight, residual, normed, codes, scales)
+        raw, count = ctypes.c_void_p(graph.raw_cuda_graph()), ctypes.c_size_t(1)
+        nodes = (ctypes.c_void_p * 1)()
+        assert driver.cuGraphGetNodes(raw, nodes, ctypes.byref(count)) == 0 and count.value == 1
+        node = _KernelNode()
+        assert driver.cuGraphKernelNodeGetParams_v2(ctypes.c_void_p(nodes[0]), ctypes.byref(node)) == 0
+        assert node.grid[0] == ((rows + 3) // 4 * 4 if 13 <= rows <= 32 else rows), rows
+        assert node.shared_bytes == 0, rows

@@ -84,7 +84,6 @@ cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_
 // ---------------------------------------------------------------- norm_quant.cu
 // threads/chunks for a row of `hidden` BF16 values; false when the row is not admitted.
 bool norm_geometry(int hidden, int* threads, int* chunks);
-cudaError_t norm_prepare();  // sets the dynamic shared-memory attribute of the norms with a quantiser once
 
 // One launch covering any of: residual add (branch != null), RMSNorm
 // (normalized_out != null) and E4M3 quantisation (codes != null).

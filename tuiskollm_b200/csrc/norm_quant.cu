@@ -78,18 +78,20 @@ __device__ __forceinline__ void keep_pair(uint32_t& v, uint32_t w) { v = w; }
 __device__ __forceinline__ F32x2 pair_f32(F32x2 v) { return v; }
 __device__ __forceinline__ F32x2 pair_f32(uint32_t v) { return bf16x2_to_f32x2(v); }
 
-template <bool HAS_BRANCH, bool DO_NORM, bool DO_QUANT, int CHUNKS>
+// PADDED: the grid is filled up to whole clusters (launch_chunks).
+template <bool HAS_BRANCH, bool DO_NORM, bool DO_QUANT, int CHUNKS, bool PADDED>
 __global__ void __launch_bounds__(CHUNKS == 3 ? 704 : 1024)  // norm_geometry: three chunks on at most 704
     resnorm_quant_kernel(const uint16_t* __restrict__ x, const uint16_t* __restrict__ branch,
                          const uint16_t* __restrict__ weight, uint16_t* __restrict__ residual_out,
                          uint16_t* __restrict__ normalized_out, uint8_t* __restrict__ codes,
                          float* __restrict__ scales, int hidden, float eps, uint32_t* status,
-                         const Nvfp4Out nv) {
+                         const Nvfp4Out nv, int rows) {
   __shared__ __align__(16) float sums[32];
   __shared__ uint32_t maxima[32];
   pdl_trigger();
   pdl_wait();  // x / branch may be the predecessor's output
   const int row = blockIdx.x;
+  if (PADDED && row >= rows) return;
   const int chunks_per_row = hidden >> 3;
   const size_t row_off = static_cast<size_t>(row) * hidden;
 
@@ -216,23 +218,33 @@ __global__ void __launch_bounds__(CHUNKS == 3 ? 704 : 1024)  // norm_geometry: t
   }
 }
 
-// Shared memory that a norm asks for and does not use, so that its rows get an SM each (from one and a half rows per SM:
-// two share one).  Left alone, the CTAs pile up three to an SM where the kernel in front frees one first, and CTAs of the
-// projection behind join them, whose weight tiles then fill the SM's way to L2 in front of the rows.
-// Without / with it, us: the norm itself (E4M3) 16 rows 2.16 / 2.01, 48 3.47 / 2.59, 100 4.10 / 2.93; with a projection
-// behind it, 16 rows 8192 x 5120 10.8 / 10.4, 16384 x 5120 17.8 / 16.9, 5120 x 6144 10.2 / 9.0, 32 rows 12.9 / 12.4,
-// 19.5 / 18.5, 11.6 / 10.6; equal up to four rows.  Two an SM: 256 rows 4.67 / 4.29, 296 4.83 / 4.40, but 200 3.97 / 4.09.
-constexpr int kOneAnSm = 160 * 1024, kTwoAnSm = 100 * 1024;
-
 template <bool HAS_BRANCH, bool DO_NORM, bool DO_QUANT>
 cudaError_t launch_chunks(cudaStream_t stream, int rows, int hidden, int threads, int chunks,
                           const uint16_t* x, const uint16_t* branch, const uint16_t* weight,
                           uint16_t* residual_out, uint16_t* normalized_out, uint8_t* codes,
-                          float* scales, float eps, uint32_t* status, const Nvfp4Out& nv, int spread_bytes) {
+                          float* scales, float eps, uint32_t* status, const Nvfp4Out& nv) {
+  // Norms with a quantiser: 13 to 32 rows in clusters of four, whose CTAs have an SM each.  Alone they pile up on the SMs
+  // that the kernel in front frees first, three to an SM, and share what it can load.  Without / with, us:
+  //   12288 x 5120 FP8 behind it, 14 / 16 / 24 / 32 rows 13.9 / 14.1 / 15.4 / 15.8, so 13.5 / 13.4 / 14.2 / 15.1 (8192
+  //     rows of weights, 16: 10.9, so 11.1); 8192 x 2048, 32 rows 8.4, so 8.1; 12288 x 4096 14.1, 13.0; x 6144 18.4, 17.1;
+  //   NVFP4 MLP of 5120 columns, 14 / 16 / 24 / 32 tokens 32.3 / 32.8 / 33.6 / 34.3, so 30.8 / 31.1 / 32.3 / 32.9.
+  // Not with fewer rows (8192 x 5120, 12 rows 10.0, so 10.4) or more (48 rows 12.4, so 13.2: clusters share SMs too, and
+  // beside another stream's kernel wait for four places), not with wider rows (10240 x 8192 equal, 8192 x 16384, 32 rows
+  // 32, so 37) or narrower ones (the norm itself, 512 columns, 1.42, so 1.45).  Shared memory asked for and not used
+  // spreads up to a wave of rows, but such a norm waits for a free SM: 32 rows beside another stream's FP8 gate/up 14,
+  // so 27, 100 rows beside attention 18, so 34; and 10240 x 8192 behind 32 rows took 23.4 for 20.4.
+  if constexpr (DO_NORM && DO_QUANT) {
+    if (rows >= 13 && rows <= 32 && hidden >= 2048 && hidden <= 6144 && chunks <= 2) {
+      const auto kernel = chunks == 1 ? resnorm_quant_kernel<HAS_BRANCH, DO_NORM, DO_QUANT, 1, true>
+                                      : resnorm_quant_kernel<HAS_BRANCH, DO_NORM, DO_QUANT, 2, true>;
+      return launch_kernel_cluster(kernel, dim3((rows + 3) & ~3), dim3(threads), 0, stream, dim3(4), x, branch, weight,
+                                   residual_out, normalized_out, codes, scales, hidden, eps, status, nv, rows);
+    }
+  }
 #define TK100_LAUNCH(C)                                                                       \
-  launch_kernel(resnorm_quant_kernel<HAS_BRANCH, DO_NORM, DO_QUANT, C>, dim3(rows), dim3(threads), \
-                spread_bytes, stream, x, branch, weight, residual_out, normalized_out, codes, scales, hidden, \
-                eps, status, nv)
+  launch_kernel(resnorm_quant_kernel<HAS_BRANCH, DO_NORM, DO_QUANT, C, false>, dim3(rows), dim3(threads), \
+                0, stream, x, branch, weight, residual_out, normalized_out, codes, scales, hidden, \
+                eps, status, nv, rows)
   switch (chunks) {
     case 1: return TK100_LAUNCH(1);
     case 2: return TK100_LAUNCH(2);
@@ -266,22 +278,6 @@ bool pdl_enabled() { return g_pdl; }
 uint32_t debug_flags() { return g_debug; }
 
 unsigned long long* debug_stamps() { return g_stamps; }
-
-cudaError_t norm_prepare() {
-  cudaError_t e = cudaSuccess;
-  auto allow = [&](auto kernel) {
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kOneAnSm);
-  };
-  allow(resnorm_quant_kernel<true, true, true, 1>);
-  allow(resnorm_quant_kernel<true, true, true, 2>);
-  allow(resnorm_quant_kernel<true, true, true, 3>);
-  allow(resnorm_quant_kernel<true, true, true, 4>);
-  allow(resnorm_quant_kernel<false, true, true, 1>);
-  allow(resnorm_quant_kernel<false, true, true, 2>);
-  allow(resnorm_quant_kernel<false, true, true, 3>);
-  allow(resnorm_quant_kernel<false, true, true, 4>);
-  return e;
-}
 
 bool norm_geometry(int hidden, int* threads, int* chunks) {
   if (hidden <= 0 || (hidden & 7) != 0) return false;
@@ -321,20 +317,15 @@ cudaError_t launch_resnorm_quant(cudaStream_t stream, int rows, int hidden, cons
   // 5120 columns, one / two / four: 600 rows 4.1 / 4.5 / 3.6, 2048 9.4 / 10.0 / 6.8.  With the norm the chunks
   // double; 5120 columns, one / two / four: 512 rows 7.0 / 6.5 / 8.7, 800 9.2 / 9.5 / 10.5, 1024 rows and
   // more equal; 10240 columns, two / four: 600 rows 13.9 / 15.1, 1024 21.8 / 20.5, 2048 38.9 / 36.9.
-  static int sms = 0;
-  if (sms == 0) {
-    int device = 0;
-    if (cudaGetDevice(&device) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
-      sms = 148;
-    }
-  }
-  int spread_bytes = 0;
-  if (do_norm && do_quant) {
-    if (rows >= 5 && rows <= sms) spread_bytes = kOneAnSm;
-    else if (2 * rows > 3 * sms && rows <= 2 * sms) spread_bytes = kTwoAnSm;
-  }
   if (chunks <= 2) {
+    static int sms = 0;
+    if (sms == 0) {
+      int device = 0;
+      if (cudaGetDevice(&device) != cudaSuccess ||
+          cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
+        sms = 148;
+      }
+    }
     const int resident = !do_norm && chunks == 2 ? 1536 : 2048;  // threads of an SM
     const int wide = do_norm ? 2 * chunks : 4;
     const int narrow = (((hidden >> 3) + wide - 1) / wide + 31) & ~31;
@@ -346,7 +337,7 @@ cudaError_t launch_resnorm_quant(cudaStream_t stream, int rows, int hidden, cons
 #define TK100_CASE(B, N, Q)                                                                      \
   if (has_branch == B && do_norm == N && do_quant == Q)                                          \
   return launch_chunks<B, N, Q>(stream, rows, hidden, threads, chunks, x, branch, weight,        \
-                                residual_out, normalized_out, codes, scales, eps, status, nv, spread_bytes)
+                                residual_out, normalized_out, codes, scales, eps, status, nv)
   TK100_CASE(true, true, true);
   TK100_CASE(true, true, false);
   TK100_CASE(false, true, true);

@@ -131,11 +131,6 @@ Status Context::create(const tk100_config& in, Context** out, std::string* error
     delete ctx;
     return TK100_ERR_MODULE;
   }
-  if ((e = norm_prepare()) != cudaSuccess) {
-    *error = std::string("[gpu.module] preparing the norm: ") + cudaGetErrorString(e);
-    delete ctx;
-    return TK100_ERR_MODULE;
-  }
   if ((e = gdn_recurrence_prepare()) != cudaSuccess) {
     *error = std::string("[gpu.module] preparing the GDN recurrence: ") + cudaGetErrorString(e);
     delete ctx;
