@@ -16,6 +16,20 @@ def test_kernel_resources_match_the_blessed_baseline(capsys):
     assert rc == 0, out[-3000:]
 
 
+def test_unsplit_pair_contractions_carry_no_code_of_split_ones():
+    """What adds the parts of a split K up needs 150 registers and more; in one kernel with it the unsplit launches took
+    up to 0.4 us longer.  (Last template argument: whether a cluster's pairs split K.)"""
+    registers = {}
+    with open(os.path.join(ROOT, "qual", "baselines", "resources-sm100.txt")) as f:
+        for line in f:
+            if "::pair_gemm_kernel<" in line:
+                name, resources = line.split(" = ")
+                registers[name.split("::")[1]] = int(resources.split()[0].split(":")[1])
+    for nvfp4 in (0, 1):
+        unsplit, split = (registers["pair_gemm_kernel<(bool)%d,(bool)0,(bool)%d>" % (nvfp4, s)] for s in (0, 1))
+        assert unsplit <= 112 < split, registers
+
+
 def test_timing_gate_arithmetic():
     import xtask
 

@@ -86,7 +86,10 @@ __device__ __forceinline__ void sts128(uint32_t addr, const uint4& v) {
 template <int N>
 using Int = std::integral_constant<int, N>;
 
-template <bool NV, bool SWIGLU>
+// SPLIT: the pairs of a cluster split K, of every tile or of those that rounds of whole ones leave (SwiGLU never does).  A
+// kernel of its own: with that code in it (158 registers instead of 96) unsplit launches took 0.2 to 0.6 us longer (NVFP4
+// down, K 4352, 301 / 777 tokens 9.9 / 15.6 us, 10.4 / 16.2 with it; FP8 5120 x 6144, 301 tokens 12.9, 13.2).
+template <bool NV, bool SWIGLU, bool SPLIT>
 __global__ void __launch_bounds__(block_threads(NV, SWIGLU), 1)
     pair_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a,
                      const __grid_constant__ CUtensorMap map_wsf, const __grid_constant__ CUtensorMap map_asf,
@@ -103,7 +106,7 @@ __global__ void __launch_bounds__(block_threads(NV, SWIGLU), 1)
   const uint32_t rank = cta & 1u;        // 0 = even CTA of its pair (issues the MMAs)
   const uint32_t leader = cta & ~1u;     // the pair's even CTA
   const int split = static_cast<int>(cta >> 1);
-  const int splits = p.splits;
+  const int splits = SPLIT ? p.splits : 1;
   const int worker = static_cast<int>(blockIdx.x) / (2 * splits);
   const int workers = static_cast<int>(gridDim.x) / (2 * splits);
   const int tok_tile = p.tok_tile;
@@ -111,7 +114,7 @@ __global__ void __launch_bounds__(block_threads(NV, SWIGLU), 1)
   const int k0 = static_cast<int>(static_cast<long long>(split) * p.nkb / splits);
   const int k1 = static_cast<int>(static_cast<long long>(split + 1) * p.nkb / splits);
   // NVFP4 projections: behind `rounds` rounds of whole tiles on all pairs the cluster's pairs split K of one more.
-  constexpr bool TAILS = NV && !SWIGLU;
+  constexpr bool TAILS = NV && SPLIT;
   const int rounds = TAILS ? p.rounds : 0;
   const int whole = rounds * workers * splits;
   // The n-th tile of this pair: index and blocks of K.
@@ -124,8 +127,8 @@ __global__ void __launch_bounds__(block_threads(NV, SWIGLU), 1)
       last_kb = p.nkb;
       return true;
     }
-    t = TAILS && splits > 1 ? whole + worker : worker + n * workers;
-    return t < tiles && (!TAILS || splits == 1 || n == rounds);
+    t = TAILS ? whole + worker : worker + n * workers;
+    return t < tiles && (!TAILS || n == rounds);
   };
   const int stages = p.stages;
   const uint32_t stage_bytes = static_cast<uint32_t>(p.stage_bytes);
@@ -467,7 +470,7 @@ __global__ void __launch_bounds__(block_threads(NV, SWIGLU), 1)
       float ws[4];
       float2 as[4];
       row_scales(unit, ws);
-      const bool shared = !SWIGLU && splits > 1 && n == rounds;  // the tile whose K the cluster's pairs split
+      const bool shared = SPLIT && n == rounds;  // the tile whose K the cluster's pairs split
       if (!shared) token_scales(tok0 + batch_of(part) * kBatch, as);
       if (!mbar_wait(&ctl->acc_full[b], (n >> 1) & 1, p.status)) break;
       tc_fence_after_sync();
@@ -513,7 +516,7 @@ __global__ void __launch_bounds__(block_threads(NV, SWIGLU), 1)
       }
     }
 
-    if (!SWIGLU && splits > 1) {
+    if constexpr (SPLIT) {
       cluster_arrive();
       cluster_wait();
       t = whole + worker;
@@ -575,7 +578,7 @@ __global__ void __launch_bounds__(block_threads(NV, SWIGLU), 1)
       }
     }
   }
-  if (!SWIGLU && splits > 1 && warp < 2) {
+  if (SPLIT && warp < 2) {
     __syncwarp();
     cluster_arrive();
     cluster_wait();
@@ -597,13 +600,14 @@ __global__ void __launch_bounds__(block_threads(NV, SWIGLU), 1)
 template <bool NV, bool SWIGLU>
 cudaError_t pg_launch(cudaStream_t stream, int workers, const CUtensorMap& w, const CUtensorMap& a,
                       const CUtensorMap& wsf, const CUtensorMap& asf, const PairGemmParams& p) {
-  return launch_kernel_cluster(pair_gemm_kernel<NV, SWIGLU>, dim3(2 * p.splits * workers), dim3(block_threads(NV, SWIGLU)),
-                               kSmemLimit, stream, dim3(2 * p.splits), w, a, wsf, asf, p);
+  const auto kernel = !SWIGLU && p.splits > 1 ? pair_gemm_kernel<NV, SWIGLU, !SWIGLU> : pair_gemm_kernel<NV, SWIGLU, false>;
+  return launch_kernel_cluster(kernel, dim3(2 * p.splits * workers), dim3(block_threads(NV, SWIGLU)), kSmemLimit, stream,
+                               dim3(2 * p.splits), w, a, wsf, asf, p);
 }
 
-template <bool NV, bool SWIGLU>
+template <bool NV, bool SWIGLU, bool SPLIT>
 cudaError_t pg_prepare() {
-  return cudaFuncSetAttribute(pair_gemm_kernel<NV, SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  return cudaFuncSetAttribute(pair_gemm_kernel<NV, SWIGLU, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               static_cast<int>(kSmemLimit));
 }
 
@@ -620,10 +624,12 @@ int pair_gemm_stages(int stage_bytes, bool one_tile) {
 
 cudaError_t pair_gemm_prepare(int* max_clusters) {
   cudaError_t e;
-  if ((e = pg_prepare<false, false>()) != cudaSuccess) return e;
-  if ((e = pg_prepare<false, true>()) != cudaSuccess) return e;
-  if ((e = pg_prepare<true, false>()) != cudaSuccess) return e;
-  if ((e = pg_prepare<true, true>()) != cudaSuccess) return e;
+  if ((e = pg_prepare<false, false, false>()) != cudaSuccess) return e;
+  if ((e = pg_prepare<false, false, true>()) != cudaSuccess) return e;
+  if ((e = pg_prepare<false, true, false>()) != cudaSuccess) return e;
+  if ((e = pg_prepare<true, false, false>()) != cudaSuccess) return e;
+  if ((e = pg_prepare<true, false, true>()) != cudaSuccess) return e;
+  if ((e = pg_prepare<true, true, false>()) != cudaSuccess) return e;
   // clusters of 2, 4, 6 and 8 CTAs (one CTA per SM) that are resident at once
   for (int s = 1; s <= kPairGemmMaxSplits; ++s) {
     cudaLaunchConfig_t cfg = {};
@@ -638,7 +644,7 @@ cudaError_t pair_gemm_prepare(int* max_clusters) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int clusters = 0;
-    e = cudaOccupancyMaxActiveClusters(&clusters, pair_gemm_kernel<true, true>, &cfg);
+    e = cudaOccupancyMaxActiveClusters(&clusters, pair_gemm_kernel<true, true, false>, &cfg);
     if (e != cudaSuccess) {
       (void)cudaGetLastError();
       clusters = 0;
