@@ -100,7 +100,8 @@ TK100_API tk100_status tk100_device_status(tk100_ctx* ctx, tk100_stream stream, 
 TK100_API uint64_t tk100_launch_count(const tk100_ctx* ctx);
 /* Name of the kernel the last projection launch on this context took with two of its parameters and
  * its K splits, e.g. "fp8_projection_kernel<16,1> splits=1" (token tile, ring variant) or
- * "pair_gemm_kernel<160,40> splits=1 cluster" (token tile, resident clusters) -- for reports and
+ * "pair_gemm_kernel<160,40> splits=1 cluster" (token tile, resident clusters); " rounds=n" where n rounds of
+ * whole tiles go before the split ones, " few" where few splits finish more tokens at a time -- for reports and
  * route tests; valid until the next call.  No counterpart in the reference. */
 TK100_API const char* tk100_last_kernel(tk100_ctx* ctx);
 

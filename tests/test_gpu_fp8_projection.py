@@ -268,10 +268,11 @@ def test_split_k_reduction_routes_agree_bit_for_bit(tk, oracle, rows, monkeypatc
 
 
 @pytest.mark.parametrize("splits", [2, 3, 4, 5])
-@pytest.mark.parametrize("rows", [1, 7, 9, 16, 17, 32])
+@pytest.mark.parametrize("rows", [1, 7, 8, 9, 12, 13, 16, 17, 32])
 def test_tokens_of_a_split_tile_in_groups_of_four_and_two(tk, rows, splits, monkeypatch):
-    """Up to four splits with more than four tokens each are finished four at a time, others two: the same bits as the tiles that meet in
-    global scratch, for every remainder of a group and an output row count that ends inside a tile."""
+    """Up to four splits with more than four tokens each are finished four at a time, others two, on both sides of
+    each line: the same bits as the tiles that meet in global scratch, for every remainder of a group and an output
+    row count that ends inside a tile."""
     from tuiskollm_b200 import synth
 
     hidden, out_rows = 1280, 400
@@ -286,6 +287,7 @@ def test_tokens_of_a_split_tile_in_groups_of_four_and_two(tk, rows, splits, monk
         tk.Fp8ProjectionOp(c).launch(None, rows, out_rows, hidden, x, planes.codes, planes.scales, w, s, planes.out)
         torch.cuda.synchronize()
         assert f"splits={splits}" in c.last_kernel and ("cluster" in c.last_kernel) == (mode == "3"), c.last_kernel
+        assert c.last_kernel.endswith(" few") == (mode == "3" and splits <= 4 and rows > 4 * splits), c.last_kernel
         planes.check_inactive(rows)
         assert c.device_status() == 0
         outs.append(_u16(planes.out)[:rows].copy())

@@ -731,3 +731,46 @@ def test_gate_up_quarters_of_the_tokens(tk, oracle, monkeypatch, rows, divisor):
     assert np.array_equal(host(got[0][2]), msc)
     if divisor < 1e-3:
         assert not msc.any() and mc.any()
+
+
+@pytest.mark.parametrize("rows", [1, 3, 8, 13, 32])
+@pytest.mark.parametrize("weight_divisor", [2.0 ** -41, 2.0 ** -105])
+def test_gate_up_quarters_of_outputs_that_are_not_finite(tk, monkeypatch, rows, weight_divisor):
+    """Outputs beyond BF16: the epilogue's codes and scales are those of the quantiser launch on the same rounded
+    outputs.  With the first scale a part of the products gate x up overflows, with the second gates and ups do
+    themselves, and a gate of -inf or an infinite up under a gate whose SiLU is zero gives NaN."""
+    from tuiskollm_b200 import synth
+
+    hidden, inter = 512, 384
+    xb = synth.normal_bf16(72, rows, (rows, hidden))
+    gu, gus, gud = synth.nvfp4_weights(72, 1, 2 * inter, hidden)
+    got = []
+    for mode in ("3", "2"):
+        monkeypatch.setenv("TK100_CLUSTER", mode)
+        c = tk.Context(device=0, hidden=hidden, intermediate=inter)
+        codes = torch.zeros((rows, hidden // 2), dtype=torch.uint8, device="cuda")
+        scales = torch.zeros((tk.ops.nvfp4_scale_plane_bytes(rows, hidden),), dtype=torch.uint8, device="cuda")
+        m_codes = sentinel_plane((rows + 1, inter // 2), torch.uint8)
+        m_scales = torch.zeros((tk.ops.nvfp4_scale_plane_bytes(rows, inter),), dtype=torch.uint8, device="cuda")
+        mid = sentinel_plane((rows + 1, inter), torch.int16)
+        op = tk.Nvfp4SwiGluOp(c)
+        # largest finite outputs get block scales around 40
+        planes = dict(activation_codes=codes, activation_scales=scales, output_global_divisor=2.0 ** -120,
+                      output_codes=m_codes, output_scales=m_scales)
+        # the codes of ordinary activations first; then outputs of 1 / weight_divisor times the sums over codes
+        op.launch_quantize(None, rows, dev(xb.view(np.int16)), dev(gu), dev(gus), float(gud), mid,
+                           input_global_divisor=448.0, **planes)
+        op.launch_quantize(None, rows, None, dev(gu), dev(gus), weight_divisor, mid, input_global_divisor=1.0, **planes)
+        torch.cuda.synchronize()
+        assert_inactive_untouched(mid, rows)
+        assert_inactive_untouched(m_codes, rows)
+        got.append((mid, m_codes, m_scales))
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+    out = got[0][0][:rows].view(torch.bfloat16).float()
+    assert torch.isinf(out).any()
+    if weight_divisor > 1e-20:
+        assert (torch.isfinite(out) & (out != 0)).any()
+    else:
+        assert torch.isnan(out).any()
+    assert got[0][1][:rows].any() and got[0][2].any()

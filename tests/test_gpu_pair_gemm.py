@@ -258,19 +258,22 @@ def test_nvfp4_down_route_rules(tk, oracle, hidden, inter, rows, kernel):
     assert c.device_status() == 0
 
 
-@pytest.mark.parametrize("rows,inter,split", [
-    (1000, 6208, True),    # 80 tiles: a round of whole ones, 14 left over; a last stage of one step
-    (1930, 4160, True),    # 160 tiles: two rounds, then split ones on the other accumulator's turn
-    (1000, 3840, False),   # fewer than eight stages a split
-    (700, 6208, False),    # 60 tiles in one round
+@pytest.mark.parametrize("hidden,rows,inter,tok,rounds", [
+    (5120, 1000, 6208, 0, 1),    # 80 tiles: a round of whole ones, 14 left over; a last stage of one step
+    (5120, 1930, 4160, 0, 2),    # 160 tiles: two rounds, then split ones on the other accumulator's turn
+    (5120, 1000, 3840, 0, 0),    # fewer than eight stages a split
+    (5120, 700, 6208, 0, 0),     # 60 tiles in one round
+    (24576, 100, 4160, 0, 1),    # 128-token tiles, whose accumulators are disjoint: 96 of them
+    (19200, 200, 6208, 128, 2),  # 150: the split ones come when the first accumulator has been read twice
+    (22528, 50, 6208, 0, 1),     # 88, three splits: up to 64 tokens too, where few tiles go to one-CTA tiles
 ])
-def test_nvfp4_down_whole_tiles_then_split_ones(tk, oracle, monkeypatch, rows, inter, split):
-    """Tiles left over by the rounds of whole tiles are split over the pairs of a cluster.  Against the unsplit
-    plan: K / 64 accumulations on either side, each within 2^-23 of a partial sum, and partial sums within twice the
-    largest result."""
+def test_nvfp4_down_whole_tiles_then_split_ones(tk, oracle, monkeypatch, hidden, rows, inter, tok, rounds):
+    """Tiles left over by the rounds of whole tiles are split over the pairs of a cluster (counts for 148 SMs: 74
+    pairs, 33 clusters of two, 22 of three).  Against the unsplit plan: K / 64 accumulations on either side, each
+    within 2^-23 of a partial sum, and partial sums within twice the largest result."""
     from tuiskollm_b200 import synth
 
-    hidden = 5120
+    monkeypatch.setenv("TK100_PAIR_TOK", str(tok))
     xb = synth.normal_bf16(67, rows, (rows, inter))
     dn, dns, dnd = synth.torch_nvfp4_weights(67, 2, hidden, inter, "cuda")
     div = float(np.float32(448.0 * 6.0 / 8.0))
@@ -285,7 +288,8 @@ def test_nvfp4_down_whole_tiles_then_split_ones(tk, oracle, monkeypatch, rows, i
         down = tk.Nvfp4DownOp(c)
         down.launch(None, rows, dev(xb.view(np.int16)), dn, dns, float(dnd), out, **kw)
         assert c.last_kernel.startswith("pair_gemm_kernel"), c.last_kernel
-        assert ("splits=1" in c.last_kernel) == (forced == 1 or not split), c.last_kernel
+        assert c.last_kernel.endswith(f" rounds={rounds}") == (forced == 0 and rounds > 0), c.last_kernel
+        assert ("splits=1" in c.last_kernel) == (forced == 1 or rounds == 0), c.last_kernel
         down.launch_partial(None, rows, None, dn, dns, float(dnd), part, **kw)
         torch.cuda.synchronize()
         first = out.clone()

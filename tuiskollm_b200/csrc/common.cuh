@@ -200,6 +200,13 @@ __device__ __forceinline__ void nvfp4_codes(const F32x2 (&x)[N], float divisor, 
   }
 }
 
+// The quotient of one value that its code is rounded from, as nvfp4_codes forms it.
+__device__ __forceinline__ float nvfp4_quotient(float x, float divisor, float s) {
+  const Reciprocal r = reciprocal_parts(s);
+  const float t = __fmul_rn(x, divisor);
+  return s == 0.0f ? copysignf(0.0f, x) : __fmaf_rn(t, r.hi, __fmul_rn(t, r.lo));
+}
+
 // NVFP4 form of 16 consecutive BF16 values (8 packed pairs, low half first):
 //   scale = e4m3_rne_sat((amax * divisor) / 6),  code = e2m1_rne_sat((x * divisor) / scale),
 // signed zeros when the scale underflows to 0.  Codes low nibble first.

@@ -876,13 +876,19 @@ __global__ void __launch_bounds__(256)
   exchange_and_merge(threadIdx.x, blockDim.x, rows, world, rank, keys, peers, s_step, out, status);
 }
 
+}  // namespace
+
 // Up to four splits and more than four tokens for each to finish: four tokens a round trip instead of two.  Behind a
-// norm, 16384 rows (three splits) 16 / 32 tokens 18.1 / 20.6 -> 17.8 / 19.6 us, 12288 (four) 32 tokens 16.3 -> 15.7.
-// An instantiation of its own, and not with fewer tokens: both loops in one kernel cost launches of six and eight
-// splits 0.2 us, and a layer of few tokens that runs both kernels 0.4 (GDN layer, one token 32.9 -> 33.3).
+// norm, 16384 rows (three splits) 16 / 20 / 32 tokens 17.1 / 18.3 / 19.8 -> 16.9 / 17.6 / 18.7 us, 12288 (four) 17 / 32
+// tokens 14.4 / 15.6 -> 14.1 / 14.9.  An instantiation of its own, and not with fewer tokens: both loops in one kernel
+// cost launches of six and eight splits 0.2 us, and two kernels in one layer cost something too: GDN layer of one token
+// 32.9 -> 33.3; layer slice (8192 rows in six splits, 12288 in four) 17 / 24 tokens 53.8 / 54.6 -> 54.0 / 54.7, but 28 / 32
+// tokens 55.8 / 56.6 -> 55.5 / 56.2, with which the line stays where single launches put it.
 bool fp8_few_splits(const Fp8ProjParams& p) {
   return p.cluster == 1 && p.splits > 1 && p.splits <= 4 && p.rows > 4 * p.splits;
 }
+
+namespace {
 
 template <int BLOCK_TOK>
 cudaError_t launch_one(cudaStream_t stream, const CUtensorMap& tmap_w, const CUtensorMap& tmap_a,

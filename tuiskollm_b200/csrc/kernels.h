@@ -265,6 +265,7 @@ struct Fp8ProjParams {
 // block_tok is the token tile (16, 32, 64, 128 or 256).
 cudaError_t launch_fp8_projection(cudaStream_t stream, int block_tok, const CUtensorMap& tmap_w,
                                   const CUtensorMap& tmap_a, const Fp8ProjParams& p);
+bool fp8_few_splits(const Fp8ProjParams& p);  // four tokens a round trip of the reduction (tiles of up to 32 tokens)
 size_t fp8_projection_smem_bytes(int block_tok);
 int fp8_projection_stages(int block_tok);
 cudaError_t fp8_projection_prepare();  // sets the dynamic shared-memory attributes once

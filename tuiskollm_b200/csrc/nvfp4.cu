@@ -124,10 +124,7 @@ __device__ __forceinline__ void finish_pair_tokens(const Nvfp4Params& p, uint32_
   for (int j = 0; j < N; ++j) {
     const float x = __uint_as_float(bits[j] << 16);
     scale[j] = nvfp4_scale_code(__uint_as_float(((amax[j / 2] >> (16 * (j & 1))) & 0x7fffu) << 16), p.q_divisor);
-    const float s = e4m3_to_f32(scale[j]);
-    const Reciprocal r = reciprocal_parts(s);
-    const float t = __fmul_rn(x, p.q_divisor);
-    q[j] = s == 0.0f ? copysignf(0.0f, x) : __fmaf_rn(t, r.hi, __fmul_rn(t, r.lo));
+    q[j] = nvfp4_quotient(x, p.q_divisor, e4m3_to_f32(scale[j]));
   }
   const int groups = p.out_rows >> 4, g = n >> 4;
 #pragma unroll

@@ -206,8 +206,12 @@ Context::~Context() {
 
 const char* Context::last_kernel() {
   char text[160];
-  std::snprintf(text, sizeof text, "%s<%d,%d> splits=%d%s", route_.family, route_.a, route_.b,
-                route_.splits, route_.cluster == 2 ? " cluster-leader" : route_.cluster ? " cluster" : "");
+  std::snprintf(text, sizeof text, "%s<%d,%d> splits=%d%s%s", route_.family, route_.a, route_.b,
+                route_.splits, route_.cluster == 2 ? " cluster-leader" : route_.cluster ? " cluster" : "", route_.variant);
+  if (route_.rounds > 0) {
+    const size_t n = std::strlen(text);
+    std::snprintf(text + n, sizeof text - n, " rounds=%d", route_.rounds);
+  }
   route_text_ = text;
   return route_text_.c_str();
 }
@@ -1074,7 +1078,8 @@ Status Fp8ProjectionOp::launch(cudaStream_t stream, int rows, int out_rows, int 
   {
     // the ring variant launch_fp8_projection picks for this tile size
     const int ring = (block_tok <= 32 && p.deep_ring == 1) ? 1 : (block_tok <= 16 && p.deep_ring == 2) ? 2 : 0;
-    ctx_.note_route("fp8_projection_kernel", block_tok, ring, splits, splits > 1 ? p.cluster : 0);
+    const bool few = block_tok <= 32 && ring == 0 && fp8_few_splits(p);
+    ctx_.note_route("fp8_projection_kernel", block_tok, ring, splits, splits > 1 ? p.cluster : 0, 0, few ? " few" : "");
   }
   TK100_TRY(ctx_.check(launch_fp8_projection(stream, block_tok, map_w, map_a, p),
                        "launching the FP8 projection"));
@@ -1317,7 +1322,7 @@ Status Nvfp4MlpOp::launch(cudaStream_t stream, bool gate_up, int rows, int out_r
         q.q_divisor = next->divisor;
       }
       ctx_.count_launch();
-      ctx_.note_route("pair_gemm_kernel", plan.tok_tile, plan.workers, plan.splits, 1);
+      ctx_.note_route("pair_gemm_kernel", plan.tok_tile, plan.workers, plan.splits, 1, plan.rounds);
       return ctx_.check(launch_pair_gemm(stream, true, gate_up, plan.workers, map_w, map_a, map_wsf, map_asf, q),
                         "launching the persistent NVFP4 projection");
     }

@@ -111,9 +111,9 @@ class Context {
   void count_launch(int n = 1) { launches_ += static_cast<uint64_t>(n); }
   uint64_t launches() const { return launches_; }
   // Which kernel instantiation the last projection launch took (for reports and route tests):
-  // a pointer and four integers per launch, formatted only when somebody asks.
-  void note_route(const char* family, int a, int b, int splits, int cluster) {
-    route_ = {family, a, b, splits, cluster};
+  // two pointers and five integers per launch, formatted only when somebody asks.
+  void note_route(const char* family, int a, int b, int splits, int cluster, int rounds = 0, const char* variant = "") {
+    route_ = {family, variant, a, b, splits, cluster, rounds};
   }
   const char* last_kernel();
 
@@ -134,8 +134,8 @@ class Context {
   Tuning tuning_;
   uint64_t launches_ = 0;
   struct RouteNote {
-    const char* family = "";
-    int a = 0, b = 0, splits = 0, cluster = 0;
+    const char *family = "", *variant = "";
+    int a = 0, b = 0, splits = 0, cluster = 0, rounds = 0;
   } route_;
   std::string route_text_;
   std::string last_error_;

@@ -7,7 +7,7 @@
 // CTA loads its 128 weight rows and half of the tokens; one pair per two SMs stays resident and walks
 // its share of the tiles (token tiles fastest: the pairs that run together read the same weights).
 //
-//   warp 0     TMA producer, one ring across all tiles of the pair (as many stages as fit 209 KB)
+//   warp 0     TMA producer, one ring across all tiles of the pair (as many stages as fit 209 KB, FP8 with one tile per pair 225)
 //   warp 1     even CTA: scale copies (NVFP4) and MMAs for both CTAs
 //   warps 2-   epilogue: two (NVFP4 SwiGLU: four) warps per TMEM lane quadrant, alternate 32-token batches
 //
@@ -355,7 +355,7 @@ __global__ void __launch_bounds__(block_threads(NV, SWIGLU), 1)
       }
     };
 
-    // Scales of this thread's tokens in [t0, t0 + 32).
+    // Scales of this thread's tokens in [t0, t0 + 32); NVFP4 has none.
     auto token_scales = [&](int t0, float2 (&as)[4]) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
@@ -465,7 +465,9 @@ __global__ void __launch_bounds__(block_threads(NV, SWIGLU), 1)
       const int b = n & 1;
       // Batches part, part + PARTS, ... in the order in which columns are due.  Token scales are requested a
       // batch ahead: behind the wait every batch of a pair's last tile paid an L2 round trip for them (12288 rows,
-      // 256 tokens 20.4 -> 20.1 us, 8192 rows, 301 tokens 15.2 -> 15.0).
+      // 256 tokens 20.4 -> 20.1 us, 8192 rows, 301 tokens 15.2 -> 15.0).  A warp's last batch asks for a batch
+      // outside the tile: the tokens behind it (checked against the row count, then dropped), and never those in front
+      // of the first tile, because only NVFP4 has overlapping accumulators and it reads no token scales.
       auto batch_of = [&](int o) { return (overlap && b == 0) ? batches - 1 - o : o; };
       float ws[4];
       float2 as[4];
