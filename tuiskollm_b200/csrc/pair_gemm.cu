@@ -106,7 +106,9 @@ __global__ void __launch_bounds__(block_threads(NV, SWIGLU), 1)
   const uint32_t rank = cta & 1u;        // 0 = even CTA of its pair (issues the MMAs)
   const uint32_t leader = cta & ~1u;     // the pair's even CTA
   const int split = static_cast<int>(cta >> 1);
-  const int splits = SPLIT ? p.splits : 1;
+  // With SwiGLU p.splits is 1.  As a constant it brings the first weight requests forward by 0.2 us, in front of the rows
+  // of a norm that ran before: NVFP4 MLP of 100 tokens 39.7 us, constant 40.0; layer slice of 48 tokens 61.2 and 60.6.
+  const int splits = SPLIT || SWIGLU ? p.splits : 1;
   const int worker = static_cast<int>(blockIdx.x) / (2 * splits);
   const int workers = static_cast<int>(gridDim.x) / (2 * splits);
   const int tok_tile = p.tok_tile;
