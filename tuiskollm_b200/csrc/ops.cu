@@ -437,8 +437,8 @@ PairPlan plan_pairs(const Context& ctx, int rows, int row_units, int nkb, bool n
       if (clusters <= 0 || (s > 1 && (!may_split || nkb / s < 8))) continue;
       // Rounds of whole tiles on all pairs, then at most one tile a cluster, its K split.  Both in one launch for
       // NVFP4 only, whose stage costs nearly the same at 128 tokens as at 256, so that no narrower tile fills the
-      // last round: down, two rounds -> one and a third, 800 tokens 48.6 -> 39.6 us, 1024 49.2 -> 40.1; three
-      // -> two and a half, 2048 tokens 73.4 -> 68.1.  FP8 takes narrower tiles instead (5120 x 6144, 1024
+      // last round: down, two rounds -> one and a third, 777 tokens 45.2 -> 37.4 us, 1000 47.5 -> 38.3; three
+      // -> two and a half, 2048 tokens 71.9 -> 67.8, although 33 clusters of two leave 8 of the 74 pairs idle.  FP8 takes narrower tiles instead (5120 x 6144, 1024
       // tokens 31 us, split behind whole tiles 36; 5120 x 17408 70 and 69).
       const long long pairs = static_cast<long long>(s) * clusters;
       const long long rounds = s > 1 ? tiles / pairs : (tiles + pairs - 1) / pairs;
@@ -1410,8 +1410,8 @@ Status Nvfp4MlpOp::launch(cudaStream_t stream, bool gate_up, int rows, int out_r
       p.cluster = 2;
     }
   }
-  // Decode shapes quantise in the epilogue of the CTA that finishes the tokens (saves a launch:
-  // M = 1 23.2 -> 22.1 us); from 128-token tiles on that epilogue work is not hidden and the
+  // Decode shapes quantise in the epilogue of the CTA that finishes the tokens, which saves a launch
+  // (1 / 8 / 32 tokens 18.4 / 18.8 / 19.6 -> 17.2 / 17.2 / 18.7 us); from 128-token tiles on that epilogue work is not hidden and the
   // quantiser kernel after the projection is faster (M = 2048: 351 against 419 us).
   const bool in_epilogue = next && as_pairs && block_tok == 32 && p.cluster != 2;
   if (in_epilogue) {
